@@ -24,55 +24,235 @@ __device__ __forceinline__ float prep_load(const float* p) { return __ldg(p); }
 __device__ __forceinline__ float prep_load(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ uint8_t prep_e4m3(float v) { return static_cast<uint8_t>(sl8::pack_e4m3x2(v, 0.0f) & 0xFFu); }
 
-// One block per (image, patch row): the C * P image rows of that strip are read with coalesced loads, quantised,
-// placed in shared memory at the position they have in the strip's `gw` rows of A (column c * P * P + py * P + px,
-// the flattening order of a Conv2d weight [N, C, P, P]) and those rows are then written whole, pad included.
-template <typename PT>
-__global__ void patchify_quantize_kernel(const PT* __restrict__ pixels, int C, int H, int W, int P, int gh, int gw,
-                                         const float* __restrict__ scale, uint8_t* __restrict__ A, long long lda,
-                                         int row_bytes) {
+// n / d for the small indices below, by one multiplication: exact while n * d < 2^32 (m = ceil(2^32 / d); d = 1: m = 0).
+struct FastDiv {
+    uint32_t m, d;
+};
+inline FastDiv fast_div(int d) { return FastDiv{d > 1 ? static_cast<uint32_t>((0x100000000ull + d - 1) / d) : 0u, static_cast<uint32_t>(d)}; }
+__device__ __forceinline__ uint32_t operator/(uint32_t n, const FastDiv& f) { return f.m ? __umulhi(n, f.m) : n; }
+
+__device__ __forceinline__ uint4 ld_once_16(const void* p) {         // 16 bytes that nothing reads again
+    uint4 q;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "l"(p));
+    return q;
+}
+
+// How the codes of one 16-byte chunk of pixels go to shared memory: byte by byte (odd patch, or rows that start on odd
+// pixels), in pairs (even patch: a pair never straddles two patches), or whole (a patch is a whole number of chunks).
+enum : int { UNFOLD_BYTES = 0, UNFOLD_PAIRS = 1, UNFOLD_CHUNKS = 2 };
+constexpr int kUnfoldThreads = 256;     // at most: a whole number of image rows, chunk by chunk
+constexpr int kUnfoldBatch = 4;         // chunks a thread has in flight
+
+__device__ __forceinline__ void sts_u8(uint32_t at, uint32_t v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts_u16(uint32_t at, uint16_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(v) : "memory"); }
+__device__ __forceinline__ void sts_u32(uint32_t at, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts_u64(uint32_t at, uint32_t lo, uint32_t hi) { asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(lo), "r"(hi) : "memory"); }
+
+// Offsets, inside the group's rows of A (pitch bytes apart), of the codes of the chunk that starts `x` pixels after the
+// group's first one; `outside` for what lies outside the group.
+template <int VP, int NO>
+__device__ __forceinline__ void unfold_offsets(int (&to)[NO], int x, int len, int P, const FastDiv& by_patch, int pitch, int outside) {
+#pragma unroll
+    for (int j = 0; j < NO; j++) {
+        const int xx = x + j * (VP / NO);
+        const uint32_t gx = static_cast<uint32_t>(max(xx, 0)) / by_patch;
+        to[j] = (xx < 0 || xx >= len) ? outside : static_cast<int>(gx) * pitch + (xx - static_cast<int>(gx) * P);
+    }
+}
+
+// Quantises the 16 bytes of pixels in q and puts the codes where `to` says, relative to shared address dst.  SOME: a
+// negative offset is dropped.
+template <typename PT, int MODE, bool SOME, int NO>
+__device__ __forceinline__ void unfold_put(const uint4& q, uint64_t inv2, uint32_t dst, const int (&to)[NO]) {
+    constexpr int VP = 16 / sizeof(PT);
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+    uint16_t code[VP / 2];                                // two codes each
+#pragma unroll
+    for (int j = 0; j < VP / 2; j++) {
+        float lo, hi;
+        if constexpr (sizeof(PT) == 4) { lo = __uint_as_float(w[2 * j]); hi = __uint_as_float(w[2 * j + 1]); }
+        else { lo = __uint_as_float(w[j] << 16); hi = __uint_as_float(w[j] & 0xFFFF0000u); }
+        sl8::unpack_f32x2(sl8::mul_f32x2(sl8::pack_f32x2(lo, hi), inv2), lo, hi);
+        code[j] = sl8::pack_e4m3x2(lo, hi);
+    }
+    if constexpr (MODE == UNFOLD_CHUNKS) {
+        const uint32_t lo = code[0] | (static_cast<uint32_t>(code[1]) << 16);
+        if constexpr (VP == 4) sts_u32(dst + to[0], lo);
+        else sts_u64(dst + to[0], lo, code[2] | (static_cast<uint32_t>(code[3]) << 16));
+    } else {
+#pragma unroll
+        for (int j = 0; j < NO; j++) {
+            if (SOME && to[j] < 0) continue;
+            if constexpr (MODE == UNFOLD_PAIRS) sts_u16(dst + to[j], code[j]);
+            else sts_u8(dst + to[j], static_cast<uint32_t>(code[j / 2]) >> (8 * (j & 1)));
+        }
+    }
+}
+
+// One block per (image, patch row, group of G patches).  The C * P image rows of the group are read in 16-byte chunks
+// (aligned down from the first pixel; what lies outside the group is dropped), quantised, placed in shared memory at
+// the position they have in the group's rows of A (column c * P * P + py * P + px, the flattening order of a Conv2d
+// weight [N, C, P, P]) and those rows are then written whole, pad included.
+// Bound by HBM where three things are seen to.  Bytes in flight: four 16-byte loads per thread (it was one load of two
+// pixels).  Banks: rows of A are multiples of 128 bytes, so unpadded the same pixel of every patch falls into one bank; 16
+// bytes of pad per row spread eight patches over all of them.  Instructions: a thread keeps its chunk position and walks
+// down the image rows, so that where its codes go is worked out once (ALIGNED: every image row starts on a 16-byte
+// boundary, and an image is less than 4 GiB) and a chunk costs its load, conversion, stores and a few additions; dividing
+// for every pair of pixels took 24 instructions per pixel, and the kernel ran at a third of the bandwidth, issue-bound.
+// 256 images of 384 x 384, patch 14: bf16 130 -> 70 us (4.9 TB/s), fp32 123 -> 97 us (5.7 TB/s); 32 images of 224 x 224,
+// patch 16, fp32: 11.5 -> 5.0 us; one such image 7.1 -> 2.2 us.
+template <typename PT, int MODE, bool ALIGNED>
+__global__ void __launch_bounds__(kUnfoldThreads, 4)
+patchify_quantize_kernel(const PT* __restrict__ pixels, long long total, int H, int W, int P, int C, int gh, int gw, int G, int groups,
+                         int rows_per_step, FastDiv by_chunks, FastDiv by_patch, FastDiv by_vecs, const float* __restrict__ scale,
+                         uint8_t* __restrict__ A, long long lda, int row_bytes) {
     extern __shared__ __align__(16) uint8_t prep_tile[];
-    const int img = blockIdx.x / gh, gy = blockIdx.x - img * gh;
-    const int K = C * P * P;
+    constexpr int VP = 16 / sizeof(PT);                   // pixels per chunk
+    constexpr int NO = MODE == UNFOLD_CHUNKS ? 1 : MODE == UNFOLD_PAIRS ? VP / 2 : VP;    // stores per chunk
+    const int strip = blockIdx.x / groups, g = blockIdx.x - strip * groups;
+    const int img = strip / gh, gy = strip - img * gh;
+    const int g0 = g * G, gn = min(G, gw - g0);           // patches of this block
+    const int xs = g0 * P, len = gn * P;                  // ... and their pixels in an image row
+    const int pitch = row_bytes + 16;
+    const int CP = C * P;
     const float inv = __frcp_rn(scale ? __ldg(scale) : 1.0f);
-    for (int i = threadIdx.x; i < gw * (row_bytes - K); i += blockDim.x)          // the zero pad K .. row_bytes
-        prep_tile[(i / (row_bytes - K)) * row_bytes + K + i % (row_bytes - K)] = 0;
-    // A warp per image row (c, gy * P + py) of the strip; its lanes read the row with consecutive 8-byte loads (two
-    // pixels each) and drop the two codes into the patch row they belong to.  Odd P or W: one pixel at a time.
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int strip = gw * P;
-    const bool pairs = (P % 2 == 0) && (W % 2 == 0);
-    for (int cp = warp; cp < C * P; cp += nwarps) {
-        const int py = cp % P, c = cp / P;
-        const PT* src = pixels + ((static_cast<long long>(img) * C + c) * H + (gy * P + py)) * W;
-        uint8_t* dst = prep_tile + c * P * P + py * P;
-        if (pairs) {
-            for (int x = 2 * lane; x < strip; x += 64) {
-                float a, b;
-                if constexpr (sizeof(PT) == 4) {
-                    const float2 v = __ldg(reinterpret_cast<const float2*>(src + x));
-                    a = v.x; b = v.y;
-                } else {
-                    const uint32_t w = __ldg(reinterpret_cast<const unsigned*>(src + x));
-                    a = __uint_as_float(w << 16); b = __uint_as_float(w & 0xFFFF0000u);
+    const uint64_t inv2 = sl8::pack_f32x2(inv, inv);
+    const uint32_t tile = sl8::smem_u32(prep_tile);
+
+    const int row0 = static_cast<int>(static_cast<uint32_t>(threadIdx.x) / by_chunks);    // first image row and chunk of this thread
+    const int v = static_cast<int>(threadIdx.x) - row0 * static_cast<int>(by_chunks.d);
+    const long long first0 = (static_cast<long long>(img) * C * H + gy * P) * W + xs;    // pixel (c = 0, py = 0) of the group
+    int to[NO];
+    if constexpr (ALIGNED) {
+        if (row0 < rows_per_step && v * VP < len) {
+            // (what the last chunk of a row has outside the group goes to a spare row behind the tile: a test for it, taken
+            // by one lane of most warps, would run the conversion twice)
+            unfold_offsets<VP, NO>(to, v * VP, len, P, by_patch, pitch, G * pitch);
+            const char* const base = reinterpret_cast<const char*>(pixels + first0);
+            const uint32_t row_step = static_cast<uint32_t>(rows_per_step) * W * sizeof(PT);
+            const uint32_t plane_step = static_cast<uint32_t>(H - P) * W * sizeof(PT);   // from the last row of a channel's strip to the next one's first
+            const uint32_t dst_step = static_cast<uint32_t>(rows_per_step) * P;
+            int py = row0, left = CP - row0;              // row inside the channel; rows still to come, this one included
+            uint32_t src = static_cast<uint32_t>(row0) * W * sizeof(PT) + 16u * v, dst = tile + row0 * P;
+            while (py >= P) { py -= P; src += plane_step; }
+            while (left > 0) {
+                uint4 q[kUnfoldBatch];
+#pragma unroll
+                for (int b = 0; b < kUnfoldBatch; b++) {
+                    if (left > b * rows_per_step) q[b] = ld_once_16(base + src);
+                    src += row_step;
+                    py += rows_per_step;
+                    while (py >= P) { py -= P; src += plane_step; }
                 }
-                const int gx = x / P, px = x - gx * P;
-                *reinterpret_cast<uint16_t*>(dst + gx * row_bytes + px) = sl8::pack_e4m3x2(a * inv, b * inv);
+#pragma unroll
+                for (int b = 0; b < kUnfoldBatch; b++) {
+                    if (left > b * rows_per_step) unfold_put<PT, MODE, false, NO>(q[b], inv2, dst, to);
+                    dst += dst_step;
+                }
+                left -= kUnfoldBatch * rows_per_step;
             }
-        } else {
-            for (int x = lane; x < strip; x += 32) {
-                const int gx = x / P, px = x - gx * P;
-                dst[gx * row_bytes + px] = prep_e4m3(prep_load(src + x) * inv);
+        }
+    } else if (row0 < rows_per_step) {
+        for (int cp0 = row0; cp0 < CP; cp0 += rows_per_step * kUnfoldBatch) {
+            uint4 q[kUnfoldBatch];
+            int x[kUnfoldBatch];                          // first pixel of the chunk relative to the group
+#pragma unroll
+            for (int b = 0; b < kUnfoldBatch; b++) {
+                const int cp = cp0 + b * rows_per_step;
+                x[b] = len;
+                if (cp >= CP) continue;
+                const int c = static_cast<int>(static_cast<uint32_t>(cp) / by_patch);
+                const long long first = first0 + static_cast<long long>(cp + static_cast<long long>(c) * (H - P)) * W;
+                x[b] = v * VP - static_cast<int>(first & (VP - 1));       // the row starts that many pixels past a chunk boundary
+                if (x[b] >= len) continue;
+                const long long at = first + x[b];
+                if (at + VP <= total) {
+                    q[b] = ld_once_16(pixels + at);
+                } else {                                  // the last chunk of the tensor, when it is not a whole one
+                    PT tail[VP] = {};
+                    for (int j = 0; at + j < total; j++) tail[j] = pixels[at + j];
+                    memcpy(&q[b], tail, 16);
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < kUnfoldBatch; b++) {
+                if (x[b] >= len) continue;
+                unfold_offsets<VP, NO>(to, x[b], len, P, by_patch, pitch, -1);
+                unfold_put<PT, MODE, true, NO>(q[b], inv2, tile + (cp0 + b * rows_per_step) * P, to);
             }
         }
     }
     __syncthreads();
-    const long long m0 = (static_cast<long long>(img) * gh + gy) * gw;
-    const int vecs = row_bytes / 16;
-    for (int i = threadIdx.x; i < gw * vecs; i += blockDim.x) {
-        const int r = i / vecs, v = i - r * vecs;
-        *reinterpret_cast<uint4*>(A + (m0 + r) * lda + 16 * v) = *reinterpret_cast<const uint4*>(prep_tile + r * row_bytes + 16 * v);
+    // 16-byte vectors of the rows of A: a thread keeps its place in the row and walks down the rows.
+    const int vecs = static_cast<int>(by_vecs.d);
+    const int r0 = static_cast<int>(static_cast<uint32_t>(threadIdx.x) / by_vecs);
+    const int steps = static_cast<int>(max(blockDim.x / by_vecs, 1u));
+    if (r0 >= steps) return;
+    const int K = CP * P;
+    for (int vv = static_cast<int>(threadIdx.x) - r0 * vecs; vv < vecs; vv += blockDim.x) {
+        const int keep = K - 16 * vv;                     // codes of this vector; the rest is the zero pad
+        uint8_t* out = A + (static_cast<long long>(strip) * gw + g0 + r0) * lda + 16 * vv;
+        for (int r = r0; r < gn; r += steps, out += steps * lda) {
+            uint4 q = *reinterpret_cast<const uint4*>(prep_tile + r * pitch + 16 * vv);
+            if (keep < 16) {
+                uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int k = keep - 4 * j;
+                    w[j] = k >= 4 ? w[j] : k <= 0 ? 0u : w[j] & (0xFFFFFFFFu >> (32 - 8 * k));
+                }
+                q = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+            *reinterpret_cast<uint4*>(out) = q;
+        }
     }
+}
+
+template <typename PT, int MODE, bool ALIGNED>
+cudaError_t launch_unfold(unsigned grid, size_t smem, cudaStream_t s, const PT* pixels, int images, int C, int H, int W, int P,
+                          int gh, int gw, int G, int groups, int chunks, const float* scale, uint8_t* A, long long lda, int row_bytes) {
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(patchify_quantize_kernel<PT, MODE, ALIGNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    const int rows_per_step = kUnfoldThreads / chunks;                       // image rows a step of the block covers
+    const int threads = (rows_per_step * chunks + 31) / 32 * 32;
+    const long long total = static_cast<long long>(images) * C * H * W;
+    patchify_quantize_kernel<PT, MODE, ALIGNED><<<grid, threads, smem, s>>>(pixels, total, H, W, P, C, gh, gw, G, groups, rows_per_step,
+                                                                            fast_div(chunks), fast_div(P), fast_div(row_bytes / 16), scale, A, lda, row_bytes);
+    return cudaGetLastError();
+}
+
+template <typename PT>
+cudaError_t unfold(cudaStream_t s, const PT* pixels, int images, int C, int H, int W, int P, int gh, int gw, const float* scale,
+                   uint8_t* A, long long lda, int row_bytes, int sm_count) {
+    constexpr int VP = 16 / sizeof(PT);
+    // A whole patch row per block is the cheapest per byte; where there are fewer of them than two blocks per SM, the
+    // patch rows are cut into groups, down to one 128-byte line of an image row (one 224 x 224 image: 14 -> 98 blocks).
+    // They are cut too where the group's rows of A leave no room for four blocks per SM, or where an image row of it has
+    // more chunks than a block has threads.
+    const long long strips = static_cast<long long>(images) * gh;
+    const int line = (128 + P * (int)sizeof(PT) - 1) / (P * (int)sizeof(PT));
+    auto chunks_of = [&](int G) {                                            // chunks an image row of a group can touch
+        return (G * P + VP - 1) / VP + (W % VP == 0 && (G == gw || (G * P) % VP == 0) ? 0 : 1);
+    };
+    int G = gw;
+    while (G > line && (strips * ((gw + G - 1) / G) < 2LL * sm_count || G * (row_bytes + 16) > 48 * 1024 || chunks_of(G) > kUnfoldThreads))
+        G = (G + 1) / 2 < line ? line : (G + 1) / 2;
+    const int groups = (gw + G - 1) / G;
+    const int chunks = chunks_of(G);
+    // The fast path wants 32-bit offsets inside an image and a spare row of A in shared memory.
+    const bool aligned = W % VP == 0 && (groups == 1 || (G * P) % VP == 0) && static_cast<long long>(C) * H * W * sizeof(PT) < (1LL << 32) &&
+                         (G + 1) * (row_bytes + 16) <= 100 * 1024;
+    const size_t smem = static_cast<size_t>(aligned ? G + 1 : G) * (row_bytes + 16);
+    const unsigned grid = static_cast<unsigned>(strips * groups);
+#define SL8_UNFOLD(MODE, AL) launch_unfold<PT, MODE, AL>(grid, smem, s, pixels, images, C, H, W, P, gh, gw, G, groups, chunks, scale, A, lda, row_bytes)
+    if (aligned && P % VP == 0) return SL8_UNFOLD(UNFOLD_CHUNKS, true);
+    if (P % 2 == 0 && aligned) return SL8_UNFOLD(UNFOLD_PAIRS, true);
+    if (P % 2 == 0 && W % 2 == 0) return SL8_UNFOLD(UNFOLD_PAIRS, false);
+    if (aligned) return SL8_UNFOLD(UNFOLD_BYTES, true);
+    return SL8_UNFOLD(UNFOLD_BYTES, false);
+#undef SL8_UNFOLD
 }
 
 // |x| of non-negative floats orders like their bit patterns: one atomicMax on the bits per block.
@@ -207,20 +387,10 @@ SL8_API int sl8_patchify_quantize_e4m3(sl8_handle_t h, const void* pixels, int p
     DeviceGuard guard(h->device);
     if (!guard.ok) return fail(h, SL8_ERR_CUDA, "cudaSetDevice failed");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaError_t e = cudaSuccess;
-    const unsigned grid = static_cast<unsigned>(images) * gh;
-    if (pixel_dtype == SL8_DT_F32) {
-        if (smem > 48 * 1024) e = cudaFuncSetAttribute(patchify_quantize_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            patchify_quantize_kernel<float><<<grid, 256, smem, s>>>(static_cast<const float*>(pixels), channels, height, width, patch,
-                                                                    gh, gw, scale, static_cast<uint8_t*>(A), lda, row_bytes);
-    } else {
-        if (smem > 48 * 1024) e = cudaFuncSetAttribute(patchify_quantize_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            patchify_quantize_kernel<__nv_bfloat16><<<grid, 256, smem, s>>>(static_cast<const __nv_bfloat16*>(pixels), channels, height,
-                                                                            width, patch, gh, gw, scale, static_cast<uint8_t*>(A), lda, row_bytes);
-    }
-    if (e == cudaSuccess) e = cudaGetLastError();
+    const cudaError_t e =
+        pixel_dtype == SL8_DT_F32
+            ? unfold(s, static_cast<const float*>(pixels), images, channels, height, width, patch, gh, gw, scale, static_cast<uint8_t*>(A), lda, row_bytes, h->sm_count)
+            : unfold(s, static_cast<const __nv_bfloat16*>(pixels), images, channels, height, width, patch, gh, gw, scale, static_cast<uint8_t*>(A), lda, row_bytes, h->sm_count);
     return e == cudaSuccess ? SL8_OK : fail_cuda(h, e, "patchify kernel launch");
 }
 

@@ -82,6 +82,32 @@ def test_patchify_quantize_on_gpu(engine, oracle, dtype, images, C, H, W, P):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("images,C,H,W,P", [
+    (1, 3, 224, 224, 16),       # whole chunks, few strips: groups of patches
+    (20, 3, 64, 224, 16),       # whole chunks, groups that do not divide the strip
+    (2, 3, 33, 250, 14),        # pairs, image rows that start off a 16-byte boundary
+    (3, 1, 43, 61, 14),         # odd rows: byte by byte, last chunk of the tensor cut short
+    (1, 2, 9, 13, 3), (1, 1, 5, 3000, 1),   # odd patch; more pixels per strip than a block's shared memory
+])
+def test_patchify_paths_on_gpu(engine, oracle, dtype, images, C, H, W, P):
+    """Every way the codes go to shared memory, at row starts and ends the 16-byte chunks do not fit: bit for bit,
+    at a pitch with a short pad (written as zeros) and one past it (left alone)."""
+    g = torch.Generator(device=DEV).manual_seed(W + P)
+    pixels = (torch.rand((images, C, H, W), generator=g, device=DEV) * 2 - 1).to(dtype)
+    scale = torch.tensor([1.0 / 448.0], device=DEV)
+    K, rows = C * P * P, images * (H // P) * (W // P)
+    for pitch in ((K + 15) // 16 * 16, (K + 15) // 16 * 16 + 160):
+        buf = torch.full((rows, pitch), 0xAA, dtype=torch.uint8, device=DEV)
+        engine.patchify_quantize(pixels, P, scale, out=buf[:, :K])
+        engine.device_status()
+        row_bytes = pitch if pitch - K < 128 else (K + 15) // 16 * 16
+        ref = oracle.patchify_quantize(pixels.float().cpu().numpy(), P, float(scale.item()), lda=pitch, row_bytes=row_bytes)
+        got = buf.cpu().numpy()
+        assert np.array_equal(got[:, :row_bytes], ref[:, :row_bytes]) and (got[:, row_bytes:] == 0xAA).all()
+
+
+@pytest.mark.gpu
 def test_patchify_feeds_the_patch_embed_gemm(engine, oracle):
     """Pixels -> operand rows -> patch-embed GEMM, against the oracle run on the oracle's own operand rows."""
     from siglip_b200 import synth
