@@ -420,8 +420,7 @@ __device__ __forceinline__ void load_bias(float (&b)[NB], const void* bias, unsi
         const int col = col0 + lane + 32 * i;
         float val = 0.0f;
         if (bias != nullptr && col < N)
-            val = (flags & FLAG_BIAS_F32) ? __ldg(static_cast<const float*>(bias) + col)
-                                          : __bfloat162float(__ldg(static_cast<const __nv_bfloat16*>(bias) + col));
+            val = (flags & FLAG_BIAS_F32) ? ld_f32(static_cast<const float*>(bias) + col) : ld_bf16(static_cast<const __nv_bfloat16*>(bias) + col);
         b[i] = val;
     }
 }
@@ -507,6 +506,10 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
+    // Everything above (barriers, tensor memory, descriptors) runs beside the tail of the kernel ahead on the stream.  No
+    // two GEMM CTAs share an SM (each takes more than half its shared memory), so the next GEMM's CTAs move in as these leave.
+    pdl_wait();
+    pdl_release();
 
     // ---------------------------------------------------------------- roles
     if (warp == 0 || warp == 3 + EPI_WARPS) {
@@ -746,8 +749,8 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         static_assert(!HAS_SIDE || NBUF >= 2, "side data needs a buffer to land in while another is stored");
 
         EpiCtx e;
-        e.scale = (p.scale_a ? __ldg(p.scale_a) : 1.0f) * (p.scale_b ? __ldg(p.scale_b) : 1.0f);
-        e.inv_out = __frcp_rn(p.out_scale ? __ldg(p.out_scale) : 1.0f);   // IEEE 1/x, as the CPU oracle computes it
+        e.scale = (p.scale_a ? ld_f32(p.scale_a) : 1.0f) * (p.scale_b ? ld_f32(p.scale_b) : 1.0f);
+        e.inv_out = __frcp_rn(p.out_scale ? ld_f32(p.out_scale) : 1.0f);   // IEEE 1/x, as the CPU oracle computes it
         e.flags = p.flags;
         e.swz = (T::REGION_ROW_BYTES == 128) ? (lane & 7) : ((lane >> 1) & 3);
         e.row_off = lane * T::REGION_ROW_BYTES;
@@ -998,7 +1001,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                         for (int i = 0; i < 32; i++) {
                             const int r = (lane >> 3) + 4 * i;      // staging row 0..127
                             uint4 val = make_uint4(0, 0, 0, 0);
-                            if (col < p.N) val = __ldg(reinterpret_cast<const uint4*>(p.side + static_cast<long long>(t) * p.ld_side + col));
+                            if (col < p.N) val = ld_16(p.side + static_cast<long long>(t) * p.ld_side + col);
                             sts128(buf + r * 128 + ((piece ^ (r & 7)) << 4), val.x, val.y, val.z, val.w);
                             t += 4;
                             while (t >= p.period) t -= p.period;

@@ -20,8 +20,8 @@ typedef Sl8DeviceGuard DeviceGuard;
 
 namespace {
 
-__device__ __forceinline__ float prep_load(const float* p) { return __ldg(p); }
-__device__ __forceinline__ float prep_load(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+__device__ __forceinline__ float prep_load(const float* p) { return sl8::ld_f32(p); }
+__device__ __forceinline__ float prep_load(const __nv_bfloat16* p) { return sl8::ld_bf16(p); }
 __device__ __forceinline__ uint8_t prep_e4m3(float v) { return static_cast<uint8_t>(sl8::pack_e4m3x2(v, 0.0f) & 0xFFu); }
 
 // n / d for the small indices below, by one multiplication: exact while n * d < 2^32 (m = ceil(2^32 / d); d = 1: m = 0).
@@ -33,7 +33,7 @@ __device__ __forceinline__ uint32_t operator/(uint32_t n, const FastDiv& f) { re
 
 __device__ __forceinline__ uint4 ld_once_16(const void* p) {         // 16 bytes that nothing reads again
     uint4 q;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "l"(p) : "memory");
     return q;
 }
 
@@ -103,9 +103,9 @@ __device__ __forceinline__ void unfold_put(const uint4& q, uint64_t inv2, uint32
 // patch 16, fp32: 11.5 -> 5.0 us; one such image 7.1 -> 2.2 us.
 template <typename PT, int MODE, bool ALIGNED>
 __global__ void __launch_bounds__(kUnfoldThreads, 4)
-patchify_quantize_kernel(const PT* __restrict__ pixels, long long total, int H, int W, int P, int C, int gh, int gw, int G, int groups,
-                         int rows_per_step, FastDiv by_chunks, FastDiv by_patch, FastDiv by_vecs, const float* __restrict__ scale,
-                         uint8_t* __restrict__ A, long long lda, int row_bytes) {
+patchify_quantize_kernel(const PT* pixels, long long total, int H, int W, int P, int C, int gh, int gw, int G, int groups,
+                         int rows_per_step, FastDiv by_chunks, FastDiv by_patch, FastDiv by_vecs, const float* scale,
+                         uint8_t* A, long long lda, int row_bytes) {
     extern __shared__ __align__(16) uint8_t prep_tile[];
     constexpr int VP = 16 / sizeof(PT);                   // pixels per chunk
     constexpr int NO = MODE == UNFOLD_CHUNKS ? 1 : MODE == UNFOLD_PAIRS ? VP / 2 : VP;    // stores per chunk
@@ -115,7 +115,9 @@ patchify_quantize_kernel(const PT* __restrict__ pixels, long long total, int H, 
     const int xs = g0 * P, len = gn * P;                  // ... and their pixels in an image row
     const int pitch = row_bytes + 16;
     const int CP = C * P;
-    const float inv = __frcp_rn(scale ? __ldg(scale) : 1.0f);
+    sl8::pdl_wait();
+    sl8::pdl_release();
+    const float inv = __frcp_rn(scale ? sl8::ld_f32(scale) : 1.0f);
     const uint64_t inv2 = sl8::pack_f32x2(inv, inv);
     const uint32_t tile = sl8::smem_u32(prep_tile);
 
@@ -218,9 +220,8 @@ cudaError_t launch_unfold(unsigned grid, size_t smem, cudaStream_t s, const PT* 
     const int rows_per_step = kUnfoldThreads / chunks;                       // image rows a step of the block covers
     const int threads = (rows_per_step * chunks + 31) / 32 * 32;
     const long long total = static_cast<long long>(images) * C * H * W;
-    patchify_quantize_kernel<PT, MODE, ALIGNED><<<grid, threads, smem, s>>>(pixels, total, H, W, P, C, gh, gw, G, groups, rows_per_step,
-                                                                            fast_div(chunks), fast_div(P), fast_div(row_bytes / 16), scale, A, lda, row_bytes);
-    return cudaGetLastError();
+    return sl8_launch_chained(patchify_quantize_kernel<PT, MODE, ALIGNED>, grid, threads, smem, s, pixels, total, H, W, P, C, gh, gw, G, groups, rows_per_step,
+                              fast_div(chunks), fast_div(P), fast_div(row_bytes / 16), scale, A, lda, row_bytes);
 }
 
 template <typename PT>
@@ -260,11 +261,13 @@ template <typename T>
 __device__ __forceinline__ float prep_absmax8(const T* p) {          // max |.| of eight consecutive elements, 16-byte loads
     float m;
     if constexpr (sizeof(T) == 4) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-        m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))),
-                  fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))));
+        const uint4 a = sl8::ld_16(p), b = sl8::ld_16(p + 4);
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        m = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; i++) m = fmaxf(m, fabsf(__uint_as_float(w[i])));
     } else {
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+        const uint4 q = sl8::ld_16(p);
         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
         m = 0.0f;
 #pragma unroll
@@ -277,8 +280,10 @@ __device__ __forceinline__ float prep_absmax8(const T* p) {          // max |.| 
 // `vectors` != 0: rows of cols = 8 * vectors_per_row elements on 16-byte boundaries, eight elements per load;
 // otherwise element by element.
 template <typename T>
-__global__ void amax_kernel(const T* __restrict__ x, long long rows, int cols, long long ld, int vectors,
-                            unsigned* __restrict__ amax_bits) {
+__global__ void amax_kernel(const T* x, long long rows, int cols, long long ld, int vectors,
+                            unsigned* amax_bits) {
+    sl8::pdl_wait();
+    sl8::pdl_release();
     float m = 0.0f;
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
     const long long first = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -311,8 +316,10 @@ __global__ void amax_kernel(const T* __restrict__ x, long long rows, int cols, l
     }
 }
 
-__global__ void scale_from_amax_kernel(const unsigned* __restrict__ amax_bits, float* __restrict__ scale) {
-    const float a = __uint_as_float(*amax_bits);
+__global__ void scale_from_amax_kernel(const float* amax, float* scale) {
+    sl8::pdl_wait();
+    sl8::pdl_release();
+    const float a = sl8::ld_f32(amax);
     *scale = a > 0.0f ? a / 448.0f : 1.0f;                 // 448 = largest e4m3 value; an all-zero tensor keeps scale 1
 }
 
@@ -320,12 +327,14 @@ template <typename T>
 __device__ __forceinline__ void ln_load8(const T* p, float (&v)[8]);
 template <>
 __device__ __forceinline__ void ln_load8<float>(const float* p, float (&v)[8]) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    const uint4 a = sl8::ld_16(p), b = sl8::ld_16(p + 4);
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = __uint_as_float(w[i]);
 }
 template <>
 __device__ __forceinline__ void ln_load8<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[8]) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 q = sl8::ld_16(p);
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -335,9 +344,10 @@ __device__ __forceinline__ void ln_load8<__nv_bfloat16>(const __nv_bfloat16* p, 
 }
 
 template <typename T>
-__global__ void quantize_e4m3_kernel(const T* __restrict__ x, long long rows, int cols, long long ld,
-                                     const float* __restrict__ scale, uint8_t* __restrict__ out, long long ld_out) {
-    const float inv = __frcp_rn(scale ? __ldg(scale) : 1.0f);
+__global__ void quantize_e4m3_kernel(const T* x, long long rows, int cols, long long ld, const float* scale, uint8_t* out, long long ld_out) {
+    sl8::pdl_wait();
+    sl8::pdl_release();
+    const float inv = __frcp_rn(scale ? sl8::ld_f32(scale) : 1.0f);
     const int groups = (cols + 7) / 8;                      // eight columns per thread: one 8-byte store
     const long long total = rows * groups;
     for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -407,12 +417,11 @@ SL8_API int sl8_amax_scale(sl8_handle_t h, const void* x, int dtype, int64_t row
     const int grid = prep_grid(h, rows * cols / 8);
     const int vectors = (cols % 8 == 0 && ld % 8 == 0 && aligned16(x)) ? 1 : 0;
     if (dtype == SL8_DT_F32)
-        amax_kernel<float><<<grid, 256, 0, s>>>(static_cast<const float*>(x), rows, cols, ld, vectors, reinterpret_cast<unsigned*>(amax));
+        e = sl8_launch_chained(amax_kernel<float>, grid, 256, 0, s, static_cast<const float*>(x), rows, cols, ld, vectors, reinterpret_cast<unsigned*>(amax));
     else
-        amax_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, vectors,
-                                                        reinterpret_cast<unsigned*>(amax));
-    if (scale) scale_from_amax_kernel<<<1, 1, 0, s>>>(reinterpret_cast<const unsigned*>(amax), scale);
-    e = cudaGetLastError();
+        e = sl8_launch_chained(amax_kernel<__nv_bfloat16>, grid, 256, 0, s, static_cast<const __nv_bfloat16*>(x), rows, cols, ld, vectors,
+                               reinterpret_cast<unsigned*>(amax));
+    if (scale && e == cudaSuccess) e = sl8_launch_chained(scale_from_amax_kernel, 1, 1, 0, s, amax, scale);
     return e == cudaSuccess ? SL8_OK : fail_cuda(h, e, "amax kernel launch");
 }
 
@@ -425,12 +434,12 @@ SL8_API int sl8_quantize_e4m3(sl8_handle_t h, const void* x, int dtype, int64_t 
     if (!guard.ok) return fail(h, SL8_ERR_CUDA, "cudaSetDevice failed");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int grid = prep_grid(h, rows * ((cols + 7) / 8));
+    cudaError_t e;
     if (dtype == SL8_DT_F32)
-        quantize_e4m3_kernel<float><<<grid, 256, 0, s>>>(static_cast<const float*>(x), rows, cols, ld, scale, static_cast<uint8_t*>(out), ld_out);
+        e = sl8_launch_chained(quantize_e4m3_kernel<float>, grid, 256, 0, s, static_cast<const float*>(x), rows, cols, ld, scale, static_cast<uint8_t*>(out), ld_out);
     else
-        quantize_e4m3_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), rows, cols, ld, scale,
-                                                                 static_cast<uint8_t*>(out), ld_out);
-    cudaError_t e = cudaGetLastError();
+        e = sl8_launch_chained(quantize_e4m3_kernel<__nv_bfloat16>, grid, 256, 0, s, static_cast<const __nv_bfloat16*>(x), rows, cols, ld, scale,
+                               static_cast<uint8_t*>(out), ld_out);
     return e == cudaSuccess ? SL8_OK : fail_cuda(h, e, "quantize kernel launch");
 }
 
@@ -443,13 +452,14 @@ namespace {
 // CHUNKS == 0: any width, three passes over the row (the second and third hit L1 / L2).  Scalar fp32 arithmetic:
 // the packed two-element forms were measured 20 - 40 % slower here.
 template <typename T, int CHUNKS>
-__global__ void __launch_bounds__(256, 3) layernorm_quantize_kernel(const T* __restrict__ x, long long rows, int cols, long long ld,
-                                          const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
-                                          const float* __restrict__ scale, uint8_t* __restrict__ out, long long ld_out) {
+__global__ void __launch_bounds__(256, 3) layernorm_quantize_kernel(const T* x, long long rows, int cols, long long ld, const float* gamma,
+                                          const float* beta, float eps, const float* scale, uint8_t* out, long long ld_out) {
     const int lane = threadIdx.x & 31;
     const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const long long warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
-    const float inv = __frcp_rn(scale ? __ldg(scale) : 1.0f);
+    sl8::pdl_wait();
+    sl8::pdl_release();
+    const float inv = __frcp_rn(scale ? sl8::ld_f32(scale) : 1.0f);
     const float inv_n = 1.0f / static_cast<float>(cols);
     constexpr int NC = CHUNKS > 0 ? CHUNKS : 1;
     for (long long r = warp; r < rows; r += warps) {
@@ -524,11 +534,11 @@ __global__ void __launch_bounds__(256, 3) layernorm_quantize_kernel(const T* __r
 }
 
 template <typename T>
-void launch_layernorm(int grid, cudaStream_t s, const T* x, long long rows, int cols, long long ld, const float* gamma,
+cudaError_t launch_layernorm(int grid, cudaStream_t s, const T* x, long long rows, int cols, long long ld, const float* gamma,
                       const float* beta, float eps, const float* scale, uint8_t* out, long long ld_out) {
-    if (cols <= 1280) layernorm_quantize_kernel<T, 5><<<grid, 256, 0, s>>>(x, rows, cols, ld, gamma, beta, eps, scale, out, ld_out);
-    else if (cols <= 2048) layernorm_quantize_kernel<T, 8><<<grid, 256, 0, s>>>(x, rows, cols, ld, gamma, beta, eps, scale, out, ld_out);
-    else layernorm_quantize_kernel<T, 0><<<grid, 256, 0, s>>>(x, rows, cols, ld, gamma, beta, eps, scale, out, ld_out);
+    if (cols <= 1280) return sl8_launch_chained(layernorm_quantize_kernel<T, 5>, grid, 256, 0, s, x, rows, cols, ld, gamma, beta, eps, scale, out, ld_out);
+    if (cols <= 2048) return sl8_launch_chained(layernorm_quantize_kernel<T, 8>, grid, 256, 0, s, x, rows, cols, ld, gamma, beta, eps, scale, out, ld_out);
+    return sl8_launch_chained(layernorm_quantize_kernel<T, 0>, grid, 256, 0, s, x, rows, cols, ld, gamma, beta, eps, scale, out, ld_out);
 }
 
 }  // namespace
@@ -547,11 +557,11 @@ SL8_API int sl8_layernorm_quantize_e4m3(sl8_handle_t h, const void* x, int dtype
     if (!guard.ok) return fail(h, SL8_ERR_CUDA, "cudaSetDevice failed");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int grid = prep_grid(h, rows * 32);            // one warp per row, eight warps per block
+    cudaError_t e;
     if (dtype == SL8_DT_F32)
-        launch_layernorm<float>(grid, s, static_cast<const float*>(x), rows, cols, ld, gamma, beta, eps, scale, static_cast<uint8_t*>(out), ld_out);
+        e = launch_layernorm<float>(grid, s, static_cast<const float*>(x), rows, cols, ld, gamma, beta, eps, scale, static_cast<uint8_t*>(out), ld_out);
     else
-        launch_layernorm<__nv_bfloat16>(grid, s, static_cast<const __nv_bfloat16*>(x), rows, cols, ld, gamma, beta, eps, scale,
+        e = launch_layernorm<__nv_bfloat16>(grid, s, static_cast<const __nv_bfloat16*>(x), rows, cols, ld, gamma, beta, eps, scale,
                                         static_cast<uint8_t*>(out), ld_out);
-    cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? SL8_OK : fail_cuda(h, e, "layernorm kernel launch");
 }

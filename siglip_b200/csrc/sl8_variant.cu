@@ -21,13 +21,15 @@ cudaError_t launch_one(const CUtensorMap* map_a, const CUtensorMap* map_b, const
     cfg.blockDim = dim3(T::THREADS, 1, 1);
     cfg.dynamicSmemBytes = T::SMEM_BYTES;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CG;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, sl8_gemm_kernel<CG, TN, TK, STAGES, EW, OP, OUT, NBUF>, *map_a, *map_b, *map_bt, *map_d, *map_s, *params);
 }
 

@@ -1,0 +1,54 @@
+"""Kernels that become resident while the one ahead of them on the stream still runs: calls that reuse each other's buffers,
+issued back to back and from a captured graph, must give bit for bit what they give with a synchronisation after each."""
+import pytest
+import torch
+
+from siglip_b200 import synth
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _chain(eng, rows, d, ff, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    weight = lambda n, k: synth.quantize_e4m3(torch.randn((n, k), generator=g, device=DEV) * 0.05)[0]
+    codes = lambda cols: torch.zeros((rows, synth.pitch128(cols)), dtype=torch.uint8, device=DEV)[:, :cols]
+    one, scale = torch.ones(1, device=DEV), torch.full((1,), 0.02, device=DEV)
+    wq, w1, w2 = weight(d, d), weight(ff, d), weight(d, ff)
+    x0 = torch.randn((rows, d), generator=g, device=DEV).to(torch.bfloat16)
+    pixels = torch.rand((1, 3, 64, 64), generator=g, device=DEV)
+    x, y, a, hidden, patches = x0.clone(), torch.empty_like(x0), codes(d), codes(ff), codes(768)[:16]
+
+    def run(step):
+        """x -> two rounds of LayerNorm / projection / MLP that overwrite a, hidden, x and y while their readers may still run."""
+        for buf, out in ((x, y), (y, x)):
+            eng.layernorm_quantize(buf, None, None, 1e-6, scale, out=a); step()
+            eng.fc2_residual(a, wq, None, buf, scale_a=one, scale_b=scale, out=out); step()
+            _, s = eng.amax_scale(out); step()
+            eng.quantize_e4m3(out, s, out=a); step()
+            eng.fc1_gelu(a, w1, None, scale_a=s, scale_b=scale, out_scale=one, out=hidden); step()
+            eng.patchify_quantize(pixels, 16, one, out=patches); step()
+            eng.fc2_residual(hidden, w2, None, out, scale_a=one, scale_b=scale, out=buf); step()
+
+    return run, (x, y, a, hidden, patches), x0
+
+
+@pytest.mark.parametrize("rows,d,ff", [(100, 256, 512), (729, 1152, 4304), (5003, 768, 3072)])
+def test_back_to_back_and_captured_calls_match_synchronised_ones(engine, rows, d, ff):
+    run, state, x0 = _chain(engine, rows, d, ff, seed=rows)
+    run(torch.cuda.synchronize)
+    want = [t.clone() for t in state]
+    same = lambda: all(torch.equal(t.contiguous().view(torch.uint8), w.contiguous().view(torch.uint8)) for t, w in zip(state, want))
+    for _ in range(5):
+        state[0].copy_(x0)
+        run(lambda: None)
+        assert same()
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        state[0].copy_(x0)
+        run(lambda: None)
+    for _ in range(5):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert same()
