@@ -505,7 +505,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         __syncthreads();
     }
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_ptr;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
     // Everything above (barriers, tensor memory, descriptors) runs beside the tail of the kernel ahead on the stream.  No
     // two GEMM CTAs share an SM (each takes more than half its shared memory), so the next GEMM's CTAs move in as these leave.
     pdl_wait();
@@ -594,17 +594,19 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         __syncwarp();
     } else if (warp == 1) {
         // ===== MMA issuer (leader CTA only) =====
-        // One thread.  Measured on B200: issuing one tcgen05.mma holds the thread for ~108 cycles and the MMA
-        // (M 256, N 256, K 32) itself takes 128, so whatever else this thread executes per k-block (~290 cycles
-        // for wait + commit + loop control when written naively) decides whether the tensor pipe idles.  Hence:
-        // the poll of the NEXT stage's barrier is issued before this stage's MMAs and read after them (the
-        // blocking wait runs only if that look-ahead failed), and k-blocks are taken several per loop iteration.
-        if (lane == 0 && cta_rank == 0) {
+        // The whole warp walks the loop and one elected lane issues: a tcgen05.mma takes its descriptors from uniform
+        // registers, and in a branch that only one lane takes each of them is moved there instruction by instruction, which
+        // cost ~110 cycles per MMA -- hidden behind the 128 cycles of a 256-column tile, but twice what a 128-column tile
+        // needs (1152-wide FC2 at 729 rows on 128 x 128 tiles 14.5 -> 11.6 us; at 46 656 rows on 256 x 256 tiles 193 -> 186).  What else the loop executes per
+        // k-block counts too: the poll of the NEXT stage's barrier is issued before this stage's MMAs and read after them
+        // (the blocking wait runs only if that look-ahead failed), and k-blocks are taken several per loop iteration.
+        if (cta_rank == 0) {
             const uint32_t idesc_full = make_idesc_e4m3_f32(T::TILE_M_CTA * CG, TN);
             const uint32_t idesc_tail = make_idesc_e4m3_f32(T::TILE_M_CTA * CG, p.tail_cols);   // the last, narrower N tile
             uint32_t idesc = idesc_full;
             // Descriptors differ between stages, atoms and K steps only in the 14-bit start-address
             // field: +2 there = 32 bytes = one K = 32 step inside the 128-byte row.
+            const auto all_ok = [](bool lane_ok) { return __all_sync(0xffffffffu, lane_ok) != 0; };
             const uint64_t adesc0 = make_kmajor_sw128_desc(base);
             const uint64_t bdesc0 = make_kmajor_sw128_desc(base + T::A_BYTES);
             constexpr uint32_t STAGE_DESC = T::STAGE_BYTES >> 4;
@@ -620,6 +622,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             uint32_t ready = 0;      // look-ahead: the barrier of `stage` was already seen complete
 
             // All MMAs of one full k-block held in `st`; `fresh` = this k-block starts a tile (overwrite D).
+            // (only inside `if (elect_one())`, which picks the same lane every time: a commit covers the MMAs its own thread issued)
             auto issue_full = [&](uint32_t d_tmem, int st, bool fresh) {
                 const uint64_t adesc = adesc0 + static_cast<uint32_t>(st) * STAGE_DESC;
                 const uint64_t bdesc = bdesc0 + static_cast<uint32_t>(st) * STAGE_DESC;
@@ -638,7 +641,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             for (int tile = cluster_id; ok && tile < p.num_tiles; tile += num_clusters) {
                 wc.tile = tile;
                 long long t0 = prof_any ? clock64() : 0;     // once per tile: timed in the coarse mode too
-                ok = wait_bar<SL8_SPIN_CRITICAL>(tempty_bar0 + 8 * acc, acc_phase ^ 1u, wc, ST_MMA_TMEM_EMPTY_WAIT, acc);
+                ok = all_ok(wait_bar<SL8_SPIN_CRITICAL>(tempty_bar0 + 8 * acc, acc_phase ^ 1u, wc, ST_MMA_TMEM_EMPTY_WAIT, acc));
                 if (prof_any) t_tmem += clock64() - t0;
                 n_tiles++;
                 if (!ok) break;
@@ -653,15 +656,16 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     auto step = [&](bool fresh, int n) -> bool {
                         if (!ready) {      // the look-ahead saw the stage still filling: counted, then waited for
                             t_full++;
-                            if (!wait_bar<SL8_SPIN_CRITICAL>(full_bar0 + 8 * stage, phase, wc, ST_MMA_FULL_WAIT, stage)) return false;
+                            if (!all_ok(wait_bar<SL8_SPIN_CRITICAL>(full_bar0 + 8 * stage, phase, wc, ST_MMA_FULL_WAIT, stage))) return false;
                         }
                         const int s1 = (stage + 1 == STAGES) ? 0 : stage + 1;
                         const uint32_t ph1 = (s1 == 0) ? (phase ^ 1u) : phase;
                         const uint32_t r1 = mbar_test_wait(full_bar0 + 8 * s1, ph1);
                         tc_fence_after();
-                        if (n == 4 * T::KATOMS) {
+                        if (elect_one()) {
+                          if (n == 4 * T::KATOMS) {
                             issue_full(d_tmem, stage, fresh);
-                        } else {
+                          } else {
                             const uint64_t adesc = adesc0 + static_cast<uint32_t>(stage) * STAGE_DESC;
                             const uint64_t bdesc = bdesc0 + static_cast<uint32_t>(stage) * STAGE_DESC;
 #pragma unroll
@@ -670,11 +674,13 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                                 const uint32_t ob = (j >> 2) * (T::B_ATOM_BYTES >> 4) + 2 * (j & 3);
                                 if (j < n) mma_f8<CG>(d_tmem, adesc + o, bdesc + ob, idesc, (j == 0 && fresh) ? 0u : 1u);
                             }
+                          }
+                          release_stage(stage);
                         }
-                        release_stage(stage);
+                        __syncwarp();
                         stage = s1;
                         phase = ph1;
-                        ready = r1;
+                        ready = all_ok(r1 != 0u) ? 1u : 0u;
                         return true;
                     };
                     for (; ok && kb + 2 <= k_full; kb += 2) {      // two k-blocks per loop iteration
@@ -693,19 +699,20 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 }
                 for (; kb < p.k_blocks; kb++) {
                     if (prof) t0 = clock64();
-                    if (!ready) ok = wait_bar<SL8_SPIN_CRITICAL>(full_bar0 + 8 * stage, phase, wc, ST_MMA_FULL_WAIT, stage);
+                    if (!ready) ok = all_ok(wait_bar<SL8_SPIN_CRITICAL>(full_bar0 + 8 * stage, phase, wc, ST_MMA_FULL_WAIT, stage));
                     if (prof) t_full += clock64() - t0;
                     if (!ok) break;
                     const int s1 = (stage + 1 == STAGES) ? 0 : stage + 1;
                     const uint32_t ph1 = (s1 == 0) ? (phase ^ 1u) : phase;
-                    ready = mbar_test_wait(full_bar0 + 8 * s1, ph1);
+                    ready = all_ok(mbar_test_wait(full_bar0 + 8 * s1, ph1) != 0u) ? 1u : 0u;
                     tc_fence_after();
                     long long t1 = prof ? clock64() : 0;
                     if (SL8_DBG(p.flags, DBG_SKIP_MMA)) {
                         // measurement aid: stages are released at once, the loads run at their own pace
-                    } else if (kb < k_full) {
+                    } else if (elect_one()) {
+                      if (kb < k_full) {
                         issue_full(d_tmem, stage, kb == 0);
-                    } else {
+                      } else {
                         const uint64_t adesc = adesc0 + static_cast<uint32_t>(stage) * STAGE_DESC;
                         const uint64_t bdesc = bdesc0 + static_cast<uint32_t>(stage) * STAGE_DESC;
                         for (int j = 0; j < p.last_kblock_mmas; j++) {
@@ -713,20 +720,26 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                             const uint32_t ob = (j >> 2) * (T::B_ATOM_BYTES >> 4) + 2 * (j & 3);
                             mma_f8<CG>(d_tmem, adesc + o, bdesc + ob, idesc, (kb | j) != 0 ? 1u : 0u);
                         }
+                      }
                     }
+                    __syncwarp();
                     if (prof) { const long long t2 = clock64(); t_mma += t2 - t1; t1 = t2; }
-                    release_stage(stage);
+                    if (elect_one()) release_stage(stage);
+                    __syncwarp();
                     if (prof) t_commit += clock64() - t1;
                     stage = s1;
                     phase = ph1;
                 }
                 if (!ok) break;
-                if constexpr (CG == 2) mma_commit_pair(tfull_bar0 + 8 * acc, 0x3);
-                else mma_commit(tfull_bar0 + 8 * acc);
+                if (elect_one()) {
+                    if constexpr (CG == 2) mma_commit_pair(tfull_bar0 + 8 * acc, 0x3);
+                    else mma_commit(tfull_bar0 + 8 * acc);
+                }
+                __syncwarp();
                 if (p.flags & FLAG_SINGLE_ACC) acc_phase ^= 1u;
                 else { acc ^= 1; if (acc == 0) acc_phase ^= 1u; }
             }
-            if (prof_any) {
+            if (prof_any && lane == 0) {
                 long long* slot = p.prof + static_cast<size_t>(blockIdx.x) * PROF_SLOTS;
                 slot[PROF_MMA_WAIT_FULL] = t_full;
                 slot[PROF_MMA_WAIT_TMEM] = t_tmem;
