@@ -6,6 +6,8 @@ import numpy as np
 import pytest
 import torch
 
+from tests.tolerance import check_e4m3
+
 DEV = "cuda"
 
 
@@ -234,3 +236,39 @@ def test_layernorm_quantize_feeds_fc1(engine, oracle):
     ref = oracle.fc1_gelu(np.ascontiguousarray(A.cpu().numpy()), p.B.cpu().numpy(), float(scale.item()), p.scale_b,
                           p.bias.view(torch.uint16).cpu().numpy())
     check_bf16(D.view(torch.uint16).cpu().numpy(), ref, "layernorm -> fc1")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(40, 8), (3, 768), (7200, 768), (7200, 776), (3, 1280), (50, 1288), (1300, 1792), (50, 1800),
+                                       (1300, 2048), (50, 2056)])     # edges of the widths kept in registers; more rows than warps x ring
+def test_layernorm_widths_on_gpu(engine, oracle, dtype, rows, cols):
+    rng = np.random.default_rng(rows + cols)
+    x = torch.from_numpy((rng.standard_normal((rows, cols + 8)) * 2 + 0.5).astype(np.float32)).to(dtype).to(DEV)[:, :cols]     # pitch != width
+    gamma, beta = rng.standard_normal((2, cols)).astype(np.float32)
+    for g, b in ((gamma, beta), (None, None)):
+        out = engine.layernorm_quantize(x, None if g is None else torch.from_numpy(g).to(DEV), None if b is None else torch.from_numpy(b).to(DEV),
+                                        1e-6, torch.tensor([0.02], device=DEV))
+        want = oracle.layernorm_quantize(np.ascontiguousarray(x.float().cpu().numpy()), np.ones(cols) if g is None else g,
+                                         np.zeros(cols) if b is None else b, 1e-6, 0.02)
+        check_e4m3(out.cpu().numpy(), want, f"layernorm {rows}x{cols}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols,pad", [(1, 8, 0), (2105, 1152, 0), (2106, 1152, 8), (5000, 1160, 0), (70000, 40, 8), (3000, 1155, 5)])
+def test_amax_and_quantize_walks_on_gpu(engine, oracle, dtype, rows, cols, pad):
+    """One vector per thread, four, several batches per block; rows that are cut by a pitch; the element-by-element path."""
+    rng = np.random.default_rng(rows)
+    x = torch.from_numpy((rng.standard_normal((rows, cols + pad)) * 3).astype(np.float32)).to(dtype)
+    x[:, cols:] = 1e4                                                   # what lies between the rows must not count
+    x[rows - 1, cols - 1] = -77.0
+    xd, xs = x.to(DEV)[:, :cols], np.ascontiguousarray(x[:, :cols].float().numpy())
+    amax, scale = engine.amax_scale(xd)
+    assert float(amax) == 77.0 and float(scale) == float(np.float32(77.0) / np.float32(448.0))
+    out = engine.quantize_e4m3(xd, scale)
+    assert np.array_equal(out.cpu().numpy(), oracle.quantize_rows(xs, float(scale)))
+    both = torch.full((1,), 5.0, device=DEV)                            # the scale in the word of the abs-max
+    assert engine._lib.sl8_amax_scale(engine._h, xd.data_ptr(), engine._dt(xd), rows, cols, xd.stride(0), both.data_ptr(), both.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert float(both) == float(scale)
