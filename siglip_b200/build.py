@@ -4,7 +4,8 @@
 
 Every kernel configuration of ``csrc/sl8_variants.h`` is one translation unit
 (``sl8_variant.cu`` compiled with ``-DSL8_VARIANT_ID=<id>``), so they compile in
-parallel; ``sl8_api.cu`` holds the C ABI.  The result is ``siglip_b200/lib/libsiglip_fp8.so``.
+parallel; ``sl8_api.cu`` holds the C ABI.  The result is ``siglip_b200/lib/libsiglip_fp8.so``; beside it
+``sl8_torch.so`` (``sl8_torch.cpp``) takes torch tensors to that ABI.
 nvcc cross-compiles without a GPU.  This is the build-system counterpart of the
 reference's Makefile (Makefile:1-28: one nvcc line per layer binary).
 """
@@ -23,6 +24,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "lib" / "obj"
 LIB = PKG / "lib" / "libsiglip_fp8.so"
+BINDING = PKG / "lib" / "sl8_torch.so"     # torch tensors -> C ABI (imported by lib.py)
 BENCH = PKG / "lib" / "siglip_bench"      # per-layer bench host speaking the reference harness's @@RESULT protocol
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -51,7 +53,7 @@ def variant_ids() -> list[int]:
 
 
 def sources_mtime() -> float:
-    files = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))
+    files = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cpp")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))
     files.append(PKG.parent / "include" / "siglip_fp8.h")
     return max(f.stat().st_mtime for f in files)
 
@@ -67,9 +69,27 @@ def compile_one(args: tuple[list[str], Path, bool]) -> str:
     return res.stderr
 
 
+def binding_compile(obj: Path) -> list[str]:
+    import sysconfig
+    import torch
+    inc = Path(torch.__file__).parent / "include"
+    cuda = Path(nvcc()).resolve().parent.parent / "include"
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-I{inc}",
+            f"-I{inc / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{cuda}", f"-I{sysconfig.get_paths()['include']}",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-c", str(CSRC / "sl8_torch.cpp"), "-o", str(obj)]
+
+
+def binding_link(obj: Path) -> list[str]:
+    import torch
+    libs = Path(torch.__file__).parent / "lib"
+    return [os.environ.get("CXX", "g++"), "-shared", "-o", str(BINDING), str(obj), f"-L{LIB.parent}", "-lsiglip_fp8", f"-L{libs}",
+            "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"]
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     """Compiles what is out of date and returns the path of the shared library."""
-    if LIB.exists() and BENCH.exists() and not force and min(LIB.stat().st_mtime, BENCH.stat().st_mtime) >= sources_mtime():
+    products = (LIB, BINDING, BENCH)
+    if not force and all(f.exists() for f in products) and min(f.stat().st_mtime for f in products) >= sources_mtime():
         return LIB
     OBJ.mkdir(parents=True, exist_ok=True)
     for stale in list(OBJ.glob("variant_*.o")) + list(OBJ.glob("variant_*.log")):
@@ -86,9 +106,15 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         o = OBJ / f"{name}.o"
         objs.append(o)
         jobs.append(([exe, *NVCC_FLAGS, "-c", str(CSRC / f"sl8_{name}.cu"), "-o", str(o)], OBJ / f"{name}.log", verbose))
+    binding = OBJ / "torch.o"
+    jobs.append((binding_compile(binding), OBJ / "torch.log", verbose))
     with cf.ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as pool:
         list(pool.map(compile_one, jobs))
     link = [exe, *ARCH_FLAGS, "-shared", "-o", str(LIB), *map(str, objs), "-cudart", "static"]
+    res = subprocess.run(link, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"link failed: {' '.join(link)}\n{res.stdout}\n{res.stderr}")
+    link = binding_link(binding)
     res = subprocess.run(link, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed: {' '.join(link)}\n{res.stdout}\n{res.stderr}")

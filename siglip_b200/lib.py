@@ -6,10 +6,14 @@ The library is looked up in-tree (``siglip_b200/lib/libsiglip_fp8.so``, produced
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 from pathlib import Path
 
 _LIB_PATH = Path(__file__).resolve().parent / "lib" / "libsiglip_fp8.so"
+_BINDING_PATH = _LIB_PATH.parent / "sl8_torch.so"
 _lib = None
+_binding = None
 
 SL8_OK = 0
 SL8_ERR_INVALID_VALUE = -1
@@ -103,3 +107,17 @@ def load_library() -> C.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+def load_binding():
+    """The extension module that takes torch tensors to the entry points of libsiglip_fp8.so (csrc/sl8_torch.cpp)."""
+    global _binding
+    if _binding is None:
+        if not _BINDING_PATH.exists():
+            raise SL8Error(SL8_ERR_CUDA, f"{_BINDING_PATH} is missing: run `python -m siglip_b200.build`; there is no fallback path")
+        loader = importlib.machinery.ExtensionFileLoader("sl8_torch", str(_BINDING_PATH))
+        spec = importlib.util.spec_from_file_location("sl8_torch", str(_BINDING_PATH), loader=loader)
+        module = importlib.util.module_from_spec(spec)
+        loader.exec_module(module)
+        _binding = module
+    return _binding
