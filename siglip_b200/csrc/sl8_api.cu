@@ -54,28 +54,69 @@ inline int fail_cuda(sl8_handle_t h, cudaError_t e, const char* what) { return s
 inline bool aligned16(const void* p) { return sl8_aligned16(p); }
 
 // ---- dispatch -------------------------------------------------------------------------
-// The table is generated from a sweep on B200 (python -m siglip_b200.sweep); shapes it does not hold fall back
-// to rules (one line per rule; the first match wins).
+// The table is generated from a sweep on B200 (python -m siglip_b200.sweep); what it does not hold is answered by a cost model.
 int kernel_slot(int op, int out_dtype) {
     if (op == SL8_OP_PATCH_EMBED) return sl8::K_PE;
     if (op == SL8_OP_FC2_RESIDUAL) return sl8::K_FC2;
     return out_dtype == SL8_OUT_E4M3 ? sl8::K_FC1_E4M3 : sl8::K_FC1_BF16;
 }
 
-int pick_variant_exact_gelu(int op, int out_dtype, long long M, int N, int K);
+// What a launch takes with a variant, in microseconds: its CTAs (or pairs) go through ceil(tiles / CTAs) rounds of tiles;
+//     start + k_blocks * first + (rounds - 1) * max(k_blocks * next, tile)
+// `start` is set-up, the first operands' way in and the last tile's epilogue; `first` a k-block of the first tile; a later tile
+// hides its mainloop (`next` per k-block, more than `first` when every SM asks L2) behind the epilogue ahead of it or the
+// other way round (`tile`: the epilogue's own pace).  The constants are fitted so that the cheapest variant by the formula is
+// the fastest one measured, over 18 (layer, N, K) from 512 to 4 800 wide and 50 to 186 624 rows (graph replays, every
+// variant): it is within 1 % of the fastest on average, 9 % at worst.  What it decides: 128 x 128 tiles on single CTAs with
+// eight epilogue warps (18) while there are few tiles (an epilogue half as long at the end: FC1 4 304 x 1 152 at 512 rows
+// 10.0 us with v3, 7.4 with v18; FC2 1 152 x 1 152 at 2 048 rows 10.2 with v1, 7.4); 256 x 128 pairs (19) where
+// 256 x 256 tiles leave most of the last round empty (FC2 1 152 x 4 304 at 3 700 rows 25.2 -> 20.7); eight epilogue warps
+// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 52.2 with v1, 39.1 with v17).
+enum CostClass : int { COST_GELU, COST_TANH, COST_NONE, COST_FC2, COST_PE };
+struct VariantCost {
+    CostClass cls;
+    int variant;
+    float start, first, next, tile;
+};
+const VariantCost kVariantCost[] = {
+    {COST_GELU, 18, 4.48f, 0.225f, 0.331f, 2.69f},
+    {COST_GELU, 15, 7.02f, 0.361f, 0.438f, 3.67f},
+    {COST_GELU, 14, 6.46f, 0.404f, 0.444f, 3.69f},
+    {COST_TANH, 18, 4.67f, 0.192f, 0.331f, 2.27f},
+    {COST_TANH, 3, 6.75f, 0.300f, 0.450f, 3.64f},
+    {COST_TANH, 15, 5.68f, 0.412f, 0.450f, 3.31f},
+    {COST_NONE, 18, 4.07f, 0.200f, 0.378f, 1.26f},
+    {COST_NONE, 3, 5.25f, 0.283f, 0.474f, 2.57f},
+    {COST_NONE, 2, 5.74f, 0.279f, 0.423f, 2.75f},
+    {COST_NONE, 1, 5.94f, 0.274f, 0.416f, 4.22f},
+    {COST_FC2, 18, 4.55f, 0.221f, 0.363f, 2.00f},
+    {COST_FC2, 19, 4.86f, 0.210f, 0.276f, 3.12f},
+    {COST_FC2, 3, 6.18f, 0.312f, 0.426f, 6.32f},
+    {COST_FC2, 17, 6.42f, 0.308f, 0.456f, 3.87f},
+    {COST_FC2, 1, 6.38f, 0.338f, 0.390f, 5.57f},
+    {COST_PE, 18, 4.92f, 0.177f, 0.383f, 2.22f},
+    {COST_PE, 17, 6.74f, 0.257f, 0.574f, 2.88f},
+};
 
-// The sweep and the rules below are for the full epilogues.  An FC1 call whose epilogue is light (no activation: the
-// Q / K / V projections; or the one-SFU-operation GELU) does not need sixteen epilogue warps to hide the SFU chain and
-// runs faster on eight with the same ring depth (So400m FC1 shape, 46 656 rows: 198 against 220 us without activation,
-// 207 against 221 us with the hardware tanh).
-int pick_variant(int op, int out_dtype, long long M, int N, int K, unsigned flags) {
-    const int v = pick_variant_exact_gelu(op, out_dtype, M, N, K);
-    if (op == SL8_OP_FC1_GELU && (flags & (SL8_FLAG_NO_ACTIVATION | SL8_FLAG_GELU_HW_TANH)) && variant(v) && variant(v)->epi_warps == 16)
-        return 2;
-    return v;
+int cheapest_variant(CostClass cls, int slot, long long M, int N, int K) {
+    int best = 1;
+    float best_us = 3.4e38f;
+    for (const VariantCost& c : kVariantCost) {
+        const VariantEntry* v = c.cls == cls ? variant(c.variant) : nullptr;
+        if (!v || !v->kernel[slot]) continue;
+        const long long tiles = ((M + 128 * v->cg - 1) / (128 * v->cg)) * ((N + v->tn - 1) / v->tn), ctas = 148 / v->cg;
+        const float rounds = static_cast<float>((tiles + ctas - 1) / ctas), k_blocks = static_cast<float>((K + 127) / 128);
+        const float later = k_blocks * c.next > c.tile ? k_blocks * c.next : c.tile;
+        const float us = c.start + k_blocks * c.first + (rounds - 1.0f) * later;
+        if (us < best_us) best_us = us, best = c.variant;
+    }
+    return best;
 }
 
-int pick_variant_exact_gelu(int op, int out_dtype, long long M, int N, int K) {
+int pick_variant(int op, int out_dtype, long long M, int N, int K, unsigned flags) {
+    const int slot = kernel_slot(op, out_dtype);
+    if (op == SL8_OP_FC1_GELU && (flags & SL8_FLAG_NO_ACTIVATION)) return cheapest_variant(COST_NONE, slot, M, N, K);
+    if (op == SL8_OP_FC1_GELU && (flags & SL8_FLAG_GELU_HW_TANH)) return cheapest_variant(COST_TANH, slot, M, N, K);
     // A (layer, N, K) the committed sweep covers: the row with the largest m_min <= M decides.
     int swept = -1;
     long long swept_m = -1;
@@ -87,20 +128,8 @@ int pick_variant_exact_gelu(int op, int out_dtype, long long M, int N, int K) {
         }
     }
     // (the sweep times bf16 outputs; a variant that has no kernel for this output type is passed over)
-    if (swept >= 0 && swept < SL8_NUM_VARIANTS && variant(swept) && variant(swept)->kernel[kernel_slot(op, out_dtype)]) return swept;
-    // Any other shape: the rules the sweeps suggest.
-    const long long tiles256 = ((M + 255) / 256) * ((N + 255) / 256);
-    if (tiles256 < 37) {
-        // Fewer 256 x 256 tiles than half the CTA pairs (M sweep: M = 729 .. 1458 at the So400m shapes):
-        // 128 x 128 tiles on single CTAs give more of the 148 SMs work.
-        return 6;
-    }
-    // A tcgen05.mma of a CTA pair takes about 150 cycles whatever its N (measured for N = 128, 192,
-    // 256), so the widest tile does the most work per instruction even where N = 1152 leaves the
-    // fifth 256-wide tile half empty.
-    if (op == SL8_OP_FC1_GELU) return 15;     // GELU epilogue: four epilogue warps per scheduler
-    if (op == SL8_OP_PATCH_EMBED) return 17;  // short K: eight epilogue warps, three staging boxes per column group, four stages
-    return 1;
+    if (swept >= 0 && swept < SL8_NUM_VARIANTS && variant(swept) && variant(swept)->kernel[slot]) return swept;
+    return cheapest_variant(op == SL8_OP_PATCH_EMBED ? COST_PE : op == SL8_OP_FC2_RESIDUAL ? COST_FC2 : COST_GELU, slot, M, N, K);
 }
 
 struct Problem {

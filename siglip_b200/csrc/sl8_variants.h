@@ -37,9 +37,11 @@
     X(14, 2, 256, 128, 4, 16, 1)  \
     X(15, 2, 256, 128, 5, 16, 1) \
     X(16, 2, 256, 128, 6, 4, 2)  \
-    X(17, 2, 256, 128, 4, 8, 3)
+    X(17, 2, 256, 128, 4, 8, 3)  \
+    X(18, 1, 128, 128, 4, 8, 2)  \
+    X(19, 2, 128, 128, 6, 8, 2)
 
-#define SL8_NUM_VARIANTS 18
+#define SL8_NUM_VARIANTS 20
 
 namespace sl8 {
 

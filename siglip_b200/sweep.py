@@ -4,7 +4,8 @@ Counterpart of the reference's ``tools/grid_search.py`` (constraint pruning ``:8
 parsing ``:124-151``, per-configuration timeout, CSV ``:170-251``) for the run-time variants of this library:
 instead of recompiling one binary per macro combination it walks the compiled variant list
 (``siglip_b200/csrc/sl8_variants.h``) through ``sl8_set_variant``, times every admissible variant on the
-seeded synthetic operands of ``siglip_b200/synth.py`` over an M ladder, writes one CSV row per
+seeded synthetic operands of ``siglip_b200/synth.py`` over an M ladder (four points per octave up to 16 images: a few
+rows more can cost a whole round of tiles) from captured graphs (a Python loop takes longer than a small layer), writes one CSV row per
 (layer, shape, variant) and turns the CSV into the table ``pick_variant`` (``sl8_api.cu``) consults:
 ``siglip_b200/csrc/sl8_dispatch_table.h``.
 
@@ -80,7 +81,8 @@ def best_rows(rows: list[dict], keep_margin: float = 0.02) -> list[dict]:
 
     Per (op, N, K) the M ladder is walked upwards; the winner of the previous (smaller) M is kept unless
     another variant beats it by more than ``keep_margin`` (noise must not flip the table), and neighbouring
-    M with the same winner collapse into one row whose ``m_min`` is the smallest of them (0 for the first)."""
+    M with the same winner collapse into one row whose ``m_min`` is the smallest of them (0 for the first).  At the
+    smallest M a single-CTA variant within 3 % of the best is taken: a CTA pair waits for two free SMs side by side."""
     groups: dict[tuple, dict[int, list[dict]]] = {}
     for r in rows:
         if r["status"] != "ok":
@@ -93,6 +95,9 @@ def best_rows(rows: list[dict], keep_margin: float = 0.02) -> list[dict]:
             cands = sorted(by_m[m], key=lambda r: float(r["ms_median"]))
             best = cands[0]
             choice = int(best["variant"])
+            if prev is None:
+                choice = next((int(r["variant"]) for r in cands if str(r.get("cta_group")) == "1"
+                               and float(r["ms_median"]) <= float(best["ms_median"]) * 1.03), choice)
             if prev is not None and prev != choice:
                 mine = [r for r in cands if int(r["variant"]) == prev]
                 if mine and float(mine[0]["ms_median"]) <= float(best["ms_median"]) * (1.0 + keep_margin):
@@ -126,26 +131,37 @@ def read_csv(path: Path) -> list[dict]:
 
 
 # ----------------------------------------------------------------------------- timing (GPU)
-def time_variant(eng, go, repeats: int, iters: int) -> list[float]:
+def ladder(per_image: int, octaves: int, per_octave: int) -> list[int]:
+    """per_image * 2^j; below 16 images, where the last round of tiles weighs, also the points that divide an octave into per_octave."""
+    return [(per_image << j) + (per_image << j) * q // per_octave for j in range(octaves) for q in range(per_octave if j < min(4, octaves - 1) else 1)]
+
+
+def capture(go, iters: int, stream):
+    """A graph of `iters` launches."""
     import torch
-    out = []
-    go()
-    torch.cuda.synchronize()
-    for _ in range(repeats):
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
+    with torch.cuda.stream(stream):
+        go()
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
         for _ in range(iters):
             go()
-        e1.record()
-        torch.cuda.synchronize()
-        out.append(e0.elapsed_time(e1) / iters)
-    eng.device_status()
-    return out
+    return graph
+
+
+def replay_ms(graph, iters: int) -> float:
+    import torch
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()
+    graph.replay()
+    e1.record()
+    torch.cuda.synchronize()
+    return e0.elapsed_time(e1) / iters
 
 
 def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out_path: Path, variants_only=None,
-              max_rows: int | None = None, log=print) -> list[dict]:
-    """Times every admissible variant on every (layer, N, K) of the named shape sets for M = rows_per_image * 2^j."""
+              max_rows: int | None = None, log=print, per_octave: int = 1) -> list[dict]:
+    """Times every admissible variant on every (layer, N, K) of the named shape sets over the M ladder."""
     import torch
     import siglip_b200
     from siglip_b200 import build, layers, synth
@@ -153,6 +169,7 @@ def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out
 
     dev = "cuda"
     eng = siglip_b200.Engine(0)
+    stream = torch.cuda.Stream()
     resources = parse_resources(build.resource_report())
     all_variants = [dict(layers.describe_variant(v), variant_id=v) for v in range(layers.num_variants())]
     rows = []
@@ -163,8 +180,7 @@ def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out
         for set_name in shape_sets:
             for op_name, n, k, per_image in SHAPE_SETS[set_name]:
                 op = OPS[op_name]
-                for j in range(m_steps):
-                    m = per_image * (1 << j)
+                for m in ladder(per_image, m_steps, per_octave):
                     if max_rows is not None and m > max_rows:
                         break
                     if op == 0:
@@ -204,19 +220,23 @@ def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out
                              if variants_only is None or v["variant_id"] in variants_only]
                     samples = {v["variant_id"]: [] for v in cands}
                     status = {v["variant_id"]: "ok" for v in cands}
-                    for rnd in range(repeats + 1):               # round 0 warms up and is not recorded
+                    graphs = {}
+                    for rnd in range(repeats + 1):               # round 0 captures and warms up and is not recorded
                         for v in cands:
                             vid = v["variant_id"]
                             if status[vid] != "ok":
                                 continue
                             try:
-                                eng.set_variant(vid)
-                                ms = time_variant(eng, go, 1, iters if rnd else 3)
+                                if rnd == 0:
+                                    eng.set_variant(vid)
+                                    graphs[vid] = capture(go, iters, stream)
+                                ms = replay_ms(graphs[vid], iters)
+                                eng.device_status()
                                 if rnd:
-                                    samples[vid] += ms
+                                    samples[vid].append(ms)
                             except SL8Error as e:        # a bounded device wait ran out, or the variant refused the shape
                                 status[vid] = "timeout" if "TIMEOUT" in str(e).upper() else "error"
-                                eng = siglip_b200.Engine(0)
+                    del graphs
                     for v in cands:
                         vid = v["variant_id"]
                         res = resources.get((vid, op, 0), {})
@@ -250,7 +270,8 @@ def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out
 def main(argv=None) -> int:
     ap = argparse.ArgumentParser(description=__doc__, formatter_class=argparse.RawDescriptionHelpFormatter)
     ap.add_argument("--shapes", default="so400m,b16", help="comma-separated shape sets: " + ", ".join(SHAPE_SETS))
-    ap.add_argument("--m-steps", type=int, default=11, help="M = rows_per_image * 2^j for j < m-steps")
+    ap.add_argument("--m-steps", type=int, default=11, help="M from rows_per_image to rows_per_image * 2^(m-steps - 1)")
+    ap.add_argument("--per-octave", type=int, default=4, help="points of the M ladder per doubling, up to 16 images")
     ap.add_argument("--max-rows", type=int, default=None)
     ap.add_argument("--repeats", type=int, default=5)
     ap.add_argument("--iters", type=int, default=10)
@@ -269,7 +290,7 @@ def main(argv=None) -> int:
         print(f"{len(table)} rows -> {TABLE_HEADER}")
         return 0
     only = {int(x) for x in a.variants.split(",")} if a.variants else None
-    run_sweep(a.shapes.split(","), a.m_steps, a.repeats, a.iters, a.out, only, a.max_rows)
+    run_sweep(a.shapes.split(","), a.m_steps, a.repeats, a.iters, a.out, only, a.max_rows, per_octave=a.per_octave)
     print(f"wrote {a.out}")
     return 0
 
