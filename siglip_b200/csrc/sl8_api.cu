@@ -525,11 +525,15 @@ int ensure(sl8_handle_t h, void** p, size_t* have, size_t need) {
     return SL8_OK;
 }
 
-// Rows per slab: about 64 MiB of output, a multiple of 256 rows so slabs start on tile rows.
-long long slab_rows_for(long long M, int N, int K, int out_bytes, bool has_res) {
-    const double per_row = (double)K + (double)N * out_bytes + (has_res ? 2.0 * N : 0.0);
-    long long rows = (long long)(64.0 * 1024 * 1024 / per_row);
-    rows = (rows / 256) * 256;
+// Rows per slab of a call that moves per_row bytes over the bus for each row: an eighth of the call, so that all but the
+// first slab's way up and the last one's way down run in both directions at once (with slabs of 64 MiB an MLP of 16 images was
+// one slab and its three legs ran one after the other: 1 550 -> 1 200 us; a sixteenth: 1 360), but no less than 10 MiB (slabs
+// of 4 MiB took 1 500 rows from 480 to 620 us: the copies' own start-up) and no more than 64 MiB, which bounds the staging.  A
+// multiple of 256 rows: slabs start on tile rows.
+long long slab_rows_for(long long M, double per_row) {
+    const double MiB = 1024.0 * 1024.0, share = (double)M * per_row / 8.0;
+    const double bytes = share < 10.0 * MiB ? 10.0 * MiB : share > 64.0 * MiB ? 64.0 * MiB : share;
+    long long rows = (long long)(bytes / per_row) / 256 * 256;
     if (rows < 256) rows = 256;
     if (rows > M) rows = M;
     return rows;
@@ -572,7 +576,7 @@ int run_host(sl8_handle_t h, Problem q, float scale_a, float scale_b, float out_
     cudaError_t e;
     int rc = pipe_init(h);
     if (rc != SL8_OK) return rc;
-    const long long slab = slab_rows_for(q.M, q.N, q.K, ob, has_res);
+    const long long slab = slab_rows_for(q.M, (double)q.K + (double)q.N * ob + (has_res ? 2.0 * q.N : 0.0));
     for (int i = 0; i < HostPipe::SLOTS; i++) {
         size_t ha = pp.a_bytes, hd = pp.d_bytes, hr = pp.r_bytes;
         if ((rc = ensure(h, &pp.d_a[i], &ha, (size_t)slab * q.lda)) != SL8_OK) return rc;
@@ -737,12 +741,8 @@ SL8_API int sl8_mlp_chain_fp8_host(sl8_handle_t h, const void* A, int64_t lda, c
     HostPipe& pp = h->pipe;
     int rc = pipe_init(h);
     if (rc != SL8_OK) return rc;
-    // Rows per slab: about 64 MiB of traffic over the bus (A up, residual up, D down); the hidden slab stays on the GPU.
     const long long ld_hidden = ((long long)d_ff + 127) / 128 * 128;
-    long long slab = (long long)(64.0 * 1024 * 1024 / ((double)d_model * 5.0));
-    slab = slab / 256 * 256;
-    if (slab < 256) slab = 256;
-    if (slab > M) slab = M;
+    const long long slab = slab_rows_for(M, (double)d_model * 5.0);      // A and the residual up, D down; the hidden slab stays on the GPU
     for (int i = 0; i < HostPipe::SLOTS; i++) {
         size_t ha = pp.a_bytes, hd = pp.d_bytes, hr = pp.r_bytes, hh = pp.h_bytes;
         if ((rc = ensure(h, &pp.d_a[i], &ha, (size_t)slab * lda)) != SL8_OK) return rc;
