@@ -208,7 +208,8 @@ int sl8_patchify_quantize_e4m3(sl8_handle_t h, const void* pixels, int pixel_dty
                                void* A, int64_t lda, sl8_stream_t stream);
 
 /* Dynamic per-tensor scale of an activation x [rows, cols] (fp32 or bf16, leading dimension ld elements):
- * *amax = max |x| and, if scale is not NULL, *scale = amax / 448 (1 for an all-zero tensor).  Device pointers. */
+ * *amax = max |x| and, if scale is not NULL, *scale = amax / 448 (1 for an all-zero tensor).  Device pointers; until the
+ * call has run on its stream both words hold intermediate values. */
 int sl8_amax_scale(sl8_handle_t h, const void* x, int dtype, int64_t rows, int cols, int64_t ld,
                    float* amax, float* scale, sl8_stream_t stream);
 

@@ -13,7 +13,7 @@
 //                 TMA unit has generated the requests of its previous one (2 cycles per 128-byte row:
 //                 64 bytes per clock per issuing thread, measured), while the unit itself serves two
 //                 threads at once at 128 bytes per clock: one thread cannot feed a 256 x 256 tile.
-//   warp 1        allocates tensor memory; one thread of the leader CTA issues
+//   warp 1        allocates tensor memory; one elected thread of the leader CTA's issues
 //                 tcgen05.mma kind::f8f6f4 (E4M3 x E4M3 -> FP32 in TMEM), four K=32 steps per
 //                 k-block (fewer in the K tail), and commits to the stage's empty barrier and,
 //                 after the last k-block, to the accumulator's full barrier.
@@ -597,8 +597,9 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         // The whole warp walks the loop and one elected lane issues: a tcgen05.mma takes its descriptors from uniform
         // registers, and in a branch that only one lane takes each of them is moved there instruction by instruction, which
         // cost ~110 cycles per MMA -- hidden behind the 128 cycles of a 256-column tile, but twice what a 128-column tile
-        // needs (1152-wide FC2 at 729 rows on 128 x 128 tiles 14.5 -> 11.6 us; at 46 656 rows on 256 x 256 tiles 193 -> 186).  What else the loop executes per
-        // k-block counts too: the poll of the NEXT stage's barrier is issued before this stage's MMAs and read after them
+        // needs (1152-wide FC2 at 729 rows on 128 x 128 tiles 14.5 -> 11.6 us; at 46 656 rows on 256 x 256 tiles 193 -> 186).
+        // What else the loop executes per k-block counts too: the poll of the NEXT stage's barrier is issued before this
+        // stage's MMAs and read after them
         // (the blocking wait runs only if that look-ahead failed), and k-blocks are taken several per loop iteration.
         if (cta_rank == 0) {
             const uint32_t idesc_full = make_idesc_e4m3_f32(T::TILE_M_CTA * CG, TN);

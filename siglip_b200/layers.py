@@ -70,8 +70,9 @@ class Engine:
         return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
     # A call whose operands are all as they should be goes through the extension module (csrc/sl8_torch.cpp), which checks
-    # and launches without Python in between: 8.9 -> 4 - 5 us a call (one image through a block, eight launches: 71 -> 51 us).  It answers None to anything else, and the method goes
-    # on in Python: there the same checks raise, and unusual tensors are read through their own attributes.
+    # and launches without Python in between: 8.9 -> 4 - 5 us a call (one image through a block, eight launches: 71 -> 51 us).
+    # It answers None to anything else, and the method goes on in Python: there the same checks raise, and unusual tensors
+    # are read through their own attributes.
     @functools.cached_property
     def _native(self):
         return _l.load_binding()
