@@ -52,3 +52,33 @@ def test_back_to_back_and_captured_calls_match_synchronised_ones(engine, rows, d
         graph.replay()
         torch.cuda.synchronize()
         assert same()
+
+
+def test_calls_behind_a_fork_and_a_fill_are_captured_in_order(engine):
+    """What a captured launch waits for may be several nodes, and not kernels only: a fill on its own stream, work joined from another."""
+    rows, d = 300, 256
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x = torch.randn((rows, d), generator=g, device=DEV).to(torch.bfloat16)
+    w = synth.quantize_e4m3(torch.randn((d, d), generator=g, device=DEV) * 0.05)[0]
+    scale = torch.full((1,), 0.02, device=DEV)
+    a = torch.zeros((rows, d), dtype=torch.uint8, device=DEV)
+    res, out = torch.empty_like(x), torch.empty_like(x)
+    want = engine.fc2_residual(engine.layernorm_quantize(x, None, None, 1e-6, scale, out=torch.zeros_like(a)), w, None, x * 2, scale_a=scale)
+    main, side = torch.cuda.Stream(), torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=main):
+        a.zero_()
+        engine.layernorm_quantize(x, None, None, 1e-6, scale, out=a)
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            res.copy_(x)
+            res.mul_(2)
+        main.wait_stream(side)
+        engine.fc2_residual(a, w, None, res, scale_a=scale, out=out)
+    for _ in range(5):
+        a.fill_(0x7E)
+        res.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
