@@ -305,7 +305,7 @@ inline int prep_batch(sl8_handle_t h, long long vectors, int vector_bytes, int s
 // otherwise element by element.  With `scale`, the block that finishes last also writes it: until then the word counts the
 // finished blocks (zero_two_kernel cleared both), which saves the launch of a kernel for one division.
 // Bound by L2 / HBM reads: 50 MB (5 832 x 4 304 bf16) with
-// the scale 10.5 -> 9.6 us, 729 x 1 152, where the launches count, 6.3 -> 4.1 us.
+// the scale 10.5 -> 6.7 us (7.5 TB/s), 46 656 x 1 152 20.6 -> 17.2, 729 x 1 152, where the launches count, 6.3 -> 4.1.
 template <typename T, int BATCH>
 __global__ void __launch_bounds__(kPrepThreads) amax_kernel(const T* x, long long rows, int cols, long long ld, int vectors, unsigned* amax_bits, float* scale) {
     sl8::pdl_wait();
@@ -587,7 +587,8 @@ constexpr int kLnThreads = 128;
 // way while it works on this one.  (Read per row, from L1, gamma and beta are four times the bytes of a bf16 row, and they were
 // asked for only after the row's two reductions.)  Scalar fp32 arithmetic: the packed two-element forms were measured
 // 20 - 40 % slower here.  bf16, 1 152 columns: 729 rows 3.6 -> 2.8 us,
-// 5 003 rows 8.5 -> 5.5, 46 656 rows 49 -> 39.5 (4.1 TB/s); 1 600 columns, 5 003 rows 15.9 -> 7.8.  A ring of three rows in
+// 5 003 rows 8.5 -> 5.5, 46 656 rows 49 -> 39.5 (4.1 TB/s); 1 600 columns, 5 003 rows 15.9 -> 7.8.  Gamma and beta read per row instead, and four
+// blocks per SM for the registers that frees: 5 003 rows 7.5 us, 46 656 rows 42.  A ring of three rows in
 // shared memory filled by cp.async was 10 % slower up to 12 000 rows and up to 60 % in fp32, 12 % faster from 46 656 bf16 rows.
 // (2 048 columns: registers for the row only, gamma and beta a chunk ahead of their use.)
 template <typename T, int CHUNKS>
