@@ -248,6 +248,11 @@ int activation(const at::Tensor& t) { return t.scalar_type() == at::kFloat ? SL8
 // (the pitch is taken from stride(0); what the strides inside a row are is the caller's business, as it is in Python)
 bool rows_of(const at::Tensor& t) { return t.dim() == 2 && t.size(1) <= INT_MAX && activation(t) >= 0; }
 
+// Whether t has room for [rows, cols] codes at its own row pitch.
+bool holds_codes(const at::Tensor& t, int64_t rows, int64_t cols) {
+    return codes(t) && t.dim() == 2 && t.size(0) >= rows && t.size(1) >= cols && (t.stride(1) == 1 || t.size(1) == 1);
+}
+
 // h, device, stream, pixels, scale, out, patch
 SL8_PY(patchify_quantize) {
     HANDLE_TH_ERRORS
@@ -257,9 +262,15 @@ SL8_PY(patchify_quantize) {
     const float* scale = a.scale();
     const at::Tensor* out = a.ok ? a.tensor() : nullptr;
     const long long patch = a.ok ? a.integer() : 0;
-    if (!a.ok || px->dim() != 4 || !px->is_contiguous() || activation(*px) < 0 || out->dim() < 1 || patch < 1) Py_RETURN_NONE;
+    if (!a.ok || px->dim() != 4 || !px->is_contiguous() || activation(*px) < 0 || patch < 1) Py_RETURN_NONE;
     for (int i = 0; i < 4; i++)
         if (px->size(i) > INT_MAX) Py_RETURN_NONE;
+    if (px->size(2) < patch || px->size(3) < patch) Py_RETURN_NONE;
+    const int64_t rows = px->size(0) * (px->size(2) / patch) * (px->size(3) / patch), cols = px->size(1) * patch * patch;
+    if (rows < 1 || cols < 1 || !holds_codes(*out, rows, cols)) Py_RETURN_NONE;
+    // (the kernel fills a pad of less than 128 bytes with zeros, the last row's too)
+    const int64_t pitch = out->stride(0), written = pitch - cols < 128 ? pitch : (cols + 15) / 16 * 16;
+    if (out->storage_offset() + (rows - 1) * pitch + written > static_cast<int64_t>(out->storage().nbytes())) Py_RETURN_NONE;
     return launched(*out, [&] {
         return sl8_patchify_quantize_e4m3(a.h, px->const_data_ptr(), activation(*px), static_cast<int>(px->size(0)), static_cast<int>(px->size(1)),
                                           static_cast<int>(px->size(2)), static_cast<int>(px->size(3)), static_cast<int>(patch), scale,
@@ -300,7 +311,7 @@ SL8_PY(quantize_e4m3) {
     const at::Tensor* x = a.tensor();
     const float* scale = a.scale();
     const at::Tensor* out = a.ok ? a.tensor() : nullptr;
-    if (!a.ok || !rows_of(*x) || out->dim() < 1) Py_RETURN_NONE;
+    if (!a.ok || !rows_of(*x) || !holds_codes(*out, x->size(0), x->size(1))) Py_RETURN_NONE;
     return launched(*out, [&] {
         return sl8_quantize_e4m3(a.h, x->const_data_ptr(), activation(*x), x->size(0), static_cast<int>(x->size(1)), x->stride(0), scale,
                                  out->mutable_data_ptr(), out->stride(0), a.stream());
@@ -317,7 +328,7 @@ SL8_PY(layernorm_quantize) {
     const float *gamma = a.scale(), *beta = a.scale(), *scale = a.scale();
     const at::Tensor* out = a.ok ? a.tensor() : nullptr;
     const double eps = a.ok ? a.real() : 0.0;
-    if (!a.ok || !rows_of(*x) || out->dim() < 1) Py_RETURN_NONE;
+    if (!a.ok || !rows_of(*x) || !holds_codes(*out, x->size(0), x->size(1))) Py_RETURN_NONE;
     return launched(*out, [&] {
         return sl8_layernorm_quantize_e4m3(a.h, x->const_data_ptr(), activation(*x), x->size(0), static_cast<int>(x->size(1)), x->stride(0), gamma, beta,
                                            static_cast<float>(eps), scale, out->mutable_data_ptr(), out->stride(0), a.stream());

@@ -313,6 +313,14 @@ class Engine:
             return _l.SL8_DT_BF16
         raise TypeError("expected an fp32 or bf16 tensor")
 
+    def _codes_into(self, out: torch.Tensor, rows: int, cols: int) -> None:
+        """A caller-supplied buffer for [rows, cols] codes: one code after the other in a row, and at least that large (the
+        library knows its address and row pitch, not where it ends)."""
+        if out.dtype not in self._E4M3_TYPES:
+            raise TypeError(f"out has dtype {out.dtype}; codes are float8_e4m3fn or uint8")
+        if out.dim() != 2 or out.shape[0] < rows or out.shape[1] < cols or (out.stride(1) != 1 and out.shape[1] != 1):
+            raise ValueError(f"out [{', '.join(map(str, out.shape))}] must hold [{rows}, {cols}] codes, columns contiguous")
+
     def patchify_quantize(self, pixels, patch: int, scale=None, *, out=None, pitch=None, stream=None) -> torch.Tensor:
         """pixels [images, C, H, W] (fp32 / bf16) -> A [images * (H // patch) * (W // patch), C * patch * patch] e4m3
         codes (uint8) at a row pitch that is a multiple of 128 bytes: the patch-embed GEMM's operand."""
@@ -329,6 +337,12 @@ class Engine:
         if out is None:
             pitch = (K + 127) // 128 * 128 if pitch is None else int(pitch)
             out = torch.empty((rows, pitch), dtype=torch.uint8, device=pixels.device)[:, :K]
+        else:
+            self._codes_into(out, rows, K)
+            pitch = out.stride(0)         # a pad of less than 128 bytes is filled with zeros, the last row's too
+            written = pitch if pitch - K < 128 else (K + 15) // 16 * 16
+            if out.storage_offset() + (rows - 1) * pitch + written > out.untyped_storage().nbytes():
+                raise ValueError("out ends inside the pad of its last row, which is written with the row")
         self._check(self._lib.sl8_patchify_quantize_e4m3(
             self._h, pixels.data_ptr(), self._dt(pixels), images, Cc, H, W, int(patch), _ptr(scale), out.data_ptr(),
             out.stride(0), self._stream(stream)))
@@ -354,6 +368,8 @@ class Engine:
         rows, cols = x.shape
         if out is None:
             out = torch.empty((rows, (cols + 127) // 128 * 128), dtype=torch.uint8, device=x.device)[:, :cols]
+        else:
+            self._codes_into(out, rows, cols)
         self._check(self._lib.sl8_quantize_e4m3(self._h, x.data_ptr(), self._dt(x), rows, cols, x.stride(0), _ptr(scale),
                                                 out.data_ptr(), out.stride(0), self._stream(stream)))
         return out
@@ -368,6 +384,8 @@ class Engine:
         rows, cols = x.shape
         if out is None:
             out = torch.empty((rows, (cols + 127) // 128 * 128), dtype=torch.uint8, device=x.device)[:, :cols]
+        else:
+            self._codes_into(out, rows, cols)
         self._check(self._lib.sl8_layernorm_quantize_e4m3(
             self._h, x.data_ptr(), self._dt(x), rows, cols, x.stride(0), _ptr(gamma), _ptr(beta), float(eps), _ptr(scale),
             out.data_ptr(), out.stride(0), self._stream(stream)))

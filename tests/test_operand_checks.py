@@ -1,0 +1,90 @@
+"""What the calls on device tensors refuse before any launch, and what they let through, with and without the extension module
+in front of the C ABI.  No GPU: the calls meet a library that writes their arguments down (tests/fake_abi.py)."""
+import json
+
+import pytest
+import torch
+
+from tests import fake_abi
+from tests.fake_abi import STREAM, cuda
+
+U8, F8, BF16, F32, F16 = torch.uint8, torch.float8_e4m3fn, torch.bfloat16, torch.float32, torch.float16
+S = dict(stream=STREAM)
+
+
+def x(rows=8, cols=32, dtype=BF16, **kw):
+    return cuda(rows, cols, dtype=dtype, **kw)
+
+
+def one():
+    return cuda(1, dtype=F32)
+
+
+def pixels(dtype=F32):
+    return cuda(2, 3, 32, 48, dtype=dtype)         # 2 x 2 x 3 patches of 16 x 16: rows of 768 codes
+
+
+# Output buffers of the producer-side steps.
+OUT_REFUSED = {
+    "quantize_few_rows": lambda e: e.quantize_e4m3(x(), one(), out=cuda(7, 32), **S),
+    "quantize_few_columns": lambda e: e.quantize_e4m3(x(), one(), out=cuda(8, 24, stride=(32, 1)), **S),
+    "quantize_wide_type": lambda e: e.quantize_e4m3(x(), one(), out=cuda(8, 32, dtype=BF16), **S),
+    "quantize_strided": lambda e: e.quantize_e4m3(x(), one(), out=cuda(8, 32, stride=(64, 2)), **S),
+    "quantize_three_dimensions": lambda e: e.quantize_e4m3(x(), one(), out=cuda(2, 4, 32), **S),
+    "layernorm_few_rows": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, one(), out=cuda(7, 32), **S),
+    "layernorm_wide_type": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, one(), out=cuda(8, 32, dtype=F32), **S),
+    "layernorm_one_dimension": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, one(), out=cuda(256), **S),
+    "patchify_few_rows": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(11, 768), **S),
+    "patchify_few_columns": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(12, 760, stride=(768, 1)), **S),
+    "patchify_wide_type": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(12, 768, dtype=BF16), **S),
+    # the rows are written whole up to a pitch that is a little wider: 16 bytes past the end of this buffer
+    "patchify_pad_past_the_end": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(12, 768, stride=(800, 1), offset=32), **S),
+}
+OUT_TAKEN = {
+    "quantize": lambda e: e.quantize_e4m3(x(), one(), out=cuda(8, 32), **S),
+    "quantize_f32_codes": lambda e: e.quantize_e4m3(x(dtype=F32), None, out=cuda(8, 32, dtype=F8), **S),
+    "quantize_more_rows": lambda e: e.quantize_e4m3(x(), one(), out=cuda(20, 32), **S),
+    "quantize_more_columns": lambda e: e.quantize_e4m3(x(), one(), out=cuda(8, 128), **S),
+    "quantize_pitched": lambda e: e.quantize_e4m3(x(), one(), out=cuda(8, 32, stride=(128, 1)), **S),
+    "quantize_one_column": lambda e: e.quantize_e4m3(x(8, 1), one(), out=cuda(8, 1, stride=(16, 16)), **S),
+    "layernorm": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, one(), out=cuda(8, 32, stride=(48, 1)), **S),
+    "layernorm_more_rows": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, one(), out=cuda(9, 40), **S),
+    "patchify": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(12, 768), **S),
+    "patchify_whole_pitch": lambda e: e.patchify_quantize(pixels(BF16), 16, one(), out=cuda(12, 768, stride=(800, 1), elements=12 * 800), **S),
+    "patchify_wide_pitch": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(12, 768, stride=(1024, 1)), **S),
+    "patchify_more_rows": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(16, 896), **S),
+}
+
+REFUSED = {f"out_{k}": v for k, v in OUT_REFUSED.items()}
+TAKEN = {f"out_{k}": v for k, v in OUT_TAKEN.items()}
+
+
+@pytest.fixture(scope="module")
+def folder(tmp_path_factory):
+    path = tmp_path_factory.mktemp("fake_abi")
+    fake_abi.install(path)
+    return path
+
+
+@pytest.fixture(scope="module")
+def results(folder):
+    out = {}
+    for table in ("REFUSED", "TAKEN"):
+        r = fake_abi.run_child(folder, __name__, table)
+        assert r.returncode == 0, r.stdout + r.stderr
+        out[table] = json.loads(r.stdout.splitlines()[-1])
+    return out
+
+
+@pytest.mark.parametrize("name", REFUSED)
+def test_refused_before_any_launch(results, name):
+    for route, (error, message, calls) in results["REFUSED"][name].items():
+        assert error in ("ValueError", "TypeError") and not calls, f"{route}: {error} {message} {calls}"
+    assert results["REFUSED"][name]["extension"] == results["REFUSED"][name]["python"]
+
+
+@pytest.mark.parametrize("name", TAKEN)
+def test_taken_with_the_same_arguments(results, name):
+    for route, (error, message, calls) in results["TAKEN"][name].items():
+        assert error is None and len(calls) == 1, f"{route}: {error} {message} {calls}"
+    assert results["TAKEN"][name]["extension"] == results["TAKEN"][name]["python"]
