@@ -112,6 +112,11 @@ class Engine:
         if t.device.index != self.device:
             raise ValueError(f"{name} is on cuda:{t.device.index}, this engine is bound to cuda:{self.device}")
 
+    def _readable(self, name: str, t: Optional[torch.Tensor]) -> None:
+        """An operand of a kernel that uses plain loads and stores: on this handle's GPU, or pinned, which every GPU reaches."""
+        if t is not None and (t.is_cuda or not t.is_pinned()):
+            self._on_device(name, t)
+
     def _check_out(self, out: torch.Tensor, M: int, N: int, allowed: tuple) -> torch.Tensor:
         """A caller-supplied output: [M, N], N contiguous, on this engine's GPU, of an element type the
         layer can write.  The kernel's output type is then taken from the tensor, never from a keyword."""
@@ -170,6 +175,7 @@ class Engine:
     def padded_table(self, table: torch.Tensor, stream=None) -> torch.Tensor:
         """bf16 [period, N] -> bf16 [sl8_padded_table_rows(period), N] whose extra rows repeat the period."""
         period, N = table.shape
+        self._on_device("table", table)
         rows = self._lib.sl8_padded_table_rows(period)
         out = torch.empty((rows, N), dtype=torch.bfloat16, device=table.device)
         self._check(self._lib.sl8_extend_periodic_table(self._h, table.data_ptr(), table.stride(0), period, N,
@@ -179,10 +185,12 @@ class Engine:
     def make_table(self, bias: Optional[torch.Tensor], pos: torch.Tensor, stream=None) -> torch.Tensor:
         """fp32 bias [N] (or None) and fp32 pos [period, N] -> padded bf16 table of bf16(bias + pos)."""
         period, N = pos.shape
+        self._on_device("pos", pos)
         rows = self._lib.sl8_padded_table_rows(period)
         out = torch.empty((rows, N), dtype=torch.bfloat16, device=pos.device)
         pos = pos.contiguous().float()
         b = None if bias is None else bias.contiguous().float()
+        self._readable("bias", b)
         self._check(self._lib.sl8_make_periodic_table(self._h, _ptr(b), pos.data_ptr(), period, N, out.data_ptr(),
                                                       out.stride(0), rows, self._stream(stream)))
         return out
@@ -316,6 +324,7 @@ class Engine:
     def _codes_into(self, out: torch.Tensor, rows: int, cols: int) -> None:
         """A caller-supplied buffer for [rows, cols] codes: one code after the other in a row, and at least that large (the
         library knows its address and row pitch, not where it ends)."""
+        self._readable("out", out)
         if out.dtype not in self._E4M3_TYPES:
             raise TypeError(f"out has dtype {out.dtype}; codes are float8_e4m3fn or uint8")
         if out.dim() != 2 or out.shape[0] < rows or out.shape[1] < cols or (out.stride(1) != 1 and out.shape[1] != 1):
@@ -334,10 +343,13 @@ class Engine:
         images, Cc, H, W = pixels.shape
         K = Cc * patch * patch
         rows = images * (H // patch) * (W // patch)
+        self._readable("scale", scale)
         if out is None:
+            self._on_device("pixels", pixels)
             pitch = (K + 127) // 128 * 128 if pitch is None else int(pitch)
             out = torch.empty((rows, pitch), dtype=torch.uint8, device=pixels.device)[:, :K]
         else:
+            self._readable("pixels", pixels)
             self._codes_into(out, rows, K)
             pitch = out.stride(0)         # a pad of less than 128 bytes is filled with zeros, the last row's too
             written = pitch if pitch - K < 128 else (K + 15) // 16 * 16
@@ -353,6 +365,7 @@ class Engine:
         r = self._native.amax_scale(self._handle, self.device, None if stream is None else self._stream(stream), x)
         if r is not None:
             return self._done(r)
+        self._on_device("x", x)
         amax = torch.empty((1,), dtype=torch.float32, device=x.device)
         scale = torch.empty((1,), dtype=torch.float32, device=x.device)
         self._check(self._lib.sl8_amax_scale(self._h, x.data_ptr(), self._dt(x), x.shape[0], x.shape[1], x.stride(0),
@@ -366,9 +379,12 @@ class Engine:
             if r is not None:
                 return self._done(r)
         rows, cols = x.shape
+        self._readable("scale", scale)
         if out is None:
+            self._on_device("x", x)
             out = torch.empty((rows, (cols + 127) // 128 * 128), dtype=torch.uint8, device=x.device)[:, :cols]
         else:
+            self._readable("x", x)
             self._codes_into(out, rows, cols)
         self._check(self._lib.sl8_quantize_e4m3(self._h, x.data_ptr(), self._dt(x), rows, cols, x.stride(0), _ptr(scale),
                                                 out.data_ptr(), out.stride(0), self._stream(stream)))
@@ -382,9 +398,13 @@ class Engine:
             if r is not None:
                 return self._done(r)
         rows, cols = x.shape
+        for name, t in (("gamma", gamma), ("beta", beta), ("scale", scale)):
+            self._readable(name, t)
         if out is None:
+            self._on_device("x", x)
             out = torch.empty((rows, (cols + 127) // 128 * 128), dtype=torch.uint8, device=x.device)[:, :cols]
         else:
+            self._readable("x", x)
             self._codes_into(out, rows, cols)
         self._check(self._lib.sl8_layernorm_quantize_e4m3(
             self._h, x.data_ptr(), self._dt(x), rows, cols, x.stride(0), _ptr(gamma), _ptr(beta), float(eps), _ptr(scale),

@@ -55,8 +55,49 @@ OUT_TAKEN = {
     "patchify_more_rows": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(16, 896), **S),
 }
 
-REFUSED = {f"out_{k}": v for k, v in OUT_REFUSED.items()}
+# Operands that are not on the engine's GPU (pageable host memory, another GPU).
+host = torch.zeros
+PLACE_REFUSED = {
+    "quantize_x": lambda e: e.quantize_e4m3(host(8, 32), one(), out=cuda(8, 32), **S),
+    "quantize_x_new_out": lambda e: e.quantize_e4m3(host(8, 32), one(), **S),
+    "quantize_x_other_gpu": lambda e: e.quantize_e4m3(x(device=1), one(), out=cuda(8, 32), **S),
+    "quantize_scale": lambda e: e.quantize_e4m3(x(), host(1), out=cuda(8, 32), **S),
+    "quantize_out": lambda e: e.quantize_e4m3(x(), one(), out=host(8, 32, dtype=U8), **S),
+    "quantize_out_other_gpu": lambda e: e.quantize_e4m3(x(), one(), out=cuda(8, 32, device=1), **S),
+    "amax_x": lambda e: e.amax_scale(host(8, 32), **S),
+    "amax_x_other_gpu": lambda e: e.amax_scale(x(device=1), **S),
+    "layernorm_x": lambda e: e.layernorm_quantize(host(8, 32), None, None, 1e-6, one(), out=cuda(8, 32), **S),
+    "layernorm_gamma": lambda e: e.layernorm_quantize(x(), host(32), None, 1e-6, one(), out=cuda(8, 32), **S),
+    "layernorm_beta": lambda e: e.layernorm_quantize(x(), None, host(32), 1e-6, one(), out=cuda(8, 32), **S),
+    "layernorm_scale": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, host(1), out=cuda(8, 32), **S),
+    "layernorm_out": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, one(), out=host(8, 32, dtype=U8), **S),
+    "patchify_pixels": lambda e: e.patchify_quantize(host(2, 3, 32, 48), 16, one(), out=cuda(12, 768), **S),
+    "patchify_pixels_new_out": lambda e: e.patchify_quantize(host(2, 3, 32, 48), 16, one(), **S),
+    "patchify_scale": lambda e: e.patchify_quantize(pixels(), 16, host(1), out=cuda(12, 768), **S),
+    "patchify_out": lambda e: e.patchify_quantize(pixels(), 16, one(), out=host(12, 768, dtype=U8), **S),
+    "padded_table": lambda e: e.padded_table(host(100, 32, dtype=BF16), **S),
+    "table_pos": lambda e: e.make_table(None, host(100, 32), **S),
+    "table_bias": lambda e: e.make_table(host(32), cuda(100, 32, dtype=F32), **S),
+}
+
+REFUSED = {f"place_{k}": v for k, v in PLACE_REFUSED.items()} | {f"out_{k}": v for k, v in OUT_REFUSED.items()}
 TAKEN = {f"out_{k}": v for k, v in OUT_TAKEN.items()}
+
+
+@pytest.mark.gpu
+def test_pinned_operands_are_read_in_place(engine):
+    """Host memory that the GPU reaches stays an operand of the producer-side steps."""
+    g = torch.Generator().manual_seed(0)
+    rows, px, scale = torch.randn((40, 64), generator=g).to(BF16), torch.rand((1, 3, 32, 32), generator=g), torch.tensor([0.05])
+    gpu = lambda t: t.to("cuda")
+    for size, call in (((40, 64), lambda f, out: engine.quantize_e4m3(f(rows), f(scale), out=out)),
+                       ((40, 64), lambda f, out: engine.layernorm_quantize(f(rows), None, None, 1e-6, f(scale), out=out)),
+                       ((4, 768), lambda f, out: engine.patchify_quantize(f(px), 16, f(scale), out=out))):
+        want = call(gpu, torch.zeros(size, dtype=U8, device="cuda"))
+        assert torch.equal(call(torch.Tensor.pin_memory, torch.zeros(size, dtype=U8, device="cuda")), want)
+        onto = call(gpu, torch.zeros(size, dtype=U8).pin_memory())
+        engine.device_status()
+        assert torch.equal(onto, want.cpu())
 
 
 @pytest.fixture(scope="module")
