@@ -186,11 +186,11 @@ class Engine:
         """fp32 bias [N] (or None) and fp32 pos [period, N] -> padded bf16 table of bf16(bias + pos)."""
         period, N = pos.shape
         self._on_device("pos", pos)
-        rows = self._lib.sl8_padded_table_rows(period)
-        out = torch.empty((rows, N), dtype=torch.bfloat16, device=pos.device)
         pos = pos.contiguous().float()
         b = None if bias is None else bias.contiguous().float()
         self._readable("bias", b)
+        rows = self._lib.sl8_padded_table_rows(period)
+        out = torch.empty((rows, N), dtype=torch.bfloat16, device=pos.device)
         self._check(self._lib.sl8_make_periodic_table(self._h, _ptr(b), pos.data_ptr(), period, N, out.data_ptr(),
                                                       out.stride(0), rows, self._stream(stream)))
         return out
