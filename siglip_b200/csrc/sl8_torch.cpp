@@ -245,8 +245,8 @@ SL8_PY(mlp_chain) {
 
 // SL8_DT_* of an activation, or -1.
 int activation(const at::Tensor& t) { return t.scalar_type() == at::kFloat ? SL8_DT_F32 : t.scalar_type() == at::kBFloat16 ? SL8_DT_BF16 : -1; }
-// (the pitch is taken from stride(0); what the strides inside a row are is the caller's business, as it is in Python)
-bool rows_of(const at::Tensor& t) { return t.dim() == 2 && t.size(1) <= INT_MAX && activation(t) >= 0; }
+// Rows of an activation, one element after the other, at a pitch of stride(0).
+bool rows_of(const at::Tensor& t) { return t.dim() == 2 && (t.stride(1) == 1 || t.size(1) == 1) && t.size(1) <= INT_MAX && activation(t) >= 0; }
 
 // Whether t has room for [rows, cols] codes at its own row pitch.
 bool holds_codes(const at::Tensor& t, int64_t rows, int64_t cols) {

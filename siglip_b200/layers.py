@@ -175,6 +175,8 @@ class Engine:
     def padded_table(self, table: torch.Tensor, stream=None) -> torch.Tensor:
         """bf16 [period, N] -> bf16 [sl8_padded_table_rows(period), N] whose extra rows repeat the period."""
         period, N = table.shape
+        if table.dtype != torch.bfloat16 or table.stride(1) != 1:
+            raise ValueError("table must be bf16 [period, N] with N contiguous")
         self._on_device("table", table)
         rows = self._lib.sl8_padded_table_rows(period)
         out = torch.empty((rows, N), dtype=torch.bfloat16, device=table.device)
@@ -321,6 +323,13 @@ class Engine:
             return _l.SL8_DT_BF16
         raise TypeError("expected an fp32 or bf16 tensor")
 
+    @staticmethod
+    def _rows(x: torch.Tensor):
+        """(rows, cols) of an activation whose rows lie stride(0) apart, one element after the other."""
+        if x.dim() != 2 or (x.stride(1) != 1 and x.shape[1] != 1):
+            raise ValueError("x must be [rows, cols] with the columns contiguous")
+        return x.shape
+
     def _codes_into(self, out: torch.Tensor, rows: int, cols: int) -> None:
         """A caller-supplied buffer for [rows, cols] codes: one code after the other in a row, and at least that large (the
         library knows its address and row pitch, not where it ends)."""
@@ -365,10 +374,11 @@ class Engine:
         r = self._native.amax_scale(self._handle, self.device, None if stream is None else self._stream(stream), x)
         if r is not None:
             return self._done(r)
+        rows, cols = self._rows(x)
         self._on_device("x", x)
         amax = torch.empty((1,), dtype=torch.float32, device=x.device)
         scale = torch.empty((1,), dtype=torch.float32, device=x.device)
-        self._check(self._lib.sl8_amax_scale(self._h, x.data_ptr(), self._dt(x), x.shape[0], x.shape[1], x.stride(0),
+        self._check(self._lib.sl8_amax_scale(self._h, x.data_ptr(), self._dt(x), rows, cols, x.stride(0),
                                              amax.data_ptr(), scale.data_ptr(), self._stream(stream)))
         return amax, scale
 
@@ -378,7 +388,7 @@ class Engine:
             r = self._native.quantize_e4m3(self._handle, self.device, None if stream is None else self._stream(stream), x, scale, out)
             if r is not None:
                 return self._done(r)
-        rows, cols = x.shape
+        rows, cols = self._rows(x)
         self._readable("scale", scale)
         if out is None:
             self._on_device("x", x)
@@ -397,7 +407,7 @@ class Engine:
                                                 x, gamma, beta, scale, out, eps)
             if r is not None:
                 return self._done(r)
-        rows, cols = x.shape
+        rows, cols = self._rows(x)
         for name, t in (("gamma", gamma), ("beta", beta), ("scale", scale)):
             self._readable(name, t)
         if out is None:

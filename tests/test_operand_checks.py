@@ -80,8 +80,26 @@ PLACE_REFUSED = {
     "table_bias": lambda e: e.make_table(host(32), cuda(100, 32, dtype=F32), **S),
 }
 
-REFUSED = {f"place_{k}": v for k, v in PLACE_REFUSED.items()} | {f"out_{k}": v for k, v in OUT_REFUSED.items()}
-TAKEN = {f"out_{k}": v for k, v in OUT_TAKEN.items()}
+# Activations whose rows are not what a base address and a row pitch describe.
+ROWS_REFUSED = {
+    "quantize_every_other_column": lambda e: e.quantize_e4m3(x(stride=(64, 2)), one(), out=cuda(8, 32), **S),
+    "quantize_transposed": lambda e: e.quantize_e4m3(x(8, 8, stride=(1, 8)), one(), out=cuda(8, 8), **S),
+    "quantize_one_row": lambda e: e.quantize_e4m3(x(1, 32, stride=(64, 2)), one(), out=cuda(1, 32), **S),
+    "quantize_three_dimensions": lambda e: e.quantize_e4m3(cuda(2, 4, 32, dtype=BF16), one(), out=cuda(8, 32), **S),
+    "amax_every_other_column": lambda e: e.amax_scale(x(stride=(64, 2)), **S),
+    "amax_three_dimensions": lambda e: e.amax_scale(cuda(2, 4, 32, dtype=BF16), **S),
+    "layernorm_every_other_column": lambda e: e.layernorm_quantize(x(stride=(64, 2)), None, None, 1e-6, one(), out=cuda(8, 32), **S),
+    "padded_table_transposed": lambda e: e.padded_table(cuda(32, 32, dtype=BF16, stride=(1, 32)), **S),
+    "padded_table_type": lambda e: e.padded_table(cuda(32, 32, dtype=F32), **S),
+}
+ROWS_TAKEN = {
+    "quantize_one_column_of_many": lambda e: e.quantize_e4m3(x(8, 1, stride=(64, 64)), one(), out=cuda(8, 16), **S),
+    "quantize_pitched": lambda e: e.quantize_e4m3(x(stride=(100, 1)), one(), out=cuda(8, 32), **S),
+    "layernorm_one_row": lambda e: e.layernorm_quantize(x(1, 32), None, None, 1e-6, one(), out=cuda(1, 32), **S),
+}
+
+REFUSED = {f"rows_{k}": v for k, v in ROWS_REFUSED.items()} | {f"place_{k}": v for k, v in PLACE_REFUSED.items()} | {f"out_{k}": v for k, v in OUT_REFUSED.items()}
+TAKEN = {f"rows_{k}": v for k, v in ROWS_TAKEN.items()} | {f"out_{k}": v for k, v in OUT_TAKEN.items()}
 
 
 @pytest.mark.gpu
