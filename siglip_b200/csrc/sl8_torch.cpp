@@ -49,12 +49,15 @@ struct Args {
         given = o != Py_None;
         return given ? plain(o) : nullptr;
     }
-    const void* optional_ptr() {
+    // `n` fp32 values in a row, or None.
+    const float* floats(int64_t n) {
         bool given;
         const at::Tensor* t = optional(given);
-        return t ? t->const_data_ptr() : nullptr;
+        if (!t) return nullptr;
+        if (t->scalar_type() != at::kFloat || t->numel() < n || (n > 1 && !t->is_contiguous())) { ok = false; return nullptr; }
+        return static_cast<const float*>(t->const_data_ptr());
     }
-    const float* scale() { return static_cast<const float*>(optional_ptr()); }
+    const float* scale() { return floats(1); }
     long long integer() {
         PyObject* o = v[at++];
         if (!PyLong_CheckExact(o)) { ok = false; return 0; }
@@ -223,11 +226,11 @@ SL8_PY(mlp_chain) {
     const at::Tensor* bias2 = a.optional(has_b2);
     const at::Tensor* residual = a.tensor();
     const float *sa = a.scale(), *s1 = a.scale(), *s2 = a.scale();
-    const at::Tensor* hidden_scale = a.tensor();
+    const float* sh = a.scale();
     const at::Tensor* hidden = a.tensor();
     const at::Tensor* given = a.optional(has_out);
     unsigned flags = static_cast<unsigned>(a.integer());
-    if (!a.ok || !codes(*W2) || !shaped(*W2, g.K, g.N) || residual->scalar_type() != at::kBFloat16 || !shaped(*residual, g.M, g.K) ||
+    if (!a.ok || !sh || !codes(*W2) || !shaped(*W2, g.K, g.N) || residual->scalar_type() != at::kBFloat16 || !shaped(*residual, g.M, g.K) ||
         !codes(*hidden) || !shaped(*hidden, g.M, g.N))
         Py_RETURN_NONE;
     if (has_b1 && bias1->scalar_type() == at::kFloat) flags |= SL8_FLAG_BIAS_F32;
@@ -236,7 +239,7 @@ SL8_PY(mlp_chain) {
     return launched(out, [&] {
         return sl8_mlp_chain_fp8(a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, s1,
                                  bias1 ? bias1->const_data_ptr() : nullptr, hidden->mutable_data_ptr(), hidden->stride(0),
-                                 static_cast<const float*>(hidden_scale->const_data_ptr()), W2->const_data_ptr(), W2->stride(0), s2,
+                                 sh, W2->const_data_ptr(), W2->stride(0), s2,
                                  bias2 ? bias2->const_data_ptr() : nullptr, residual->const_data_ptr(), residual->stride(0), out.mutable_data_ptr(),
                                  out.stride(0), g.M, static_cast<int>(g.K), static_cast<int>(g.N), flags, a.stream());
     });
@@ -325,7 +328,8 @@ SL8_PY(layernorm_quantize) {
     Args a(args, count, 6);
     if (!a.ok) Py_RETURN_NONE;
     const at::Tensor* x = a.tensor();
-    const float *gamma = a.scale(), *beta = a.scale(), *scale = a.scale();
+    const int64_t cols = a.ok && x->dim() == 2 ? x->size(1) : 0;
+    const float *gamma = a.floats(cols), *beta = a.floats(cols), *scale = a.scale();
     const at::Tensor* out = a.ok ? a.tensor() : nullptr;
     const double eps = a.ok ? a.real() : 0.0;
     if (!a.ok || !rows_of(*x) || !holds_codes(*out, x->size(0), x->size(1))) Py_RETURN_NONE;

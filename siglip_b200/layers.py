@@ -112,10 +112,21 @@ class Engine:
         if t.device.index != self.device:
             raise ValueError(f"{name} is on cuda:{t.device.index}, this engine is bound to cuda:{self.device}")
 
+    def _scales(self, **scales) -> None:
+        for name, t in scales.items():
+            self._on_device(name, t)
+            self._floats(name, t)
+
     def _readable(self, name: str, t: Optional[torch.Tensor]) -> None:
         """An operand of a kernel that uses plain loads and stores: on this handle's GPU, or pinned, which every GPU reaches."""
         if t is not None and (t.is_cuda or not t.is_pinned()):
             self._on_device(name, t)
+
+    @staticmethod
+    def _floats(name: str, t: Optional[torch.Tensor], n: int = 1) -> None:
+        """A scale, or a vector of n: the kernels read fp32 values in a row."""
+        if t is not None and (t.dtype != torch.float32 or t.numel() < n or (n > 1 and not t.is_contiguous())):
+            raise ValueError(f"{name} must be float32, {n} element{'s, contiguous' if n > 1 else ''}")
 
     def _check_out(self, out: torch.Tensor, M: int, N: int, allowed: tuple) -> torch.Tensor:
         """A caller-supplied output: [M, N], N contiguous, on this engine's GPU, of an element type the
@@ -163,8 +174,8 @@ class Engine:
         if table.dtype != torch.bfloat16 or table.dim() != 2 or table.shape[1] != N or table.stride(1) != 1:
             raise ValueError("table must be bf16 [rows, N] with N contiguous")
         period = table.shape[0] if period is None else int(period)
-        for name, t in (("table", table), ("scale_a", scale_a), ("scale_b", scale_b)):
-            self._on_device(name, t)
+        self._on_device("table", table)
+        self._scales(scale_a=scale_a, scale_b=scale_b)
         D = self._new_out(M, N, torch.bfloat16, A.device) if out is None else self._check_out(out, M, N, (torch.bfloat16,))
         self._check(self._lib.sl8_patch_embed_fp8(
             self._h, A.data_ptr(), A.stride(0), B.data_ptr(), B.stride(0), _ptr(scale_a), _ptr(scale_b),
@@ -213,8 +224,8 @@ class Engine:
             flags |= _l.SL8_FLAG_BIAS_F32
         elif bias is not None and bias.dtype != torch.bfloat16:
             raise TypeError("bias must be bf16 or fp32")
-        for name, t in (("bias", bias), ("scale_a", scale_a), ("scale_b", scale_b), ("out_scale", out_scale)):
-            self._on_device(name, t)
+        self._on_device("bias", bias)
+        self._scales(scale_a=scale_a, scale_b=scale_b, out_scale=out_scale)
         D, out_code = self._resolve_out(out, out_dtype, M, N, A.device)
         self._check(self._lib.sl8_fc1_gelu_fp8(
             self._h, A.data_ptr(), A.stride(0), B.data_ptr(), B.stride(0), _ptr(scale_a), _ptr(scale_b), _ptr(bias),
@@ -237,8 +248,8 @@ class Engine:
             flags |= _l.SL8_FLAG_BIAS_F32
         elif bias is not None and bias.dtype != torch.bfloat16:
             raise TypeError("bias must be bf16 or fp32")
-        for name, t in (("bias", bias), ("scale_a", scale_a), ("scale_b", scale_b), ("out_scale", out_scale)):
-            self._on_device(name, t)
+        self._on_device("bias", bias)
+        self._scales(scale_a=scale_a, scale_b=scale_b, out_scale=out_scale)
         D, out_code = self._resolve_out(out, out_dtype, M, N, A.device)
         self._check(self._lib.sl8_linear_bias_fp8(
             self._h, A.data_ptr(), A.stride(0), B.data_ptr(), B.stride(0), _ptr(scale_a), _ptr(scale_b), _ptr(bias),
@@ -258,8 +269,9 @@ class Engine:
             flags |= _l.SL8_FLAG_BIAS_F32
         if residual.dtype != torch.bfloat16 or residual.shape != (M, N) or residual.stride(1) != 1:
             raise ValueError("residual must be bf16 [M, N] with N contiguous")
-        for name, t in (("bias", bias), ("residual", residual), ("scale_a", scale_a), ("scale_b", scale_b)):
+        for name, t in (("bias", bias), ("residual", residual)):
             self._on_device(name, t)
+        self._scales(scale_a=scale_a, scale_b=scale_b)
         D = self._new_out(M, N, torch.bfloat16, A.device) if out is None else self._check_out(out, M, N, (torch.bfloat16,))
         self._check(self._lib.sl8_fc2_residual_fp8(
             self._h, A.data_ptr(), A.stride(0), B.data_ptr(), B.stride(0), _ptr(scale_a), _ptr(scale_b), _ptr(bias),
@@ -290,9 +302,9 @@ class Engine:
         if hidden is None:
             hidden = torch.empty((M, (d_ff + 127) // 128 * 128), dtype=torch.uint8, device=A.device)[:, :d_ff]
         self._check_out(hidden, M, d_ff, self._E4M3_TYPES)
-        for name, t in (("W2", W2), ("bias1", bias1), ("bias2", bias2), ("residual", residual), ("scale_a", scale_a),
-                        ("scale_w1", scale_w1), ("scale_w2", scale_w2), ("hidden_scale", hidden_scale)):
+        for name, t in (("W2", W2), ("bias1", bias1), ("bias2", bias2), ("residual", residual)):
             self._on_device(name, t)
+        self._scales(scale_a=scale_a, scale_w1=scale_w1, scale_w2=scale_w2, hidden_scale=hidden_scale)
         D = self._new_out(M, d_model, torch.bfloat16, A.device) if out is None else self._check_out(out, M, d_model, (torch.bfloat16,))
         self._check(self._lib.sl8_mlp_chain_fp8(
             self._h, A.data_ptr(), A.stride(0), W1.data_ptr(), W1.stride(0), _ptr(scale_a), _ptr(scale_w1), _ptr(bias1),
@@ -352,6 +364,7 @@ class Engine:
         images, Cc, H, W = pixels.shape
         K = Cc * patch * patch
         rows = images * (H // patch) * (W // patch)
+        self._floats("scale", scale)
         self._readable("scale", scale)
         if out is None:
             self._on_device("pixels", pixels)
@@ -389,6 +402,7 @@ class Engine:
             if r is not None:
                 return self._done(r)
         rows, cols = self._rows(x)
+        self._floats("scale", scale)
         self._readable("scale", scale)
         if out is None:
             self._on_device("x", x)
@@ -408,7 +422,8 @@ class Engine:
             if r is not None:
                 return self._done(r)
         rows, cols = self._rows(x)
-        for name, t in (("gamma", gamma), ("beta", beta), ("scale", scale)):
+        for name, t, n in (("gamma", gamma, cols), ("beta", beta, cols), ("scale", scale, 1)):
+            self._floats(name, t, n)
             self._readable(name, t)
         if out is None:
             self._on_device("x", x)

@@ -22,7 +22,8 @@ STREAM = 77       # the stream every case names: torch's current one needs a dri
 
 _CTYPE = {C.c_void_p: "void*", C.c_int: "int", C.c_int64: "long long", C.c_uint: "unsigned", C.c_float: "float", C.c_char_p: "const char*"}
 _SPECIAL = {"sl8_create": "*(void**)a0 = (void*)0x1000; return 0;", "sl8_destroy": "return 0;", "sl8_last_error_string": 'return "";',
-            "sl8_version": 'return "";', "sl8_padded_table_rows": "return a0 + 127;"}
+            "sl8_version": 'return "";', "sl8_padded_table_rows": "return a0 + 127;",
+            "sl8_linear_bias_fp8": f"return sl8_fc1_gelu_fp8({', '.join(f'a{i}' for i in range(15))}, a15 | 4, a16);"}
 
 
 def source(signatures: dict) -> str:

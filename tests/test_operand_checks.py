@@ -98,8 +98,39 @@ ROWS_TAKEN = {
     "layernorm_one_row": lambda e: e.layernorm_quantize(x(1, 32), None, None, 1e-6, one(), out=cuda(1, 32), **S),
 }
 
-REFUSED = {f"rows_{k}": v for k, v in ROWS_REFUSED.items()} | {f"place_{k}": v for k, v in PLACE_REFUSED.items()} | {f"out_{k}": v for k, v in OUT_REFUSED.items()}
-TAKEN = {f"rows_{k}": v for k, v in ROWS_TAKEN.items()} | {f"out_{k}": v for k, v in OUT_TAKEN.items()}
+# Scales and affine vectors that are not fp32 values in a row, as many as are read.
+def gemm(e, f, **kw):
+    A, W, res, out = cuda(8, 32), cuda(64, 32), cuda(8, 64, dtype=BF16), cuda(8, 64, dtype=BF16)
+    if f == "fc2":
+        return e.fc2_residual(A, W, kw.pop("bias", None), res, out=out, **kw, **S)
+    if f == "embed":
+        return e.patch_embed(A, W, cuda(100, 64, dtype=BF16), out=out, **kw, **S)
+    if f == "mlp":
+        kw = dict(bias1=None, bias2=None, scale_a=None, scale_w1=None, scale_w2=None, hidden_scale=one()) | kw
+        return e.mlp_chain(A, W, kw.pop("bias1"), cuda(32, 64), kw.pop("bias2"), cuda(8, 32, dtype=BF16), hidden=cuda(8, 64),
+                           out=cuda(8, 32, dtype=BF16), **kw, **S)
+    return (e.fc1_gelu if f == "fc1" else e.linear_bias)(A, W, kw.pop("bias", None), out=out, **kw, **S)
+
+
+GEMM_SCALES = [(f, s) for f, names in (("fc1", "scale_a scale_b out_scale"), ("linear", "scale_a scale_b out_scale"), ("fc2", "scale_a scale_b"),
+                                       ("embed", "scale_a scale_b"), ("mlp", "scale_a scale_w1 scale_w2 hidden_scale")) for s in names.split()]
+FLOATS_REFUSED = {f"{f}_{s}_{t}": (lambda e, f=f, s=s, t=t: gemm(e, f, **{s: cuda(1, dtype=t) if t else cuda(0, dtype=F32, stride=(1,))}))
+                  for f, s in GEMM_SCALES for t in (BF16, torch.float64, None)} | {
+    "quantize_scale_bf16": lambda e: e.quantize_e4m3(x(), cuda(1, dtype=BF16), out=cuda(8, 32), **S),
+    "patchify_scale_f64": lambda e: e.patchify_quantize(pixels(), 16, cuda(1, dtype=torch.float64), out=cuda(12, 768), **S),
+    "layernorm_scale_int": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, cuda(1, dtype=torch.int32), out=cuda(8, 32), **S),
+    "layernorm_gamma_bf16": lambda e: e.layernorm_quantize(x(), cuda(32, dtype=BF16), None, 1e-6, one(), out=cuda(8, 32), **S),
+    "layernorm_beta_short": lambda e: e.layernorm_quantize(x(), None, cuda(31, dtype=F32), 1e-6, one(), out=cuda(8, 32), **S),
+    "layernorm_gamma_strided": lambda e: e.layernorm_quantize(x(), cuda(32, dtype=F32, stride=(2,)), None, 1e-6, one(), out=cuda(8, 32), **S),
+}
+FLOATS_TAKEN = {f"{f}_{s}": (lambda e, f=f, s=s: gemm(e, f, **{s: one()})) for f, s in GEMM_SCALES} | {
+    "fc1_scale_of_more": lambda e: gemm(e, "fc1", scale_a=cuda(4, dtype=F32), scale_b=cuda(1, 1, dtype=F32)),
+    "fc1_scale_expanded": lambda e: gemm(e, "fc1", scale_a=cuda(4, dtype=F32, stride=(0,))),
+    "layernorm_affine": lambda e: e.layernorm_quantize(x(), cuda(32, dtype=F32), cuda(2, 32, dtype=F32), 1e-6, one(), out=cuda(8, 32), **S),
+}
+
+REFUSED = {f"floats_{k}": v for k, v in FLOATS_REFUSED.items()} | {f"rows_{k}": v for k, v in ROWS_REFUSED.items()} | {f"place_{k}": v for k, v in PLACE_REFUSED.items()} | {f"out_{k}": v for k, v in OUT_REFUSED.items()}
+TAKEN = {f"floats_{k}": v for k, v in FLOATS_TAKEN.items()} | {f"rows_{k}": v for k, v in ROWS_TAKEN.items()} | {f"out_{k}": v for k, v in OUT_TAKEN.items()}
 
 
 @pytest.mark.gpu
