@@ -105,6 +105,15 @@ struct Gemm {
     }
 };
 
+// A bias of n elements (bf16, or fp32 with the flag), or none: what the kernel reads.  The flag and the type must not contradict.
+const void* bias_of(Args& a, const at::Tensor* t, int64_t n, unsigned& flags) {
+    if (!a.ok || !t) return nullptr;
+    const bool f32 = t->scalar_type() == at::kFloat;
+    if (f32) flags |= SL8_FLAG_BIAS_F32;
+    if ((!f32 && (t->scalar_type() != at::kBFloat16 || (flags & SL8_FLAG_BIAS_F32))) || t->numel() < n || !t->is_contiguous()) a.ok = false;
+    return a.ok ? t->const_data_ptr() : nullptr;
+}
+
 // `out`, or a new [M, N] beside A.  Defined unless the call is not the plain case.
 at::Tensor output(Args& a, const at::Tensor* given, const at::Tensor& A, int64_t M, int64_t N, at::ScalarType type, bool e4m3_too) {
     if (!given) return at::empty({M, N}, A.options().dtype(type));
@@ -143,17 +152,14 @@ SL8_PY(linear) {
     const at::Tensor* given = a.optional(has_out);
     const long long new_type = a.integer();
     unsigned flags = static_cast<unsigned>(a.integer());
-    if (a.ok && has_bias) {
-        if (bias->scalar_type() == at::kFloat) flags |= SL8_FLAG_BIAS_F32;
-        else if (bias->scalar_type() != at::kBFloat16) a.ok = false;
-    }
+    const void* const b = bias_of(a, bias, g.N, flags);
     if (!a.ok) Py_RETURN_NONE;
     const at::Tensor out = output(a, given, *g.A, g.M, g.N, new_type == 0 ? at::kBFloat16 : new_type == 1 ? at::kFloat8_e4m3fn : at::kByte, true);
     if (!a.ok) Py_RETURN_NONE;
     const int type = codes(out) ? SL8_OUT_E4M3 : SL8_OUT_BF16;
     return launched(out, [&] {
         return sl8_fc1_gelu_fp8(a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, sb,
-                                bias ? bias->const_data_ptr() : nullptr, out.mutable_data_ptr(), out.stride(0), type, so, g.M,
+                                b, out.mutable_data_ptr(), out.stride(0), type, so, g.M,
                                 static_cast<int>(g.N), static_cast<int>(g.K), flags, a.stream());
     });
     END_HANDLE_TH_ERRORS
@@ -201,13 +207,13 @@ SL8_PY(fc2_residual) {
     const float *sa = a.scale(), *sb = a.scale();
     const at::Tensor* given = a.optional(has_out);
     unsigned flags = static_cast<unsigned>(a.integer());
+    const void* const b = bias_of(a, bias, g.N, flags);
     if (!a.ok || residual->scalar_type() != at::kBFloat16 || !shaped(*residual, g.M, g.N)) Py_RETURN_NONE;
-    if (has_bias && bias->scalar_type() == at::kFloat) flags |= SL8_FLAG_BIAS_F32;
     const at::Tensor out = output(a, given, *g.A, g.M, g.N, at::kBFloat16, false);
     if (!a.ok) Py_RETURN_NONE;
     return launched(out, [&] {
         return sl8_fc2_residual_fp8(a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, sb,
-                                    bias ? bias->const_data_ptr() : nullptr, residual->const_data_ptr(), residual->stride(0), out.mutable_data_ptr(),
+                                    b, residual->const_data_ptr(), residual->stride(0), out.mutable_data_ptr(),
                                     out.stride(0), g.M, static_cast<int>(g.N), static_cast<int>(g.K), flags, a.stream());
     });
     END_HANDLE_TH_ERRORS
@@ -233,14 +239,16 @@ SL8_PY(mlp_chain) {
     if (!a.ok || !sh || !codes(*W2) || !shaped(*W2, g.K, g.N) || residual->scalar_type() != at::kBFloat16 || !shaped(*residual, g.M, g.K) ||
         !codes(*hidden) || !shaped(*hidden, g.M, g.N))
         Py_RETURN_NONE;
-    if (has_b1 && bias1->scalar_type() == at::kFloat) flags |= SL8_FLAG_BIAS_F32;
+    // One flag speaks for both: it is known before either is looked at.
+    if ((has_b1 && bias1->scalar_type() == at::kFloat) || (has_b2 && bias2->scalar_type() == at::kFloat)) flags |= SL8_FLAG_BIAS_F32;
+    const void *const b1 = bias_of(a, bias1, g.N, flags), *const b2 = bias_of(a, bias2, g.K, flags);
     const at::Tensor out = output(a, given, *g.A, g.M, g.K, at::kBFloat16, false);
     if (!a.ok) Py_RETURN_NONE;
     return launched(out, [&] {
         return sl8_mlp_chain_fp8(a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, s1,
-                                 bias1 ? bias1->const_data_ptr() : nullptr, hidden->mutable_data_ptr(), hidden->stride(0),
+                                 b1, hidden->mutable_data_ptr(), hidden->stride(0),
                                  sh, W2->const_data_ptr(), W2->stride(0), s2,
-                                 bias2 ? bias2->const_data_ptr() : nullptr, residual->const_data_ptr(), residual->stride(0), out.mutable_data_ptr(),
+                                 b2, residual->const_data_ptr(), residual->stride(0), out.mutable_data_ptr(),
                                  out.stride(0), g.M, static_cast<int>(g.K), static_cast<int>(g.N), flags, a.stream());
     });
     END_HANDLE_TH_ERRORS

@@ -112,6 +112,23 @@ class Engine:
         if t.device.index != self.device:
             raise ValueError(f"{name} is on cuda:{t.device.index}, this engine is bound to cuda:{self.device}")
 
+    @staticmethod
+    def _bias_flags(flags: int, *biases) -> int:
+        """`flags` with the bit that says the biases, each given with its name and the elements read, are fp32 and not bf16."""
+        flags = int(flags)
+        given = [(name, b, n) for name, b, n in biases if b is not None]
+        if any(b.dtype == torch.float32 for _, b, _ in given):
+            flags |= _l.SL8_FLAG_BIAS_F32
+        kind = torch.float32 if flags & _l.SL8_FLAG_BIAS_F32 else torch.bfloat16
+        for name, b, n in given:
+            if b.dtype not in (torch.float32, torch.bfloat16):
+                raise TypeError(f"{name} must be bf16 or fp32")
+            if b.dtype != kind:
+                raise TypeError(f"{name} is {b.dtype}, but the other bias or SL8_FLAG_BIAS_F32 says {kind}")
+            if b.numel() < n or not b.is_contiguous():
+                raise ValueError(f"{name} must have {n} elements, contiguous")
+        return flags
+
     def _scales(self, **scales) -> None:
         for name, t in scales.items():
             self._on_device(name, t)
@@ -220,10 +237,7 @@ class Engine:
             if r is not None:
                 return self._done(r)
         M, N, K = self._operands(A, B)
-        if bias is not None and bias.dtype == torch.float32:
-            flags |= _l.SL8_FLAG_BIAS_F32
-        elif bias is not None and bias.dtype != torch.bfloat16:
-            raise TypeError("bias must be bf16 or fp32")
+        flags = self._bias_flags(flags, ("bias", bias, N))
         self._on_device("bias", bias)
         self._scales(scale_a=scale_a, scale_b=scale_b, out_scale=out_scale)
         D, out_code = self._resolve_out(out, out_dtype, M, N, A.device)
@@ -244,10 +258,7 @@ class Engine:
             if r is not None:
                 return self._done(r)
         M, N, K = self._operands(A, B)
-        if bias is not None and bias.dtype == torch.float32:
-            flags |= _l.SL8_FLAG_BIAS_F32
-        elif bias is not None and bias.dtype != torch.bfloat16:
-            raise TypeError("bias must be bf16 or fp32")
+        flags = self._bias_flags(flags, ("bias", bias, N))
         self._on_device("bias", bias)
         self._scales(scale_a=scale_a, scale_b=scale_b, out_scale=out_scale)
         D, out_code = self._resolve_out(out, out_dtype, M, N, A.device)
@@ -265,8 +276,7 @@ class Engine:
         if r is not None:
             return self._done(r)
         M, N, K = self._operands(A, B)
-        if bias is not None and bias.dtype == torch.float32:
-            flags |= _l.SL8_FLAG_BIAS_F32
+        flags = self._bias_flags(flags, ("bias", bias, N))
         if residual.dtype != torch.bfloat16 or residual.shape != (M, N) or residual.stride(1) != 1:
             raise ValueError("residual must be bf16 [M, N] with N contiguous")
         for name, t in (("bias", bias), ("residual", residual)):
@@ -297,8 +307,7 @@ class Engine:
             raise ValueError("residual must be bf16 [M, d_model] with d_model contiguous")
         if hidden_scale is None:
             raise ValueError("hidden_scale (device float) is required: the scale of the e4m3 hidden activations")
-        if bias1 is not None and bias1.dtype == torch.float32:
-            flags |= _l.SL8_FLAG_BIAS_F32
+        flags = self._bias_flags(flags, ("bias1", bias1, d_ff), ("bias2", bias2, d_model))
         if hidden is None:
             hidden = torch.empty((M, (d_ff + 127) // 128 * 128), dtype=torch.uint8, device=A.device)[:, :d_ff]
         self._check_out(hidden, M, d_ff, self._E4M3_TYPES)

@@ -129,8 +129,28 @@ FLOATS_TAKEN = {f"{f}_{s}": (lambda e, f=f, s=s: gemm(e, f, **{s: one()})) for f
     "layernorm_affine": lambda e: e.layernorm_quantize(x(), cuda(32, dtype=F32), cuda(2, 32, dtype=F32), 1e-6, one(), out=cuda(8, 32), **S),
 }
 
-REFUSED = {f"floats_{k}": v for k, v in FLOATS_REFUSED.items()} | {f"rows_{k}": v for k, v in ROWS_REFUSED.items()} | {f"place_{k}": v for k, v in PLACE_REFUSED.items()} | {f"out_{k}": v for k, v in OUT_REFUSED.items()}
-TAKEN = {f"floats_{k}": v for k, v in FLOATS_TAKEN.items()} | {f"rows_{k}": v for k, v in ROWS_TAKEN.items()} | {f"out_{k}": v for k, v in OUT_TAKEN.items()}
+# Biases: bf16, or fp32 with the flag that says so, as many as the layer is wide.
+BIAS_REFUSED = {f"{f}_{what}": (lambda e, f=f, b=b, kw=kw: gemm(e, f, bias=b(), **kw)) for f in ("fc1", "linear", "fc2") for what, b, kw in (
+    ("fp16", lambda: cuda(64, dtype=F16), {}), ("fp64", lambda: cuda(64, dtype=torch.float64), {}),
+    ("flag_contradicts", lambda: cuda(64, dtype=BF16), dict(flags=1)), ("short", lambda: cuda(63, dtype=BF16), {}),
+    ("short_f32", lambda: cuda(48, dtype=F32), {}), ("strided", lambda: cuda(64, dtype=BF16, stride=(2,)), {}))} | {
+    "mlp_bias2_fp16": lambda e: gemm(e, "mlp", bias2=cuda(32, dtype=F16)),
+    "mlp_bias1_fp16": lambda e: gemm(e, "mlp", bias1=cuda(64, dtype=F16)),
+    "mlp_types_differ": lambda e: gemm(e, "mlp", bias1=cuda(64, dtype=F32), bias2=cuda(32, dtype=BF16)),
+    "mlp_types_differ_too": lambda e: gemm(e, "mlp", bias1=cuda(64, dtype=BF16), bias2=cuda(32, dtype=F32)),
+    "mlp_bias1_short": lambda e: gemm(e, "mlp", bias1=cuda(32, dtype=BF16)),
+    "mlp_bias2_short": lambda e: gemm(e, "mlp", bias2=cuda(31, dtype=BF16)),
+}
+BIAS_TAKEN = {f"{f}_{what}": (lambda e, f=f, b=b, kw=kw: gemm(e, f, bias=b(), **kw)) for f in ("fc1", "linear", "fc2") for what, b, kw in (
+    ("bf16", lambda: cuda(64, dtype=BF16), {}), ("f32", lambda: cuda(64, dtype=F32), {}), ("f32_flag", lambda: cuda(64, dtype=F32), dict(flags=1)),
+    ("none_flag", lambda: None, dict(flags=1)), ("row", lambda: cuda(1, 64, dtype=BF16), {}), ("longer", lambda: cuda(80, dtype=BF16), {}))} | {
+    "mlp_bf16": lambda e: gemm(e, "mlp", bias1=cuda(64, dtype=BF16), bias2=cuda(32, dtype=BF16)),
+    "mlp_f32": lambda e: gemm(e, "mlp", bias1=cuda(64, dtype=F32), bias2=cuda(32, dtype=F32)),
+    "mlp_second_f32": lambda e: gemm(e, "mlp", bias2=cuda(32, dtype=F32)),
+}
+
+REFUSED = {f"bias_{k}": v for k, v in BIAS_REFUSED.items()} | {f"floats_{k}": v for k, v in FLOATS_REFUSED.items()} | {f"rows_{k}": v for k, v in ROWS_REFUSED.items()} | {f"place_{k}": v for k, v in PLACE_REFUSED.items()} | {f"out_{k}": v for k, v in OUT_REFUSED.items()}
+TAKEN = {f"bias_{k}": v for k, v in BIAS_TAKEN.items()} | {f"floats_{k}": v for k, v in FLOATS_TAKEN.items()} | {f"rows_{k}": v for k, v in ROWS_TAKEN.items()} | {f"out_{k}": v for k, v in OUT_TAKEN.items()}
 
 
 @pytest.mark.gpu
@@ -171,6 +191,12 @@ def test_refused_before_any_launch(results, name):
     for route, (error, message, calls) in results["REFUSED"][name].items():
         assert error in ("ValueError", "TypeError") and not calls, f"{route}: {error} {message} {calls}"
     assert results["REFUSED"][name]["extension"] == results["REFUSED"][name]["python"]
+
+
+def test_the_flag_says_what_the_biases_are(results):
+    """The last argument but the stream of mlp_chain: one bit for both biases, whichever is given."""
+    flag = {k: int(results["TAKEN"][f"bias_mlp_{k}"]["python"][2][0].split()[-2]) for k in ("bf16", "f32", "second_f32")}
+    assert flag == {"bf16": 0, "f32": 1, "second_f32": 1}
 
 
 @pytest.mark.parametrize("name", TAKEN)
