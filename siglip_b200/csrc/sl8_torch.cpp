@@ -4,7 +4,7 @@
 // converting seventeen arguments through ctypes (about 9 us a call).  Each function here checks what the method of
 // the same name checks, and launches.  It returns the output, or the negative status of the C ABI as an int, or None:
 // whatever it does not take as it stands (another type of tensor, an operand out of place, an error to be raised) is
-// left to the method, which does the same through Python and raises.  The interpreter lock is released around the call.
+// left to the method, which does the same through Python and raises.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -127,14 +127,16 @@ PyObject* result(int rc, const at::Tensor& out) {
     return THPVariable_Wrap(out);
 }
 
-// A negative status, or what `call` launched on `out`.
-template <typename F>
-PyObject* launched(const at::Tensor& out, F call) {
+// The status of `entry`, a function of the C ABI, with the interpreter lock released.  The arguments are numbers and addresses,
+// read from the tensors while the lock is held: that may throw (a tensor without memory, no driver), and an exception must not
+// leave the part without the lock; nor may another thread change a tensor halfway through its reading.
+template <typename... P, typename... V>
+int unlocked(int (*entry)(P...), V... values) {
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = call();
+    rc = entry(values...);
     Py_END_ALLOW_THREADS
-    return result(rc, out);
+    return rc;
 }
 
 #define SL8_PY(name) PyObject* name(PyObject*, PyObject* const* args, Py_ssize_t count)
@@ -157,11 +159,10 @@ SL8_PY(linear) {
     const at::Tensor out = output(a, given, *g.A, g.M, g.N, new_type == 0 ? at::kBFloat16 : new_type == 1 ? at::kFloat8_e4m3fn : at::kByte, true);
     if (!a.ok) Py_RETURN_NONE;
     const int type = codes(out) ? SL8_OUT_E4M3 : SL8_OUT_BF16;
-    return launched(out, [&] {
-        return sl8_fc1_gelu_fp8(a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, sb,
-                                b, out.mutable_data_ptr(), out.stride(0), type, so, g.M,
-                                static_cast<int>(g.N), static_cast<int>(g.K), flags, a.stream());
-    });
+    const int rc = unlocked(sl8_fc1_gelu_fp8, a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, sb,
+                            b, out.mutable_data_ptr(), out.stride(0), type, so, g.M,
+                            static_cast<int>(g.N), static_cast<int>(g.K), flags, a.stream());
+    return result(rc, out);
     END_HANDLE_TH_ERRORS
 }
 
@@ -186,11 +187,10 @@ SL8_PY(patch_embed) {
     if (whole) period = table->size(0);
     const at::Tensor out = output(a, given, *g.A, g.M, g.N, at::kBFloat16, false);
     if (!a.ok) Py_RETURN_NONE;
-    return launched(out, [&] {
-        return sl8_patch_embed_fp8(a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, sb, table->const_data_ptr(),
-                                   table->stride(0), static_cast<int>(period), static_cast<int>(table->size(0)), static_cast<int>(row_phase),
-                                   out.mutable_data_ptr(), out.stride(0), g.M, static_cast<int>(g.N), static_cast<int>(g.K), flags, a.stream());
-    });
+    const int rc = unlocked(sl8_patch_embed_fp8, a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, sb, table->const_data_ptr(),
+                            table->stride(0), static_cast<int>(period), static_cast<int>(table->size(0)), static_cast<int>(row_phase),
+                            out.mutable_data_ptr(), out.stride(0), g.M, static_cast<int>(g.N), static_cast<int>(g.K), flags, a.stream());
+    return result(rc, out);
     END_HANDLE_TH_ERRORS
 }
 
@@ -211,11 +211,10 @@ SL8_PY(fc2_residual) {
     if (!a.ok || residual->scalar_type() != at::kBFloat16 || !shaped(*residual, g.M, g.N)) Py_RETURN_NONE;
     const at::Tensor out = output(a, given, *g.A, g.M, g.N, at::kBFloat16, false);
     if (!a.ok) Py_RETURN_NONE;
-    return launched(out, [&] {
-        return sl8_fc2_residual_fp8(a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, sb,
-                                    b, residual->const_data_ptr(), residual->stride(0), out.mutable_data_ptr(),
-                                    out.stride(0), g.M, static_cast<int>(g.N), static_cast<int>(g.K), flags, a.stream());
-    });
+    const int rc = unlocked(sl8_fc2_residual_fp8, a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, sb,
+                            b, residual->const_data_ptr(), residual->stride(0), out.mutable_data_ptr(),
+                            out.stride(0), g.M, static_cast<int>(g.N), static_cast<int>(g.K), flags, a.stream());
+    return result(rc, out);
     END_HANDLE_TH_ERRORS
 }
 
@@ -244,13 +243,12 @@ SL8_PY(mlp_chain) {
     const void *const b1 = bias_of(a, bias1, g.N, flags), *const b2 = bias_of(a, bias2, g.K, flags);
     const at::Tensor out = output(a, given, *g.A, g.M, g.K, at::kBFloat16, false);
     if (!a.ok) Py_RETURN_NONE;
-    return launched(out, [&] {
-        return sl8_mlp_chain_fp8(a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, s1,
-                                 b1, hidden->mutable_data_ptr(), hidden->stride(0),
-                                 sh, W2->const_data_ptr(), W2->stride(0), s2,
-                                 b2, residual->const_data_ptr(), residual->stride(0), out.mutable_data_ptr(),
-                                 out.stride(0), g.M, static_cast<int>(g.K), static_cast<int>(g.N), flags, a.stream());
-    });
+    const int rc = unlocked(sl8_mlp_chain_fp8, a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, s1,
+                            b1, hidden->mutable_data_ptr(), hidden->stride(0),
+                            sh, W2->const_data_ptr(), W2->stride(0), s2,
+                            b2, residual->const_data_ptr(), residual->stride(0), out.mutable_data_ptr(),
+                            out.stride(0), g.M, static_cast<int>(g.K), static_cast<int>(g.N), flags, a.stream());
+    return result(rc, out);
     END_HANDLE_TH_ERRORS
 }
 
@@ -282,11 +280,10 @@ SL8_PY(patchify_quantize) {
     // (the kernel fills a pad of less than 128 bytes with zeros, the last row's too)
     const int64_t pitch = out->stride(0), written = pitch - cols < 128 ? pitch : (cols + 15) / 16 * 16;
     if (out->storage_offset() + (rows - 1) * pitch + written > static_cast<int64_t>(out->storage().nbytes())) Py_RETURN_NONE;
-    return launched(*out, [&] {
-        return sl8_patchify_quantize_e4m3(a.h, px->const_data_ptr(), activation(*px), static_cast<int>(px->size(0)), static_cast<int>(px->size(1)),
-                                          static_cast<int>(px->size(2)), static_cast<int>(px->size(3)), static_cast<int>(patch), scale,
-                                          out->mutable_data_ptr(), out->stride(0), a.stream());
-    });
+    const int rc = unlocked(sl8_patchify_quantize_e4m3, a.h, px->const_data_ptr(), activation(*px), static_cast<int>(px->size(0)), static_cast<int>(px->size(1)),
+                            static_cast<int>(px->size(2)), static_cast<int>(px->size(3)), static_cast<int>(patch), scale,
+                            out->mutable_data_ptr(), out->stride(0), a.stream());
+    return result(rc, *out);
     END_HANDLE_TH_ERRORS
 }
 
@@ -299,11 +296,8 @@ SL8_PY(amax_scale) {
     if (!a.ok || !rows_of(*x)) Py_RETURN_NONE;
     const auto options = x->options().dtype(at::kFloat);
     const at::Tensor amax = at::empty({1}, options), scale = at::empty({1}, options);
-    int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = sl8_amax_scale(a.h, x->const_data_ptr(), activation(*x), x->size(0), static_cast<int>(x->size(1)), x->stride(0),
-                        static_cast<float*>(amax.mutable_data_ptr()), static_cast<float*>(scale.mutable_data_ptr()), a.stream());
-    Py_END_ALLOW_THREADS
+    const int rc = unlocked(sl8_amax_scale, a.h, x->const_data_ptr(), activation(*x), x->size(0), static_cast<int>(x->size(1)), x->stride(0),
+                            static_cast<float*>(amax.mutable_data_ptr()), static_cast<float*>(scale.mutable_data_ptr()), a.stream());
     if (rc != SL8_OK) return PyLong_FromLong(rc);
     PyObject* first = THPVariable_Wrap(amax);
     PyObject* second = first ? THPVariable_Wrap(scale) : nullptr;
@@ -323,10 +317,9 @@ SL8_PY(quantize_e4m3) {
     const float* scale = a.scale();
     const at::Tensor* out = a.ok ? a.tensor() : nullptr;
     if (!a.ok || !rows_of(*x) || !holds_codes(*out, x->size(0), x->size(1))) Py_RETURN_NONE;
-    return launched(*out, [&] {
-        return sl8_quantize_e4m3(a.h, x->const_data_ptr(), activation(*x), x->size(0), static_cast<int>(x->size(1)), x->stride(0), scale,
-                                 out->mutable_data_ptr(), out->stride(0), a.stream());
-    });
+    const int rc = unlocked(sl8_quantize_e4m3, a.h, x->const_data_ptr(), activation(*x), x->size(0), static_cast<int>(x->size(1)), x->stride(0), scale,
+                            out->mutable_data_ptr(), out->stride(0), a.stream());
+    return result(rc, *out);
     END_HANDLE_TH_ERRORS
 }
 
@@ -341,10 +334,9 @@ SL8_PY(layernorm_quantize) {
     const at::Tensor* out = a.ok ? a.tensor() : nullptr;
     const double eps = a.ok ? a.real() : 0.0;
     if (!a.ok || !rows_of(*x) || !holds_codes(*out, x->size(0), x->size(1))) Py_RETURN_NONE;
-    return launched(*out, [&] {
-        return sl8_layernorm_quantize_e4m3(a.h, x->const_data_ptr(), activation(*x), x->size(0), static_cast<int>(x->size(1)), x->stride(0), gamma, beta,
-                                           static_cast<float>(eps), scale, out->mutable_data_ptr(), out->stride(0), a.stream());
-    });
+    const int rc = unlocked(sl8_layernorm_quantize_e4m3, a.h, x->const_data_ptr(), activation(*x), x->size(0), static_cast<int>(x->size(1)), x->stride(0), gamma, beta,
+                            static_cast<float>(eps), scale, out->mutable_data_ptr(), out->stride(0), a.stream());
+    return result(rc, *out);
     END_HANDLE_TH_ERRORS
 }
 

@@ -168,6 +168,9 @@ def test_pinned_operands_are_read_in_place(engine):
         engine.device_status()
         assert torch.equal(onto, want.cpu())
 
+# Calls whose stream is torch's current one: without a driver asking for it throws, in the middle of the extension's work.
+THROWS = {"quantize": lambda e: e.quantize_e4m3(x(), one(), out=cuda(8, 32)), "fc1": lambda e: e.fc1_gelu(cuda(8, 32), cuda(64, 32), None, out=cuda(8, 64, dtype=BF16))}
+
 
 @pytest.fixture(scope="module")
 def folder(tmp_path_factory):
@@ -191,6 +194,24 @@ def test_refused_before_any_launch(results, name):
     for route, (error, message, calls) in results["REFUSED"][name].items():
         assert error in ("ValueError", "TypeError") and not calls, f"{route}: {error} {message} {calls}"
     assert results["REFUSED"][name]["extension"] == results["REFUSED"][name]["python"]
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="with a driver nothing throws here")
+def test_a_throw_inside_the_extension_is_an_exception(folder):
+    r = fake_abi.run_child(folder, __name__, "THROWS")
+    assert r.returncode == 0, f"the process died ({r.returncode}): {r.stderr[-2000:]}"
+    for name, routes in json.loads(r.stdout.splitlines()[-1]).items():
+        assert routes["extension"][0] and not routes["extension"][2], (name, routes)
+
+
+@pytest.mark.gpu
+def test_a_new_output_without_memory_is_an_exception(engine):
+    """Under a fake-tensor mode the output that the call allocates has no address: an error, as without the extension."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    A, W = torch.zeros((128, 64), dtype=U8, device="cuda"), torch.zeros((64, 64), dtype=U8, device="cuda")
+    with FakeTensorMode(allow_non_fake_inputs=True), pytest.raises(Exception):
+        engine.fc1_gelu(A, W, None)
+    engine.device_status()
 
 
 def test_the_flag_says_what_the_biases_are(results):
