@@ -53,7 +53,7 @@ def variant_ids() -> list[int]:
 
 
 def sources_mtime() -> float:
-    files = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cpp")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))
+    files = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))
     files.append(PKG.parent / "include" / "siglip_fp8.h")
     return max(f.stat().st_mtime for f in files)
 
@@ -69,6 +69,18 @@ def compile_one(args: tuple[list[str], Path, bool]) -> str:
     return res.stderr
 
 
+def torch_tag() -> str:
+    """What the extension module is tied to: the torch it is compiled against, and the interpreter."""
+    import torch
+    return f"{torch.__version__} {sys.implementation.cache_tag}"
+
+
+def binding_current() -> bool:
+    stamp = BINDING.with_suffix(".tag")
+    return (BINDING.exists() and stamp.exists() and stamp.read_text() == torch_tag() and
+            BINDING.stat().st_mtime >= max((CSRC / "sl8_torch.cpp").stat().st_mtime, (PKG.parent / "include" / "siglip_fp8.h").stat().st_mtime))
+
+
 def binding_compile(obj: Path) -> list[str]:
     import sysconfig
     import torch
@@ -76,7 +88,7 @@ def binding_compile(obj: Path) -> list[str]:
     cuda = Path(nvcc()).resolve().parent.parent / "include"
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-I{inc}",
             f"-I{inc / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{cuda}", f"-I{sysconfig.get_paths()['include']}",
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-c", str(CSRC / "sl8_torch.cpp"), "-o", str(obj)]
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DSL8_TORCH_VERSION="{torch.__version__}"', "-c", str(CSRC / "sl8_torch.cpp"), "-o", str(obj)]
 
 
 def binding_link(obj: Path) -> list[str]:
@@ -88,10 +100,25 @@ def binding_link(obj: Path) -> list[str]:
 
 def build(force: bool = False, verbose: bool = False) -> Path:
     """Compiles what is out of date and returns the path of the shared library."""
-    products = (LIB, BINDING, BENCH)
-    if not force and all(f.exists() for f in products) and min(f.stat().st_mtime for f in products) >= sources_mtime():
-        return LIB
     OBJ.mkdir(parents=True, exist_ok=True)
+    products = (LIB, BENCH)
+    if force or not all(f.exists() for f in products) or min(f.stat().st_mtime for f in products) < sources_mtime():
+        build_library(verbose)
+    if force or not binding_current():
+        binding = OBJ / "torch.o"
+        compile_one((binding_compile(binding), OBJ / "torch.log", verbose))
+        run_link(binding_link(binding))
+        BINDING.with_suffix(".tag").write_text(torch_tag())
+    return LIB
+
+
+def run_link(cmd: list[str]) -> None:
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"link failed: {' '.join(cmd)}\n{res.stdout}\n{res.stderr}")
+
+
+def build_library(verbose: bool) -> None:
     for stale in list(OBJ.glob("variant_*.o")) + list(OBJ.glob("variant_*.log")):
         stale.unlink()
     exe = nvcc()
@@ -106,24 +133,11 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         o = OBJ / f"{name}.o"
         objs.append(o)
         jobs.append(([exe, *NVCC_FLAGS, "-c", str(CSRC / f"sl8_{name}.cu"), "-o", str(o)], OBJ / f"{name}.log", verbose))
-    binding = OBJ / "torch.o"
-    jobs.append((binding_compile(binding), OBJ / "torch.log", verbose))
     with cf.ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as pool:
         list(pool.map(compile_one, jobs))
-    link = [exe, *ARCH_FLAGS, "-shared", "-o", str(LIB), *map(str, objs), "-cudart", "static"]
-    res = subprocess.run(link, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"link failed: {' '.join(link)}\n{res.stdout}\n{res.stderr}")
-    link = binding_link(binding)
-    res = subprocess.run(link, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"link failed: {' '.join(link)}\n{res.stdout}\n{res.stderr}")
-    bench = [exe, *ARCH_FLAGS, "-O3", "-std=c++17", "-lineinfo", str(CSRC / "sl8_bench.cu"), "-o", str(BENCH),
-             f"-L{LIB.parent}", "-lsiglip_fp8", "-lcublasLt", "-ldl", "-Xlinker", "-rpath=$ORIGIN", "-cudart", "static"]
-    res = subprocess.run(bench, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"bench host build failed: {' '.join(bench)}\n{res.stdout}\n{res.stderr}")
-    return LIB
+    run_link([exe, *ARCH_FLAGS, "-shared", "-o", str(LIB), *map(str, objs), "-cudart", "static"])
+    run_link([exe, *ARCH_FLAGS, "-O3", "-std=c++17", "-lineinfo", str(CSRC / "sl8_bench.cu"), "-o", str(BENCH),
+              f"-L{LIB.parent}", "-lsiglip_fp8", "-lcublasLt", "-ldl", "-Xlinker", "-rpath=$ORIGIN", "-cudart", "static"])
 
 
 def resource_report() -> str:

@@ -348,4 +348,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "sl8_torch", nullptr, -1, methods, 
 
 }  // namespace
 
-extern "C" __attribute__((visibility("default"))) PyObject* PyInit_sl8_torch(void) { return PyModule_Create(&module); }
+extern "C" __attribute__((visibility("default"))) PyObject* PyInit_sl8_torch(void) {
+    PyObject* m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "torch_version", SL8_TORCH_VERSION) != 0) Py_CLEAR(m);     // the torch whose headers this was compiled with
+    return m;
+}

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes as C
 import functools
+import warnings
 from typing import Optional
 
 import torch
@@ -39,7 +40,7 @@ class Engine:
         if rc != _l.SL8_OK:
             raise _l.SL8Error(rc, self._lib.sl8_last_error_string(None).decode())
         self._handle = self._h.value
-        self._native       # (missing: raises here, not in the first call)
+        self._native       # (looked for here and not in the first call)
 
     # ------------------------------------------------------------------ plumbing
     def close(self) -> None:
@@ -72,10 +73,14 @@ class Engine:
     # A call whose operands are all as they should be goes through the extension module (csrc/sl8_torch.cpp), which checks
     # and launches without Python in between: 8.9 -> 4 - 5 us a call (one image through a block, eight launches: 71 -> 51 us).
     # It answers None to anything else, and the method goes on in Python: there the same checks raise, and unusual tensors
-    # are read through their own attributes.
+    # are read through their own attributes.  Without the module (or with one built for another torch) every call goes there.
     @functools.cached_property
     def _native(self):
-        return _l.load_binding()
+        try:
+            return _l.load_binding()
+        except _l.SL8Error as e:
+            warnings.warn(f"calls take about 5 us longer: {e}", RuntimeWarning, stacklevel=3)
+            return _l.NoBinding()
 
     def _done(self, r):
         """The output of a call the extension took (a negative status raises)."""

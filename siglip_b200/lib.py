@@ -110,14 +110,30 @@ def load_library() -> C.CDLL:
 
 
 def load_binding():
-    """The extension module that takes torch tensors to the entry points of libsiglip_fp8.so (csrc/sl8_torch.cpp)."""
+    """The extension module that takes torch tensors to the entry points of libsiglip_fp8.so (csrc/sl8_torch.cpp).  SL8Error
+    where it is missing or belongs to another torch or interpreter: its calls can all be made without it."""
     global _binding
     if _binding is None:
+        import torch
+        again = "run `python -m siglip_b200.build`"
         if not _BINDING_PATH.exists():
-            raise SL8Error(SL8_ERR_CUDA, f"{_BINDING_PATH} is missing: run `python -m siglip_b200.build`; there is no fallback path")
+            raise SL8Error(SL8_ERR_CUDA, f"{_BINDING_PATH} is missing: {again}")
         loader = importlib.machinery.ExtensionFileLoader("sl8_torch", str(_BINDING_PATH))
         spec = importlib.util.spec_from_file_location("sl8_torch", str(_BINDING_PATH), loader=loader)
-        module = importlib.util.module_from_spec(spec)
-        loader.exec_module(module)
+        try:
+            module = importlib.util.module_from_spec(spec)
+            loader.exec_module(module)
+        except ImportError as e:
+            raise SL8Error(SL8_ERR_CUDA, f"{_BINDING_PATH} does not load ({e}): {again}") from e
+        built_for = getattr(module, "torch_version", "of another build")
+        if built_for != torch.__version__:
+            raise SL8Error(SL8_ERR_CUDA, f"{_BINDING_PATH} was compiled for torch {built_for}, this is {torch.__version__}: {again}")
         _binding = module
     return _binding
+
+
+class NoBinding:
+    """In the place of the extension module: takes no call, and every method goes on in Python."""
+
+    def __getattr__(self, name):
+        return lambda *args: None

@@ -1,6 +1,9 @@
 """What the calls on device tensors refuse before any launch, and what they let through, with and without the extension module
 in front of the C ABI.  No GPU: the calls meet a library that writes their arguments down (tests/fake_abi.py)."""
 import json
+import shutil
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -202,6 +205,35 @@ def test_a_throw_inside_the_extension_is_an_exception(folder):
     assert r.returncode == 0, f"the process died ({r.returncode}): {r.stderr[-2000:]}"
     for name, routes in json.loads(r.stdout.splitlines()[-1]).items():
         assert routes["extension"][0] and not routes["extension"][2], (name, routes)
+
+
+@pytest.mark.parametrize("state", ["missing", "not a module", "another torch"])
+def test_without_the_extension_the_calls_go_through_python(folder, tmp_path, state):
+    """An engine needs libsiglip_fp8.so; a missing or stale extension module is said, and costs time only."""
+    shutil.copy(folder / "libsiglip_fp8.so", tmp_path)
+    if state == "not a module":
+        (tmp_path / "sl8_torch.so").write_text("no ELF file")
+    if state == "another torch":
+        shutil.copy(folder / "sl8_torch.so", tmp_path)
+    pretend = "import torch; torch.__version__ = '0.0.1'; " if state == "another torch" else ""
+    code = (f"{pretend}import pathlib, warnings; from tests import fake_abi, test_operand_checks as t\n"
+            "with warnings.catch_warnings(record=True) as said:\n    warnings.simplefilter('always')\n"
+            f"    fast, _, calls = fake_abi.engines(pathlib.Path({str(tmp_path)!r}))\n"
+            "assert any('python -m siglip_b200.build' in str(w.message) for w in said), said\n"
+            "t.TAKEN['bias_fc1_bf16'](fast); t.TAKEN['out_quantize'](fast); assert len(calls()) == 2")
+    r = subprocess.run([sys.executable, "-c", code], cwd=fake_abi.ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+
+
+def test_the_build_asks_which_torch_the_extension_was_built_for(tmp_path, monkeypatch):
+    from siglip_b200 import build
+    monkeypatch.setattr(build, "BINDING", tmp_path / "sl8_torch.so")
+    assert not build.binding_current()
+    build.BINDING.touch()
+    (tmp_path / "sl8_torch.tag").write_text(build.torch_tag())
+    assert build.binding_current()
+    (tmp_path / "sl8_torch.tag").write_text("0.0.1 cpython-38")
+    assert not build.binding_current()
 
 
 @pytest.mark.gpu
