@@ -95,7 +95,7 @@ def binding_link(obj: Path) -> list[str]:
     import torch
     libs = Path(torch.__file__).parent / "lib"
     return [os.environ.get("CXX", "g++"), "-shared", "-o", str(BINDING), str(obj), f"-L{LIB.parent}", "-lsiglip_fp8", f"-L{libs}",
-            "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"]
+            "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN,--disable-new-dtags"]
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:

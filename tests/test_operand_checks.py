@@ -1,6 +1,7 @@
 """What the calls on device tensors refuse before any launch, and what they let through, with and without the extension module
 in front of the C ABI.  No GPU: the calls meet a library that writes their arguments down (tests/fake_abi.py)."""
 import json
+import os
 import shutil
 import subprocess
 import sys
@@ -205,6 +206,15 @@ def test_a_throw_inside_the_extension_is_an_exception(folder):
     assert r.returncode == 0, f"the process died ({r.returncode}): {r.stderr[-2000:]}"
     for name, routes in json.loads(r.stdout.splitlines()[-1]).items():
         assert routes["extension"][0] and not routes["extension"][2], (name, routes)
+
+
+def test_the_extension_calls_the_library_beside_it(folder, tmp_path):
+    """Another copy of the library on LD_LIBRARY_PATH must not get the handles of the one the engine loaded."""
+    other = tmp_path / "libsiglip_fp8.so"
+    (tmp_path / "other.c").write_text("int nothing;")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(other), str(tmp_path / "other.c")], check=True)      # holds none of the entry points
+    r = fake_abi.run_child(folder, __name__, "OUT_TAKEN", LD_LIBRARY_PATH=f"{tmp_path}:{os.environ.get('LD_LIBRARY_PATH', '')}")
+    assert r.returncode == 0 and "RuntimeWarning" not in r.stderr, r.stderr
 
 
 @pytest.mark.parametrize("state", ["missing", "not a module", "another torch"])
