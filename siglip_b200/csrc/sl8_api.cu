@@ -98,14 +98,20 @@ const VariantCost kVariantCost[] = {
     {COST_PE, 17, 6.74f, 0.257f, 0.574f, 2.88f},
 };
 
-int cheapest_variant(CostClass cls, int slot, long long M, int N, int K) {
+// CTAs, or pairs of them, that a launch on this handle's GPU can spread over (a B200's 148 SMs without a handle).
+long long clusters_of(sl8_handle_t h, const VariantEntry* v) {
+    const int clusters = (h ? h->sm_count : 148) / v->cg;
+    return h && h->max_clusters_override > 0 && clusters > h->max_clusters_override ? h->max_clusters_override : clusters;
+}
+
+int cheapest_variant(sl8_handle_t h, CostClass cls, int slot, long long M, int N, int K) {
     int best = 1;
     float best_us = 3.4e38f;
     for (const VariantCost& c : kVariantCost) {
         const VariantEntry* v = c.cls == cls ? variant(c.variant) : nullptr;
         if (!v || !v->kernel[slot]) continue;
-        const long long tiles = ((M + 128 * v->cg - 1) / (128 * v->cg)) * ((N + v->tn - 1) / v->tn), ctas = 148 / v->cg;
-        const float rounds = static_cast<float>((tiles + ctas - 1) / ctas), k_blocks = static_cast<float>((K + 127) / 128);
+        const long long tiles = ((M + 128 * v->cg - 1) / (128 * v->cg)) * ((N + v->tn - 1) / v->tn), clusters = clusters_of(h, v);
+        const float rounds = static_cast<float>((tiles + clusters - 1) / clusters), k_blocks = static_cast<float>((K + 127) / 128);
         const float later = k_blocks * c.next > c.tile ? k_blocks * c.next : c.tile;
         const float us = c.start + k_blocks * c.first + (rounds - 1.0f) * later;
         if (us < best_us) best_us = us, best = c.variant;
@@ -113,10 +119,10 @@ int cheapest_variant(CostClass cls, int slot, long long M, int N, int K) {
     return best;
 }
 
-int pick_variant(int op, int out_dtype, long long M, int N, int K, unsigned flags) {
+int pick_variant(sl8_handle_t h, int op, int out_dtype, long long M, int N, int K, unsigned flags) {
     const int slot = kernel_slot(op, out_dtype);
-    if (op == SL8_OP_FC1_GELU && (flags & SL8_FLAG_NO_ACTIVATION)) return cheapest_variant(COST_NONE, slot, M, N, K);
-    if (op == SL8_OP_FC1_GELU && (flags & SL8_FLAG_GELU_HW_TANH)) return cheapest_variant(COST_TANH, slot, M, N, K);
+    if (op == SL8_OP_FC1_GELU && (flags & SL8_FLAG_NO_ACTIVATION)) return cheapest_variant(h, COST_NONE, slot, M, N, K);
+    if (op == SL8_OP_FC1_GELU && (flags & SL8_FLAG_GELU_HW_TANH)) return cheapest_variant(h, COST_TANH, slot, M, N, K);
     // A (layer, N, K) the committed sweep covers: the row with the largest m_min <= M decides.
     int swept = -1;
     long long swept_m = -1;
@@ -129,7 +135,7 @@ int pick_variant(int op, int out_dtype, long long M, int N, int K, unsigned flag
     }
     // (the sweep times bf16 outputs; a variant that has no kernel for this output type is passed over)
     if (swept >= 0 && swept < SL8_NUM_VARIANTS && variant(swept) && variant(swept)->kernel[slot]) return swept;
-    return cheapest_variant(op == SL8_OP_PATCH_EMBED ? COST_PE : op == SL8_OP_FC2_RESIDUAL ? COST_FC2 : COST_GELU, slot, M, N, K);
+    return cheapest_variant(h, op == SL8_OP_PATCH_EMBED ? COST_PE : op == SL8_OP_FC2_RESIDUAL ? COST_FC2 : COST_GELU, slot, M, N, K);
 }
 
 struct Problem {
@@ -260,7 +266,7 @@ int run(sl8_handle_t h, const Problem& q, cudaStream_t stream) {
     DeviceGuard guard(h->device);
     if (!guard.ok) return fail(h, SL8_ERR_CUDA, "cudaSetDevice failed");
 
-    int vid = h->forced_variant >= 0 ? h->forced_variant : pick_variant(q.op, q.out_dtype, q.M, q.N, q.K, q.flags);
+    int vid = h->forced_variant >= 0 ? h->forced_variant : pick_variant(h, q.op, q.out_dtype, q.M, q.N, q.K, q.flags);
     const VariantEntry* v = variant(vid);
     if (!v) return fail(h, SL8_ERR_INVALID_VALUE, "no such kernel variant");
     const int slot = kernel_slot(q.op, q.out_dtype);
@@ -808,14 +814,13 @@ SL8_API int sl8_describe_variant(int variant_id, sl8_config* out) {
 
 SL8_API int sl8_query_config(sl8_handle_t h, int op, int out_dtype, int64_t M, int N, int K, sl8_config* out) {
     if (!out || M < 1 || N < 1 || K < 1 || op < 0 || op > 2) return SL8_ERR_INVALID_VALUE;
-    int vid = (h && h->forced_variant >= 0) ? h->forced_variant : pick_variant(op, out_dtype, M, N, K, 0u);
+    int vid = (h && h->forced_variant >= 0) ? h->forced_variant : pick_variant(h, op, out_dtype, M, N, K, 0u);
     const VariantEntry* v = variant(vid);
     if (!v) return SL8_ERR_INVALID_VALUE;
     const int slot = kernel_slot(op, out_dtype);
     const int tile_m = 128 * v->cg;
     const long long nt = ((M + tile_m - 1) / tile_m) * ((N + v->tn - 1) / v->tn);
-    const int sms = h ? h->sm_count : 148;
-    long long clusters = sms / v->cg;
+    long long clusters = clusters_of(h, v);
     if (nt < clusters) clusters = nt;
     fill_config(v, slot, (int)clusters * v->cg, out);
     return SL8_OK;

@@ -4,6 +4,7 @@ cost model draws: one tile, a last tile of 16 columns, a full round of tiles and
 import pytest
 import torch
 
+import siglip_b200
 from siglip_b200 import lib as L, synth
 
 pytestmark = pytest.mark.gpu
@@ -40,3 +41,14 @@ def test_the_picked_variant_agrees_with_the_general_one(engine, M, N, K):
             engine.set_variant(-1)
         engine.device_status()
         assert torch.equal(got.view(torch.uint8), want.view(torch.uint8)), f"call {i} at {M} x {N} x {K}"
+
+
+def test_the_pick_follows_the_ctas_a_launch_may_use(engine, monkeypatch):
+    """A handle held to eight CTAs (or pairs) has many rounds of tiles where the whole chip has less than one."""
+    for op, M, N, K, whole, held in ((2, 2048, 768, 768, 18, 17), (1, 4096, 512, 1600, 18, 15)):
+        assert engine.query_config(op, M, N, K)["variant_id"] == whole
+        monkeypatch.setenv("SL8_MAX_CLUSTERS", "8")
+        with siglip_b200.Engine(0) as few:
+            cfg = few.query_config(op, M, N, K)
+        monkeypatch.delenv("SL8_MAX_CLUSTERS")
+        assert cfg["variant_id"] == held and cfg["grid"] == 8 * cfg["cta_group"]
