@@ -284,10 +284,11 @@ int sl8_mlp_chain_fp8_host(sl8_handle_t h,
 
 /* ---- dispatch ------------------------------------------------------------------------- */
 
-/* Variant the dispatch table selects for (op, out_dtype, M, N, K) and flags = 0; the reference has a
- * single compile-time configuration (kernel_common.cuh:18-51,86-88).  An FC1 call with SL8_FLAG_NO_ACTIVATION or
- * SL8_FLAG_GELU_HW_TANH runs the eight-epilogue-warp variant where this answers with a sixteen-warp one. */
+/* Variant that a call of layer `op` with these sizes and `flags` runs, and its grid: from the dispatch table for the (layer, N, K)
+ * it holds, by the cost model otherwise and for FC1 calls with SL8_FLAG_NO_ACTIVATION or SL8_FLAG_GELU_HW_TANH.  (The
+ * reference has a single compile-time configuration, kernel_common.cuh:18-51,86-88.)  sl8_query_config: flags = 0. */
 int sl8_query_config(sl8_handle_t h, int op, int out_dtype, int64_t M, int N, int K, sl8_config* out);
+int sl8_query_config_flags(sl8_handle_t h, int op, int out_dtype, unsigned flags, int64_t M, int N, int K, sl8_config* out);
 
 /* Number of compiled variants, and the description of variant `variant_id`. */
 int sl8_num_variants(void);

@@ -4,7 +4,7 @@ FC2 + bias + residual.
 
 The product is the C-ABI shared library ``libsiglip_fp8.so`` (declared in
 ``include/siglip_fp8.h``).  This package holds its CUDA sources (``csrc/``), its build
-step (``build.py``), a ctypes binding (``lib.py``), the host-side layer interface over
+step (``build.py``), a binding (``lib.py``), the host-side layer interface over
 torch tensors (``layers.py``) and the seeded synthetic operands of the benchmark
 configurations (``synth.py``).  There is no CPU fallback: without the built library, or
 without an sm_100 device, the calls raise.

@@ -812,9 +812,9 @@ SL8_API int sl8_describe_variant(int variant_id, sl8_config* out) {
     return SL8_OK;
 }
 
-SL8_API int sl8_query_config(sl8_handle_t h, int op, int out_dtype, int64_t M, int N, int K, sl8_config* out) {
+SL8_API int sl8_query_config_flags(sl8_handle_t h, int op, int out_dtype, unsigned flags, int64_t M, int N, int K, sl8_config* out) {
     if (!out || M < 1 || N < 1 || K < 1 || op < 0 || op > 2) return SL8_ERR_INVALID_VALUE;
-    int vid = (h && h->forced_variant >= 0) ? h->forced_variant : pick_variant(h, op, out_dtype, M, N, K, 0u);
+    int vid = (h && h->forced_variant >= 0) ? h->forced_variant : pick_variant(h, op, out_dtype, M, N, K, flags);
     const VariantEntry* v = variant(vid);
     if (!v) return SL8_ERR_INVALID_VALUE;
     const int slot = kernel_slot(op, out_dtype);
@@ -824,6 +824,10 @@ SL8_API int sl8_query_config(sl8_handle_t h, int op, int out_dtype, int64_t M, i
     if (nt < clusters) clusters = nt;
     fill_config(v, slot, (int)clusters * v->cg, out);
     return SL8_OK;
+}
+
+SL8_API int sl8_query_config(sl8_handle_t h, int op, int out_dtype, int64_t M, int N, int K, sl8_config* out) {
+    return sl8_query_config_flags(h, op, out_dtype, 0u, M, N, K, out);
 }
 
 SL8_API int sl8_set_variant(sl8_handle_t h, int variant_id) {

@@ -1,6 +1,6 @@
 // sl8_dispatch_table.h -- GENERATED by `python -m siglip_b200.sweep --emit-table siglip_b200/sweeps/b200.csv`.
 // One row per (layer, N, K, smallest M) -> kernel variant, from the sweep on B200; pick_variant() takes the
-// row with the largest m_min <= M for an exact (layer, N, K) match and falls back to its rules otherwise.
+// row with the largest m_min <= M for an exact (layer, N, K) match and asks its cost model otherwise.
 #pragma once
 
 struct Sl8DispatchRow { int op; int n; int k; long long m_min; int variant; };

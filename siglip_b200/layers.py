@@ -71,7 +71,7 @@ class Engine:
         return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
     # A call whose operands are all as they should be goes through the extension module (csrc/sl8_torch.cpp), which checks
-    # and launches without Python in between: 8.9 -> 4 - 5 us a call (one image through a block, eight launches: 71 -> 51 us).
+    # and launches without Python in between: 8.9 -> 4 - 5 us a call (one image through a block, seven launches from six calls: 71 -> 51 us).
     # It answers None to anything else, and the method goes on in Python: there the same checks raise, and unusual tensors
     # are read through their own attributes.  Without the module (or with one built for another torch) every call goes there.
     @functools.cached_property
@@ -485,9 +485,9 @@ class Engine:
         return out
 
     # ------------------------------------------------------------------ dispatch and watchdog
-    def query_config(self, op: int, M: int, N: int, K: int, out_dtype: int = _l.SL8_OUT_BF16) -> dict:
+    def query_config(self, op: int, M: int, N: int, K: int, out_dtype: int = _l.SL8_OUT_BF16, flags: int = 0) -> dict:
         cfg = _l.Config()
-        self._check(self._lib.sl8_query_config(self._h, op, out_dtype, M, N, K, C.byref(cfg)))
+        self._check(self._lib.sl8_query_config_flags(self._h, op, out_dtype, int(flags), M, N, K, C.byref(cfg)))
         return cfg.as_dict()
 
     def set_variant(self, variant_id: int) -> None:

@@ -1,4 +1,5 @@
-"""ctypes binding of libsiglip_fp8.so: one Python function per symbol of include/siglip_fp8.h.
+"""Binding of libsiglip_fp8.so: through ctypes one function per symbol of include/siglip_fp8.h, and the extension module
+that takes torch tensors to the layer calls among them.
 
 The library is looked up in-tree (``siglip_b200/lib/libsiglip_fp8.so``, produced by
 ``python -m siglip_b200.build``).  A missing library is an error, never a fallback.
@@ -76,6 +77,7 @@ SIGNATURES = {
     "sl8_mlp_chain_fp8": (_I, [_P, _P, _I64, _P, _I64, _P, _P, _P, _P, _I64, _P, _P, _I64, _P, _P, _P, _I64, _P, _I64, _I64, _I, _I, _U, _P]),
     "sl8_mlp_chain_fp8_host": (_I, [_P, _P, _I64, _P, _I64, _F, _F, _P, _F, _P, _I64, _F, _P, _P, _I64, _P, _I64, _I64, _I, _I, _U]),
     "sl8_query_config": (_I, [_P, _I, _I, _I64, _I, _I, C.POINTER(Config)]),
+    "sl8_query_config_flags": (_I, [_P, _I, _I, _U, _I64, _I, _I, C.POINTER(Config)]),
     "sl8_num_variants": (_I, []),
     "sl8_describe_variant": (_I, [_I, C.POINTER(Config)]),
     "sl8_set_variant": (_I, [_P, _I]),

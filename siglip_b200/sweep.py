@@ -111,7 +111,7 @@ def best_rows(rows: list[dict], keep_margin: float = 0.02) -> list[dict]:
 def emit_header(table: list[dict], source: str, path: Path = TABLE_HEADER) -> str:
     lines = ["// sl8_dispatch_table.h -- GENERATED by `python -m siglip_b200.sweep --emit-table " + source + "`.",
              "// One row per (layer, N, K, smallest M) -> kernel variant, from the sweep on B200; pick_variant() takes the",
-             "// row with the largest m_min <= M for an exact (layer, N, K) match and falls back to its rules otherwise.",
+             "// row with the largest m_min <= M for an exact (layer, N, K) match and asks its cost model otherwise.",
              "#pragma once", "",
              "struct Sl8DispatchRow { int op; int n; int k; long long m_min; int variant; };", "",
              "static const Sl8DispatchRow kSl8DispatchTable[] = {"]
