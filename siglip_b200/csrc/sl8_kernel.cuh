@@ -167,6 +167,8 @@ struct KernelTraits {
     static_assert(STAGE_BYTES % 1024 == 0, "every operand tile must start on a swizzle-atom boundary");
     static_assert(COLS_PER_WARP % REGION_COLS == 0, "a warp stores whole staging regions");
     static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KiB a CTA may use");
+    // A launch that waits for the one ahead of it (pdl_wait) already holds tensor memory: it must not sit on that one's SMs.
+    static_assert(2 * SMEM_BYTES > 228 * 1024, "two CTAs must not fit one SM");
 };
 
 struct WaitCtx {
