@@ -216,8 +216,8 @@ def test_fc1_fc2_chain_through_e4m3(engine, oracle):
 def test_mlp_chain_entry_points(engine, oracle):
     """sl8_mlp_chain_fp8 (device operands) and sl8_mlp_chain_fp8_host (host operands, slabs on three streams, the
     hidden activations never leaving the GPU): the hidden codes against the oracle's FC1, D against the oracle's FC2
-    run on those very codes, and the host form bit-identical to the device form on 25 000 rows (three slabs of 11 520 rows:
-    64 MiB of A + residual + D each)."""
+    run on those very codes, and the host form bit-identical to the device form on 25 000 rows (nine slabs of up to
+    3 072 rows: an eighth of the call's A + residual + D each)."""
     import siglip_b200.lib as L
     M, D_MODEL, D_FF = 1500, 1152, 4304
     p1 = synth.make_fc1(M, D_FF, D_MODEL, seed=41, device=DEV)
@@ -352,3 +352,24 @@ def test_host_operand_entry_points(engine, oracle):
     rows = np.r_[0:300, 33000:33300, M - 300:M]
     ref = oracle.fc1_gelu(np.ascontiguousarray(p.A.numpy()[rows]), p.B.numpy(), p.scale_a, p.scale_b, bits(p.bias))
     check_bf16(out.view(torch.uint16).numpy()[rows], ref, "fc1 host operands")
+
+
+@pytest.mark.parametrize("layer,M", [("fc2", m) for m in (4864, 4865, 39715, 39725, 254195, 254210)] + [("pe", m) for m in (9472, 9473, 77095, 77105, 493445, 493455)])
+def test_host_slabs_at_the_edges_of_their_rule(engine, layer, M):
+    """One slab and one row more; on both sides of where an eighth of the call is 10 MiB and 64 MiB of bus traffic: the host form
+    gives what the device form gives.  (Per row: 2 112 bytes of A, residual and D here, 1 088 of A and D for the table.)"""
+    N, K, period = 512, 64, 100
+    g = torch.Generator(device=DEV).manual_seed(M)
+    codes = lambda r: torch.randint(0, 256, (r, K), generator=g, device=DEV, dtype=torch.uint8) & 0xBF
+    A, B = codes(M), codes(N)
+    side = torch.randn((M if layer == "fc2" else period, N), generator=g, device=DEV).to(torch.bfloat16)
+    host = lambda t: torch.empty(t.shape, dtype=t.dtype).copy_(t)
+    out = torch.empty((M, N), dtype=torch.bfloat16)
+    if layer == "fc2":
+        want = engine.fc2_residual(A, B, None, side)
+        engine.fc2_residual_host(host(A), host(B), None, host(side), out)
+    else:
+        want = engine.patch_embed(A, B, side, row_phase=7)
+        engine.patch_embed_host(host(A), host(B), host(side), out, row_phase=7)
+    engine.device_status()
+    assert torch.equal(out.to(DEV).view(torch.uint8), want.view(torch.uint8))

@@ -1,5 +1,7 @@
 """Kernels that become resident while the one ahead of them on the stream still runs: calls that reuse each other's buffers,
 issued back to back and from a captured graph, must give bit for bit what they give with a synchronisation after each."""
+import threading
+
 import pytest
 import torch
 
@@ -82,3 +84,37 @@ def test_calls_behind_a_fork_and_a_fill_are_captured_in_order(engine):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, want)
+
+
+def test_two_threads_on_their_own_streams(engine):
+    """Chains of overlapped launches from two threads at once, through one handle: each stream keeps its own order."""
+    chains = [_chain(engine, rows, d, ff, seed=rows) for rows, d, ff in ((729, 1152, 4304), (1300, 768, 3072))]
+    wants = []
+    for run, state, _ in chains:
+        run(torch.cuda.synchronize)
+        wants.append([t.clone() for t in state])
+    errors = []
+
+    def work(i):
+        run, state, x0 = chains[i]
+        stream = torch.cuda.Stream()
+        try:
+            with torch.cuda.stream(stream):
+                for _ in range(10):
+                    state[0].copy_(x0)
+                    run(lambda: None)
+                    stream.synchronize()
+                    for t, want in zip(state, wants[i]):
+                        assert torch.equal(t.contiguous().view(torch.uint8), want.contiguous().view(torch.uint8))
+        except BaseException as e:      # noqa: BLE001 - handed to the test's own thread
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    engine.device_status()
+    if errors:
+        raise errors[0]
