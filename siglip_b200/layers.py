@@ -358,7 +358,9 @@ class Engine:
 
     def _codes_into(self, out: torch.Tensor, rows: int, cols: int) -> None:
         """A caller-supplied buffer for [rows, cols] codes: one code after the other in a row, and at least that large (the
-        library knows its address and row pitch, not where it ends)."""
+        library knows its address and row pitch, not where it ends).  A pitch below a row's codes it refuses itself."""
+        if out.dim() > 0 and out.stride(0) < cols:
+            return
         self._readable("out", out)
         if out.dtype not in self._E4M3_TYPES:
             raise TypeError(f"out has dtype {out.dtype}; codes are float8_e4m3fn or uint8")
@@ -389,7 +391,7 @@ class Engine:
             self._codes_into(out, rows, K)
             pitch = out.stride(0)         # a pad of less than 128 bytes is filled with zeros, the last row's too
             written = pitch if pitch - K < 128 else (K + 15) // 16 * 16
-            if out.storage_offset() + (rows - 1) * pitch + written > out.untyped_storage().nbytes():
+            if pitch >= K and out.storage_offset() + (rows - 1) * pitch + written > out.untyped_storage().nbytes():
                 raise ValueError("out ends inside the pad of its last row, which is written with the row")
         self._check(self._lib.sl8_patchify_quantize_e4m3(
             self._h, pixels.data_ptr(), self._dt(pixels), images, Cc, H, W, int(patch), _ptr(scale), out.data_ptr(),

@@ -37,7 +37,6 @@ OUT_REFUSED = {
     "quantize_three_dimensions": lambda e: e.quantize_e4m3(x(), one(), out=cuda(2, 4, 32), **S),
     "layernorm_few_rows": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, one(), out=cuda(7, 32), **S),
     "layernorm_wide_type": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, one(), out=cuda(8, 32, dtype=F32), **S),
-    "layernorm_one_dimension": lambda e: e.layernorm_quantize(x(), None, None, 1e-6, one(), out=cuda(256), **S),
     "patchify_few_rows": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(11, 768), **S),
     "patchify_few_columns": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(12, 760, stride=(768, 1)), **S),
     "patchify_wide_type": lambda e: e.patchify_quantize(pixels(), 16, one(), out=cuda(12, 768, dtype=BF16), **S),
