@@ -373,3 +373,22 @@ def test_host_slabs_at_the_edges_of_their_rule(engine, layer, M):
         engine.patch_embed_host(host(A), host(B), host(side), out, row_phase=7)
     engine.device_status()
     assert torch.equal(out.to(DEV).view(torch.uint8), want.view(torch.uint8))
+
+
+@pytest.mark.parametrize("period", [1, 3, 49, 100, 127, 196, 300])
+def test_tables_with_and_without_padding_agree(engine, period):
+    """Boxes of a table that ends in the middle of them are gathered row by row: bit for bit what a padded table gives."""
+    M, N, K = 1000, 400, 80
+    g = torch.Generator(device=DEV).manual_seed(period)
+    codes = lambda r: torch.randint(0, 256, (r, K), generator=g, device=DEV, dtype=torch.uint8) & 0xBF
+    A, B, table = codes(M), codes(N), torch.randn((period, N), generator=g, device=DEV).to(torch.bfloat16)
+    for phase in (0, period - 1, 2 * period + 1):
+        for v in (-1, 1, 3, 17, 18):
+            engine.set_variant(v)
+            try:
+                got = engine.patch_embed(A, B, table, row_phase=phase)
+                want = engine.patch_embed(A, B, engine.padded_table(table), period=period, row_phase=phase)
+            finally:
+                engine.set_variant(-1)
+            engine.device_status()
+            assert torch.equal(got.view(torch.uint8), want.view(torch.uint8)), (phase, v)
