@@ -122,6 +122,17 @@ at::Tensor output(Args& a, const at::Tensor* given, const at::Tensor& A, int64_t
     return *given;
 }
 
+// Whether t has room for [rows, cols] codes at its own row pitch.
+bool holds_codes(const at::Tensor& t, int64_t rows, int64_t cols) {
+    return codes(t) && t.dim() == 2 && t.size(0) >= rows && t.size(1) >= cols && (t.stride(1) == 1 || t.size(1) == 1);
+}
+
+// `out`, or new codes beside x: [rows, cols] of rows on 128-byte lines.  Undefined if `out` has no room for them.
+at::Tensor codes_into(const at::Tensor* given, const at::Tensor& x, int64_t rows, int64_t cols) {
+    if (!given) return at::empty({rows, (cols + 127) / 128 * 128}, x.options().dtype(at::kByte)).narrow(1, 0, cols);
+    return holds_codes(*given, rows, cols) ? *given : at::Tensor();
+}
+
 PyObject* result(int rc, const at::Tensor& out) {
     if (rc != SL8_OK) return PyLong_FromLong(rc);
     return THPVariable_Wrap(out);
@@ -225,26 +236,27 @@ SL8_PY(mlp_chain) {
     if (!a.ok) Py_RETURN_NONE;
     Gemm g(a);                                   // [M, d_model] x [d_ff, d_model]
     if (!a.ok) Py_RETURN_NONE;
-    bool has_b1, has_b2, has_out;
+    bool has_b1, has_b2, has_hidden, has_out;
     const at::Tensor* bias1 = a.optional(has_b1);
     const at::Tensor* W2 = a.tensor();
     const at::Tensor* bias2 = a.optional(has_b2);
     const at::Tensor* residual = a.tensor();
     const float *sa = a.scale(), *s1 = a.scale(), *s2 = a.scale();
     const float* sh = a.scale();
-    const at::Tensor* hidden = a.tensor();
+    const at::Tensor* hidden = a.optional(has_hidden);
     const at::Tensor* given = a.optional(has_out);
     unsigned flags = static_cast<unsigned>(a.integer());
     if (!a.ok || !sh || !codes(*W2) || !shaped(*W2, g.K, g.N) || residual->scalar_type() != at::kBFloat16 || !shaped(*residual, g.M, g.K) ||
-        !codes(*hidden) || !shaped(*hidden, g.M, g.N))
+        (has_hidden && (!codes(*hidden) || !shaped(*hidden, g.M, g.N))))
         Py_RETURN_NONE;
     // One flag speaks for both: it is known before either is looked at.
     if ((has_b1 && bias1->scalar_type() == at::kFloat) || (has_b2 && bias2->scalar_type() == at::kFloat)) flags |= SL8_FLAG_BIAS_F32;
     const void *const b1 = bias_of(a, bias1, g.N, flags), *const b2 = bias_of(a, bias2, g.K, flags);
     const at::Tensor out = output(a, given, *g.A, g.M, g.K, at::kBFloat16, false);
     if (!a.ok) Py_RETURN_NONE;
+    const at::Tensor scratch = codes_into(hidden, *g.A, g.M, g.N);
     const int rc = unlocked(sl8_mlp_chain_fp8, a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, s1,
-                            b1, hidden->mutable_data_ptr(), hidden->stride(0),
+                            b1, scratch.mutable_data_ptr(), scratch.stride(0),
                             sh, W2->const_data_ptr(), W2->stride(0), s2,
                             b2, residual->const_data_ptr(), residual->stride(0), out.mutable_data_ptr(),
                             out.stride(0), g.M, static_cast<int>(g.K), static_cast<int>(g.N), flags, a.stream());
@@ -257,11 +269,6 @@ int activation(const at::Tensor& t) { return t.scalar_type() == at::kFloat ? SL8
 // Rows of an activation, one element after the other, at a pitch of stride(0).
 bool rows_of(const at::Tensor& t) { return t.dim() == 2 && (t.stride(1) == 1 || t.size(1) == 1) && t.size(1) <= INT_MAX && activation(t) >= 0; }
 
-// Whether t has room for [rows, cols] codes at its own row pitch.
-bool holds_codes(const at::Tensor& t, int64_t rows, int64_t cols) {
-    return codes(t) && t.dim() == 2 && t.size(0) >= rows && t.size(1) >= cols && (t.stride(1) == 1 || t.size(1) == 1);
-}
-
 // h, device, stream, pixels, scale, out, patch
 SL8_PY(patchify_quantize) {
     HANDLE_TH_ERRORS
@@ -269,21 +276,24 @@ SL8_PY(patchify_quantize) {
     if (!a.ok) Py_RETURN_NONE;
     const at::Tensor* px = a.tensor();
     const float* scale = a.scale();
-    const at::Tensor* out = a.ok ? a.tensor() : nullptr;
+    bool has_out;
+    const at::Tensor* given = a.ok ? a.optional(has_out) : nullptr;
     const long long patch = a.ok ? a.integer() : 0;
     if (!a.ok || px->dim() != 4 || !px->is_contiguous() || activation(*px) < 0 || patch < 1) Py_RETURN_NONE;
     for (int i = 0; i < 4; i++)
         if (px->size(i) > INT_MAX) Py_RETURN_NONE;
     if (px->size(2) < patch || px->size(3) < patch) Py_RETURN_NONE;
     const int64_t rows = px->size(0) * (px->size(2) / patch) * (px->size(3) / patch), cols = px->size(1) * patch * patch;
-    if (rows < 1 || cols < 1 || !holds_codes(*out, rows, cols)) Py_RETURN_NONE;
+    if (rows < 1 || cols < 1) Py_RETURN_NONE;
+    const at::Tensor out = codes_into(given, *px, rows, cols);
+    if (!out.defined()) Py_RETURN_NONE;
     // (the kernel fills a pad of less than 128 bytes with zeros, the last row's too)
-    const int64_t pitch = out->stride(0), written = pitch - cols < 128 ? pitch : (cols + 15) / 16 * 16;
-    if (out->storage_offset() + (rows - 1) * pitch + written > static_cast<int64_t>(out->storage().nbytes())) Py_RETURN_NONE;
+    const int64_t pitch = out.stride(0), written = pitch - cols < 128 ? pitch : (cols + 15) / 16 * 16;
+    if (out.storage_offset() + (rows - 1) * pitch + written > static_cast<int64_t>(out.storage().nbytes())) Py_RETURN_NONE;
     const int rc = unlocked(sl8_patchify_quantize_e4m3, a.h, px->const_data_ptr(), activation(*px), static_cast<int>(px->size(0)), static_cast<int>(px->size(1)),
                             static_cast<int>(px->size(2)), static_cast<int>(px->size(3)), static_cast<int>(patch), scale,
-                            out->mutable_data_ptr(), out->stride(0), a.stream());
-    return result(rc, *out);
+                            out.mutable_data_ptr(), out.stride(0), a.stream());
+    return result(rc, out);
     END_HANDLE_TH_ERRORS
 }
 
@@ -315,11 +325,14 @@ SL8_PY(quantize_e4m3) {
     if (!a.ok) Py_RETURN_NONE;
     const at::Tensor* x = a.tensor();
     const float* scale = a.scale();
-    const at::Tensor* out = a.ok ? a.tensor() : nullptr;
-    if (!a.ok || !rows_of(*x) || !holds_codes(*out, x->size(0), x->size(1))) Py_RETURN_NONE;
+    bool has_out;
+    const at::Tensor* given = a.ok ? a.optional(has_out) : nullptr;
+    if (!a.ok || !rows_of(*x)) Py_RETURN_NONE;
+    const at::Tensor out = codes_into(given, *x, x->size(0), x->size(1));
+    if (!out.defined()) Py_RETURN_NONE;
     const int rc = unlocked(sl8_quantize_e4m3, a.h, x->const_data_ptr(), activation(*x), x->size(0), static_cast<int>(x->size(1)), x->stride(0), scale,
-                            out->mutable_data_ptr(), out->stride(0), a.stream());
-    return result(rc, *out);
+                            out.mutable_data_ptr(), out.stride(0), a.stream());
+    return result(rc, out);
     END_HANDLE_TH_ERRORS
 }
 
@@ -331,12 +344,15 @@ SL8_PY(layernorm_quantize) {
     const at::Tensor* x = a.tensor();
     const int64_t cols = a.ok && x->dim() == 2 ? x->size(1) : 0;
     const float *gamma = a.floats(cols), *beta = a.floats(cols), *scale = a.scale();
-    const at::Tensor* out = a.ok ? a.tensor() : nullptr;
+    bool has_out;
+    const at::Tensor* given = a.ok ? a.optional(has_out) : nullptr;
     const double eps = a.ok ? a.real() : 0.0;
-    if (!a.ok || !rows_of(*x) || !holds_codes(*out, x->size(0), x->size(1))) Py_RETURN_NONE;
+    if (!a.ok || !rows_of(*x)) Py_RETURN_NONE;
+    const at::Tensor out = codes_into(given, *x, x->size(0), x->size(1));
+    if (!out.defined()) Py_RETURN_NONE;
     const int rc = unlocked(sl8_layernorm_quantize_e4m3, a.h, x->const_data_ptr(), activation(*x), x->size(0), static_cast<int>(x->size(1)), x->stride(0), gamma, beta,
-                            static_cast<float>(eps), scale, out->mutable_data_ptr(), out->stride(0), a.stream());
-    return result(rc, *out);
+                            static_cast<float>(eps), scale, out.mutable_data_ptr(), out.stride(0), a.stream());
+    return result(rc, out);
     END_HANDLE_TH_ERRORS
 }
 

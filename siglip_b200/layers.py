@@ -298,12 +298,11 @@ class Engine:
                   out=None, flags: int = 0, stream=None) -> torch.Tensor:
         """D = FC2(e4m3(GELU(FC1(A)) / hidden_scale)) + residual: the block's MLP as one call (sl8_mlp_chain_fp8).
         ``hidden`` is the e4m3 scratch [M, d_ff] (uint8, row pitch a multiple of 16 bytes); allocated when None."""
-        if hidden is not None:
-            r = self._native.mlp_chain(self._handle, self.device, None if stream is None else self._stream(stream),
-                                       A, W1, bias1, W2, bias2, residual, scale_a, scale_w1, scale_w2,
-                                       hidden_scale, hidden, out, flags)
-            if r is not None:
-                return self._done(r)
+        r = self._native.mlp_chain(self._handle, self.device, None if stream is None else self._stream(stream),
+                                   A, W1, bias1, W2, bias2, residual, scale_a, scale_w1, scale_w2,
+                                   hidden_scale, hidden, out, flags)
+        if r is not None:
+            return self._done(r)
         M, d_ff, d_model = self._operands(A, W1)
         n2, k2 = W2.shape
         if (n2, k2) != (d_model, d_ff) or not _is_fp8(W2) or W2.stride(1) != 1:
@@ -370,7 +369,7 @@ class Engine:
     def patchify_quantize(self, pixels, patch: int, scale=None, *, out=None, pitch=None, stream=None) -> torch.Tensor:
         """pixels [images, C, H, W] (fp32 / bf16) -> A [images * (H // patch) * (W // patch), C * patch * patch] e4m3
         codes (uint8) at a row pitch that is a multiple of 128 bytes: the patch-embed GEMM's operand."""
-        if out is not None:
+        if pitch is None or out is not None:
             r = self._native.patchify_quantize(self._handle, self.device, None if stream is None else self._stream(stream),
                                                pixels, scale, out, patch)
             if r is not None:
@@ -413,10 +412,9 @@ class Engine:
 
     def quantize_e4m3(self, x, scale=None, *, out=None, stream=None) -> torch.Tensor:
         """e4m3 codes (uint8) of x / scale, row pitch a multiple of 128 bytes unless `out` is given."""
-        if out is not None:
-            r = self._native.quantize_e4m3(self._handle, self.device, None if stream is None else self._stream(stream), x, scale, out)
-            if r is not None:
-                return self._done(r)
+        r = self._native.quantize_e4m3(self._handle, self.device, None if stream is None else self._stream(stream), x, scale, out)
+        if r is not None:
+            return self._done(r)
         rows, cols = self._rows(x)
         self._floats("scale", scale)
         self._readable("scale", scale)
@@ -432,11 +430,10 @@ class Engine:
 
     def layernorm_quantize(self, x, gamma=None, beta=None, eps: float = 1e-6, scale=None, *, out=None, stream=None) -> torch.Tensor:
         """e4m3 codes (uint8) of LayerNorm(x) / scale: FC1's A operand, row pitch a multiple of 128 bytes."""
-        if out is not None:
-            r = self._native.layernorm_quantize(self._handle, self.device, None if stream is None else self._stream(stream),
-                                                x, gamma, beta, scale, out, eps)
-            if r is not None:
-                return self._done(r)
+        r = self._native.layernorm_quantize(self._handle, self.device, None if stream is None else self._stream(stream),
+                                            x, gamma, beta, scale, out, eps)
+        if r is not None:
+            return self._done(r)
         rows, cols = self._rows(x)
         for name, t, n in (("gamma", gamma, cols), ("beta", beta, cols), ("scale", scale, 1)):
             self._floats(name, t, n)
