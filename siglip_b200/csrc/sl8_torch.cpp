@@ -42,6 +42,10 @@ struct Args {
     sl8_stream_t stream() const {
         return current ? static_cast<sl8_stream_t>(c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream()) : given_stream;
     }
+    // A temporary of this call that its stream still uses when the call returns and the temporary goes.
+    void outlives(const at::Tensor& t) const {
+        if (!current) t.record_stream(c10::cuda::getStreamFromExternal(static_cast<cudaStream_t>(given_stream), static_cast<c10::DeviceIndex>(device)));
+    }
     // A plain strided tensor on the handle's GPU (subclasses, wrappers of a transform and the like go through Python).
     const at::Tensor* tensor() { return plain(v[at++]); }
     const at::Tensor* optional(bool& given) {
@@ -255,6 +259,7 @@ SL8_PY(mlp_chain) {
     const at::Tensor out = output(a, given, *g.A, g.M, g.K, at::kBFloat16, false);
     if (!a.ok) Py_RETURN_NONE;
     const at::Tensor scratch = codes_into(hidden, *g.A, g.M, g.N);
+    if (!hidden) a.outlives(scratch);
     const int rc = unlocked(sl8_mlp_chain_fp8, a.h, g.A->const_data_ptr(), g.A->stride(0), g.B->const_data_ptr(), g.B->stride(0), sa, s1,
                             b1, scratch.mutable_data_ptr(), scratch.stride(0),
                             sh, W2->const_data_ptr(), W2->stride(0), s2,

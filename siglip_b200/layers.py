@@ -9,6 +9,7 @@ tensors may be ``torch.float8_e4m3fn`` or raw ``torch.uint8`` codes.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import functools
 import warnings
@@ -221,9 +222,12 @@ class Engine:
         """fp32 bias [N] (or None) and fp32 pos [period, N] -> padded bf16 table of bf16(bias + pos)."""
         period, N = pos.shape
         self._on_device("pos", pos)
-        pos = pos.contiguous().float()
-        b = None if bias is None else bias.contiguous().float()
-        self._readable("bias", b)
+        self._readable("bias", bias)
+        # (converted on the stream that reads them)
+        with contextlib.nullcontext() if stream is None else torch.cuda.stream(torch.cuda.ExternalStream(self._stream(stream), device=self.device)):
+            pos = pos.contiguous().float()
+            b = None if bias is None else bias.contiguous().float()
+        self._readable("bias", b)         # (pinned memory does not survive a conversion)
         rows = self._lib.sl8_padded_table_rows(period)
         out = torch.empty((rows, N), dtype=torch.bfloat16, device=pos.device)
         self._check(self._lib.sl8_make_periodic_table(self._h, _ptr(b), pos.data_ptr(), period, N, out.data_ptr(),
@@ -314,6 +318,8 @@ class Engine:
         flags = self._bias_flags(flags, ("bias1", bias1, d_ff), ("bias2", bias2, d_model))
         if hidden is None:
             hidden = torch.empty((M, (d_ff + 127) // 128 * 128), dtype=torch.uint8, device=A.device)[:, :d_ff]
+            if stream is not None:        # it goes when this call returns, but the stream still uses it
+                hidden.record_stream(torch.cuda.ExternalStream(self._stream(stream), device=self.device))
         self._check_out(hidden, M, d_ff, self._E4M3_TYPES)
         for name, t in (("W2", W2), ("bias1", bias1), ("bias2", bias2), ("residual", residual)):
             self._on_device(name, t)

@@ -123,3 +123,28 @@ def test_subclasses_go_through_python_and_outputs_are_the_tensor_given():
     assert fast.fc1_gelu(o.A, torch.nn.Parameter(o.W1, requires_grad=False), o.b1, out=out) is out
     with pytest.raises(Exception):
         torch.func.vmap(lambda a: fast.fc1_gelu(a, o.W1, o.b1))(o.A.view(torch.uint8)[None])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("route", [0, 1])
+def test_hidden_activations_stay_until_the_stream_is_done(route):
+    """The scratch that mlp_chain allocates must not be handed out again while the stream it was given still has to use it."""
+    e, M, d, ff = _engines()[route], 2048, 256, 4096
+    g = torch.Generator(device=DEV).manual_seed(1)
+    codes = lambda r, c: torch.randint(0, 256, (r, c), generator=g, device=DEV, dtype=torch.uint8) & 0xBF
+    A, W1, W2, res, s = codes(M, d), codes(ff, d), codes(d, ff), torch.zeros((M, d), dtype=torch.bfloat16, device=DEV), torch.ones(1, device=DEV)
+    out, side = torch.empty_like(res), torch.cuda.Stream()
+    kw = dict(scale_a=s, scale_w1=s, scale_w2=s, hidden_scale=s, out=out)
+    e.mlp_chain(A, W1, None, W2, None, res, **kw)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.empty((M, ff), dtype=torch.uint8, device=DEV)
+    where = free.data_ptr()
+    del free                                       # the one free block of that size: the call's scratch
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)
+    e.mlp_chain(A, W1, None, W2, None, res, stream=side, **kw)
+    again = torch.empty((M, ff), dtype=torch.uint8, device=DEV)
+    assert not side.query() and again.data_ptr() != where
+    side.synchronize()
+    e.device_status()
