@@ -65,13 +65,13 @@ int kernel_slot(int op, int out_dtype) {
 //     start + k_blocks * first + (rounds - 1) * max(k_blocks * next, tile)
 // `start` is set-up, the first operands' way in and the last tile's epilogue; `first` a k-block of the first tile; a later tile
 // hides its mainloop (`next` per k-block, more than `first` when every SM asks L2) behind the epilogue ahead of it or the
-// other way round (`tile`: the epilogue's own pace).  The constants are fitted so that the cheapest variant by the formula is
-// the fastest one measured, over 18 (layer, N, K) from 512 to 4 800 wide and 50 to 186 624 rows (graph replays, every
-// variant): it is within 1 % of the fastest on average, 9 % at worst.  What it decides: 128 x 128 tiles on single CTAs with
+// other way round (`tile`: the epilogue's own pace).  The constants (sl8_cost_model.h) are fitted so that the cheapest variant by
+// the formula is the fastest one measured, from 512 to 4 800 wide and 50 to 186 624 rows: on that sweep (346 points that the table
+// leaves to it, sweeps/b200_model.csv) it is 0.1 - 1.1 % off the fastest on average, by class, and 9.3 % at worst.  What it decides: 128 x 128 tiles on single CTAs with
 // eight epilogue warps (18) while there are few tiles (an epilogue half as long at the end: FC1 4 304 x 1 152 at 512 rows
-// 10.0 us with v3, 7.4 with v18; FC2 1 152 x 1 152 at 2 048 rows 10.2 with v1, 7.4); 256 x 128 pairs (19) where
-// 256 x 256 tiles leave most of the last round empty (FC2 1 152 x 4 304 at 3 700 rows 25.2 -> 20.7); eight epilogue warps
-// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 52.2 with v1, 39.1 with v17).
+// 9.9 us with v3, 7.3 with v18; FC2 1 152 x 1 152 at 2 048 rows 10.0 with v1, 7.3); 256 x 128 pairs (19) where
+// 256 x 256 tiles leave most of the last round empty (FC2 1 152 x 1 152 at 5 003 rows 14.8 with v1, 11.8); eight epilogue warps
+// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 52.0 with v1, 38.6 with v17).
 enum CostClass : int { COST_GELU, COST_TANH, COST_NONE, COST_FC2, COST_PE };
 struct VariantCost {
     CostClass cls;
@@ -79,23 +79,7 @@ struct VariantCost {
     float start, first, next, tile;
 };
 const VariantCost kVariantCost[] = {
-    {COST_GELU, 18, 4.48f, 0.225f, 0.331f, 2.69f},
-    {COST_GELU, 15, 7.02f, 0.361f, 0.438f, 3.67f},
-    {COST_GELU, 14, 6.46f, 0.404f, 0.444f, 3.69f},
-    {COST_TANH, 18, 4.67f, 0.192f, 0.331f, 2.27f},
-    {COST_TANH, 3, 6.75f, 0.300f, 0.450f, 3.64f},
-    {COST_TANH, 15, 5.68f, 0.412f, 0.450f, 3.31f},
-    {COST_NONE, 18, 4.07f, 0.200f, 0.378f, 1.26f},
-    {COST_NONE, 3, 5.25f, 0.283f, 0.474f, 2.57f},
-    {COST_NONE, 2, 5.74f, 0.279f, 0.423f, 2.75f},
-    {COST_NONE, 1, 5.94f, 0.274f, 0.416f, 4.22f},
-    {COST_FC2, 18, 4.55f, 0.221f, 0.363f, 2.00f},
-    {COST_FC2, 19, 4.86f, 0.210f, 0.276f, 3.12f},
-    {COST_FC2, 3, 6.18f, 0.312f, 0.426f, 6.32f},
-    {COST_FC2, 17, 6.42f, 0.308f, 0.456f, 3.87f},
-    {COST_FC2, 1, 6.38f, 0.338f, 0.390f, 5.57f},
-    {COST_PE, 18, 4.92f, 0.177f, 0.383f, 2.22f},
-    {COST_PE, 17, 6.74f, 0.257f, 0.574f, 2.88f},
+#include "sl8_cost_model.h"
 };
 
 // CTAs, or pairs of them, that a launch on this handle's GPU can spread over (a B200's 148 SMs without a handle).

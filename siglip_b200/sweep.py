@@ -267,6 +267,161 @@ def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out
     return rows
 
 
+# ----------------------------------------------------------------------------- the cost model of pick_variant
+# (class, N, K): the widths of the two encoders and two of no model's, per kind of epilogue the model knows.
+MODEL_SHAPES = {
+    "GELU": [(4304, 1152), (3072, 768), (1600, 512), (4800, 1600)],
+    "TANH": [(4304, 1152), (3072, 768)],
+    "NONE": [(3456, 1152), (2304, 768), (4800, 1600), (1536, 512)],
+    "FC2": [(1152, 4304), (768, 3072), (1152, 1152), (768, 768), (1600, 4800), (512, 1600)],
+    "PE": [(1152, 588), (768, 768)],
+}
+MODEL_ROWS = [50, 128, 196, 256, 392, 512, 729, 1000, 1458, 1568, 2048, 2916, 3700, 4374, 5003, 5832, 7000, 8748, 11664, 14580, 17496,
+              23328, 32000, 46656, 93312, 186624]
+MODEL_CSV = PKG / "sweeps" / "b200_model.csv"
+MODEL_HEADER = PKG / "csrc" / "sl8_cost_model.h"
+
+
+def shown_path(path: Path) -> str:
+    try:
+        return str(path.resolve().relative_to(PKG.parent))
+    except ValueError:
+        return str(path)
+
+
+def variant_tiles() -> dict:
+    """{variant: (CTAs per tile, tile N)} from the list they are compiled from."""
+    return {int(v): (int(cg), int(tn)) for v, cg, tn in re.findall(r"X\((\d+), (\d), (\d+),", (PKG / "csrc" / "sl8_variants.h").read_text())}
+
+
+def cost_constants(path: Path = MODEL_HEADER) -> dict:
+    """{(class, variant): (start, first, next, tile)} as the committed header holds them."""
+    found = re.findall(r"\{COST_(\w+), (\d+), ([\d.]+)f, ([\d.]+)f, ([\d.]+)f, ([\d.]+)f\}", path.read_text())
+    return {(c, int(v)): tuple(map(float, k)) for c, v, *k in found}
+
+
+def emit_model(constants: dict, source: str, path: Path = MODEL_HEADER) -> None:
+    lines = ["// sl8_cost_model.h -- GENERATED by `python -m siglip_b200.sweep --fit-model " + source + "`: class of epilogue, variant, start, first, next, tile."]
+    for (cls, v), k in constants.items():
+        lines.append(f"    {{COST_{cls}, {v}, " + ", ".join(f"{x!r}f" for x in k) + "},")
+    path.write_text("\n".join(lines) + "\n")
+
+
+def model_us(k: tuple, cg: int, tn: int, M: int, N: int, K: int, sms: int = 148) -> float:
+    """The formula beside kVariantCost."""
+    tiles, k_blocks = -(-M // (128 * cg)) * -(-N // tn), -(-K // 128)
+    rounds = -(-tiles // (sms // cg))
+    return k[0] + k_blocks * k[1] + (rounds - 1) * max(k_blocks * k[2], k[3])
+
+
+def asked_rows(rows: list[dict]) -> list[dict]:
+    """The points of the sweep that the dispatch table leaves to the model (of a class that the table has whole: all of them)."""
+    table = {(r["op"], r["N"], r["K"]) for r in best_rows(read_csv(PKG / "sweeps" / "b200.csv"))}
+    ops = {"GELU": OPS["fc1"], "FC2": OPS["fc2"], "PE": OPS["pe"]}
+    asked = [r for r in rows if (ops.get(r["cls"]), int(r["N"]), int(r["K"])) not in table]
+    return asked + [r for r in rows if r["cls"] not in {a["cls"] for a in asked}]
+
+
+def model_regret(rows: list[dict], constants: dict, variants: dict) -> dict:
+    """{class: [(how much longer than the fastest variant the cheapest one by the formula took, the row)]}."""
+    out = {}
+    for r in rows:
+        m, n, k = int(r["M"]), int(r["N"]), int(r["K"])
+        times = {int(f[1:]): float(t) for f, t in r.items() if f[0] == "v" and t}
+        mine = [(model_us(c, *variants[v], m, n, k), v) for (cls, v), c in constants.items() if cls == r["cls"] and v in times]
+        out.setdefault(r["cls"], []).append((times[min(mine)[1]] / min(times.values()) - 1.0, r))
+    return out
+
+
+def fit_model(rows: list[dict], constants: dict, variants: dict, steps=(0.98, 1.02, 0.95, 1.05, 0.9, 1.1)) -> dict:
+    """`constants` with every number moved in small steps, one after the other and as long as it helps, to where the variant
+    picked is slower than the fastest by less: on average, plus a tenth of the worst case.  Its own result it leaves as it is."""
+    out = dict(constants)
+    for cls in sorted({c for c, _ in constants}):
+        mine = [v for c, v in constants if c == cls]
+        points = [(int(r["M"]), int(r["N"]), int(r["K"]), {int(f[1:]): float(t) for f, t in r.items() if f[0] == "v" and t}) for r in rows if r["cls"] == cls]
+        points = [(m, n, k, {v: t[v] / min(t.values()) - 1.0 for v in mine if v in t}) for m, n, k, t in points]
+        cost = {v: [model_us(out[cls, v], *variants[v], m, n, k) for m, n, k, _ in points] for v in mine}
+
+        def lost():
+            return [t[min((cost[v][i], v) for v in t)[1]] for i, (_, _, _, t) in enumerate(points)]
+
+        def score(now):
+            return statistics.fmean(now) + 0.1 * max(now)
+
+        best, moved = score(lost()), True
+        while moved:
+            moved = False
+            for v in mine:
+                for j in range(4):
+                    for f in steps:
+                        old, kept = out[cls, v], cost[v]
+                        out[cls, v] = old[:j] + (float(f"{old[j] * f:.3g}"),) + old[j + 1:]
+                        cost[v] = [model_us(out[cls, v], *variants[v], m, n, k) for m, n, k, _ in points]
+                        now = lost()
+                        if score(now) < best - 1e-5:
+                            best, moved = score(now), True
+                        else:
+                            out[cls, v], cost[v] = old, kept
+    return out
+
+
+def run_model_sweep(out_path: Path, repeats: int = 3, log=print) -> None:
+    """Graph-replay microseconds of every admissible variant over MODEL_SHAPES x MODEL_ROWS, two operand sets in turn."""
+    import torch
+    import siglip_b200
+    from siglip_b200 import build, layers, lib, synth
+
+    eng, stream = siglip_b200.Engine(0), torch.cuda.Stream()
+    resources = parse_resources(build.resource_report())
+    every = [dict(layers.describe_variant(v), variant_id=v) for v in range(layers.num_variants())]
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    normal = lambda *s: torch.randn(s, generator=gen, device="cuda").to(torch.bfloat16)
+    codes = lambda r, c: (torch.randint(0, 256, (r, synth.pitch128(c)), generator=gen, device="cuda", dtype=torch.uint8) & 0xBF)[:, :c]
+    s = torch.full((1,), 0.01, device="cuda")
+    with open(out_path, "w", newline="") as f:
+        w = csv.writer(f)
+        w.writerow(["cls", "N", "K", "M"] + [f"v{v['variant_id']}" for v in every])
+        for cls, shapes in MODEL_SHAPES.items():
+            op = OPS["pe"] if cls == "PE" else OPS["fc2"] if cls == "FC2" else OPS["fc1"]
+            for n, k in shapes:
+                B, bias, table = codes(n, k), normal(n), normal(729 + 128, n)
+                for m in MODEL_ROWS:
+                    if m > 46656 and (n, k) not in [(x[1], x[2]) for shape_set in SHAPE_SETS.values() for x in shape_set]:
+                        break
+                    A, D = [codes(m, k) for _ in range(2)], [torch.empty((m, n), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+                    res = [normal(m, n) for _ in range(2)] if cls == "FC2" else None
+                    turn = [0]
+
+                    def go():
+                        i = turn[0] = 1 - turn[0]
+                        kw = dict(scale_a=s, scale_b=s, out=D[i])
+                        if cls == "PE":
+                            eng.patch_embed(A[i], B, table, period=729, **kw)
+                        elif cls == "FC2":
+                            eng.fc2_residual(A[i], B, bias, res[i], **kw)
+                        elif cls == "NONE":
+                            eng.linear_bias(A[i], B, bias, **kw)
+                        else:
+                            eng.fc1_gelu(A[i], B, bias, flags=lib.SL8_FLAG_GELU_HW_TANH if cls == "TANH" else 0, **kw)
+
+                    iters, us = 12 if m <= 8748 else 6, {}
+                    for v in prune(every, op, resources):
+                        eng.set_variant(v["variant_id"])
+                        try:
+                            graph = capture(go, iters, stream)
+                            replay_ms(graph, iters)
+                            us[v["variant_id"]] = statistics.median(replay_ms(graph, iters) for _ in range(repeats)) * 1e3
+                        except lib.SL8Error:
+                            pass
+                    eng.set_variant(-1)
+                    eng.device_status()
+                    w.writerow([cls, n, k, m] + [f"{us[v['variant_id']]:.3f}" if v["variant_id"] in us else "" for v in every])
+                    f.flush()
+                    del A, D, res
+                log(f"{cls} {n} x {k}")
+
+
 def main(argv=None) -> int:
     ap = argparse.ArgumentParser(description=__doc__, formatter_class=argparse.RawDescriptionHelpFormatter)
     ap.add_argument("--shapes", default="so400m,b16", help="comma-separated shape sets: " + ", ".join(SHAPE_SETS))
@@ -279,14 +434,25 @@ def main(argv=None) -> int:
     ap.add_argument("--variants", default="", help="restrict to these variant ids")
     ap.add_argument("--emit-table", type=Path, default=None, metavar="CSV",
                     help="no GPU work: turn this CSV into csrc/sl8_dispatch_table.h")
+    ap.add_argument("--model-sweep", action="store_true", help="time the points of the cost model (25 s of B200 time) into " + MODEL_CSV.name)
+    ap.add_argument("--fit-model", type=Path, default=None, metavar="CSV",
+                    help="no GPU work: move the constants of csrc/sl8_cost_model.h to where they pick best on this CSV")
     a = ap.parse_args(argv)
+    if a.model_sweep:
+        run_model_sweep(MODEL_CSV)
+        return 0
+    if a.fit_model is not None:
+        variants, constants = variant_tiles(), cost_constants()
+        rows = asked_rows(read_csv(a.fit_model))
+        fitted = fit_model(rows, constants, variants)
+        emit_model(fitted, shown_path(a.fit_model))
+        for name, k in (("before", constants), ("after", fitted)):
+            for cls, lost in model_regret(rows, k, variants).items():
+                print(f"{name} {cls}: {100 * statistics.fmean(x for x, _ in lost):.2f} % off the fastest on average, {100 * max(x for x, _ in lost):.1f} % at worst")
+        return 0
     if a.emit_table is not None:
         table = best_rows(read_csv(a.emit_table))
-        try:
-            shown = a.emit_table.resolve().relative_to(PKG.parent)
-        except ValueError:
-            shown = a.emit_table
-        emit_header(table, str(shown))
+        emit_header(table, shown_path(a.emit_table))
         print(f"{len(table)} rows -> {TABLE_HEADER}")
         return 0
     only = {int(x) for x in a.variants.split(",")} if a.variants else None

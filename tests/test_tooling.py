@@ -75,6 +75,38 @@ def test_the_committed_table_is_what_its_sweep_produces():
     assert f"kSl8DispatchRows = {len(table)};" in header
 
 
+def test_the_committed_cost_model_is_what_its_sweep_produces(tmp_path):
+    """csrc/sl8_cost_model.h is fitted: the fit leaves it as it is, and it picks as well as the comment beside it says."""
+    points, constants, variants = sweep.read_csv(sweep.MODEL_CSV), sweep.cost_constants(), sweep.variant_tiles()
+    assert len({(r["cls"], r["N"], r["K"]) for r in points}) == sum(map(len, sweep.MODEL_SHAPES.values())) == 18
+    rows = sweep.asked_rows(points)
+    assert 300 < len(rows) < len(points)
+    assert sweep.fit_model(rows, constants, variants) == constants
+    sweep.emit_model(constants, "siglip_b200/sweeps/b200_model.csv", tmp_path / "m.h")
+    assert (tmp_path / "m.h").read_text() == sweep.MODEL_HEADER.read_text()
+    lost = {cls: [x for x, _ in points] for cls, points in sweep.model_regret(rows, constants, variants).items()}
+    assert max(map(max, lost.values())) < 0.0935 and all(0.0005 < sum(x) / len(x) < 0.0115 for x in lost.values())
+
+
+def test_the_cost_formula_is_the_one_the_library_uses(tmp_path):
+    """The fit's restatement of the formula and the library's pick the same variant, at every point of the sweep that the dispatch
+    table leaves to them."""
+    import ctypes as C
+    from siglip_b200 import build, lib as L
+    build.build()
+    library, cfg = L.load_library(), L.Config()
+    constants, variants = sweep.cost_constants(), sweep.variant_tiles()
+    kinds = {"GELU": (1, 0), "TANH": (1, L.SL8_FLAG_GELU_HW_TANH), "NONE": (1, L.SL8_FLAG_NO_ACTIVATION), "FC2": (2, 0), "PE": (0, 0)}
+    for r in sweep.asked_rows(sweep.read_csv(sweep.MODEL_CSV)):
+        if r["cls"] == "PE":              # (both widths are the table's)
+            continue
+        m, n, k = int(r["M"]), int(r["N"]), int(r["K"])
+        op, flags = kinds[r["cls"]]
+        cost = {v: sweep.model_us(c, *variants[v], m, n, k) for (cls, v), c in constants.items() if cls == r["cls"]}
+        assert library.sl8_query_config_flags(None, op, L.SL8_OUT_BF16, flags, m, n, k, C.byref(cfg)) == 0
+        assert cost[cfg.variant_id] <= min(cost.values()) * (1 + 1e-6), r       # (single precision there)
+
+
 def test_anova_known_answer():
     # Textbook example: three groups, F = 9.3 exactly? computed by hand below.
     g = [[6.0, 8.0, 4.0, 5.0, 3.0, 4.0], [8.0, 12.0, 9.0, 11.0, 6.0, 8.0], [13.0, 9.0, 11.0, 8.0, 7.0, 12.0]]
