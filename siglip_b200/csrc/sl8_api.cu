@@ -66,12 +66,14 @@ int kernel_slot(int op, int out_dtype) {
 // `start` is set-up, the first operands' way in and the last tile's epilogue; `first` a k-block of the first tile; a later tile
 // hides its mainloop (`next` per k-block, more than `first` when every SM asks L2) behind the epilogue ahead of it or the
 // other way round (`tile`: the epilogue's own pace).  The constants (sl8_cost_model.h) are fitted so that the cheapest variant by
-// the formula is the fastest one measured, from 512 to 4 800 wide and 50 to 186 624 rows: on that sweep (346 points that the table
-// leaves to it, sweeps/b200_model.csv) it is 0.1 - 1.1 % off the fastest on average, by class, and 9.3 % at worst.  What it decides: 128 x 128 tiles on single CTAs with
+// the formula is the fastest one measured, from 512 to 4 800 wide and 50 to 186 624 rows: on that sweep (488 points that the table
+// leaves to it, sweeps/b200_model.csv) it is 0.1 - 2.2 % off the fastest on average, by class, and 15 % at worst (GELU, 32 000 x
+// 1 152 x 4 304).  What it decides: 128 x 128 tiles on single CTAs with
 // eight epilogue warps (18) while there are few tiles (an epilogue half as long at the end: FC1 4 304 x 1 152 at 512 rows
 // 9.9 us with v3, 7.3 with v18; FC2 1 152 x 1 152 at 2 048 rows 10.0 with v1, 7.3); 256 x 128 pairs (19) where
 // 256 x 256 tiles leave most of the last round empty (FC2 1 152 x 1 152 at 5 003 rows 14.8 with v1, 11.8); eight epilogue warps
-// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 52.0 with v1, 38.6 with v17).
+// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 52.0 with v1,
+// 38.6 with v17); a fifth stage (2) where K is deep behind a light epilogue (hardware tanh, 1 152 x 4 304 at 46 656 rows 197.7 with v3, 180.8).
 enum CostClass : int { COST_GELU, COST_TANH, COST_NONE, COST_FC2, COST_PE };
 struct VariantCost {
     CostClass cls;

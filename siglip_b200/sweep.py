@@ -270,9 +270,9 @@ def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out
 # ----------------------------------------------------------------------------- the cost model of pick_variant
 # (class, N, K): the widths of the two encoders and two of no model's, per kind of epilogue the model knows.
 MODEL_SHAPES = {
-    "GELU": [(4304, 1152), (3072, 768), (1600, 512), (4800, 1600)],
-    "TANH": [(4304, 1152), (3072, 768)],
-    "NONE": [(3456, 1152), (2304, 768), (4800, 1600), (1536, 512)],
+    "GELU": [(4304, 1152), (3072, 768), (1600, 512), (4800, 1600), (1152, 4304), (1600, 4800)],
+    "TANH": [(4304, 1152), (3072, 768), (1152, 4304), (1600, 4800)],
+    "NONE": [(3456, 1152), (2304, 768), (4800, 1600), (1536, 512), (1152, 4304), (1600, 4800)],
     "FC2": [(1152, 4304), (768, 3072), (1152, 1152), (768, 768), (1600, 4800), (512, 1600)],
     "PE": [(1152, 588), (768, 768)],
 }
@@ -387,7 +387,7 @@ def run_model_sweep(out_path: Path, repeats: int = 3, log=print) -> None:
             for n, k in shapes:
                 B, bias, table = codes(n, k), normal(n), normal(729 + 128, n)
                 for m in MODEL_ROWS:
-                    if m > 46656 and (n, k) not in [(x[1], x[2]) for shape_set in SHAPE_SETS.values() for x in shape_set]:
+                    if m > 46656 and (op, n, k) not in [(OPS[x[0]], x[1], x[2]) for shape_set in SHAPE_SETS.values() for x in shape_set]:
                         break
                     A, D = [codes(m, k) for _ in range(2)], [torch.empty((m, n), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
                     res = [normal(m, n) for _ in range(2)] if cls == "FC2" else None

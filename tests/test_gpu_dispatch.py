@@ -13,8 +13,8 @@ GENERAL = 6       # 128 x 128 tiles on single CTAs: serves every layer and outpu
 # (kind of call, the variant its cost picks, shapes): every row of the cost model, at row counts and widths that end in the
 # middle of a tile and K that ends in the middle of a block.
 CASES = [("gelu", 18, (1, 16, 16), (769, 400, 592)), ("gelu", 14, (9473, 144, 80), (5121, 1296, 592)), ("gelu", 15, (9473, 144, 2128)),
-         ("tanh", 18, (127, 144, 80)), ("tanh", 3, (9473, 144, 1616)), ("tanh", 15, (9473, 144, 80)),
-         ("none", 18, (129, 400, 592)), ("none", 3, (9473, 144, 592)), ("none", 2, (9473, 1040, 1104)), ("none", 1, (9473, 528, 3152)),
+         ("tanh", 18, (127, 144, 80)), ("tanh", 3, (9473, 144, 1616)), ("tanh", 15, (9473, 144, 80)), ("tanh", 2, (20001, 528, 2128)),
+         ("none", 18, (129, 400, 592)), ("none", 3, (9473, 144, 592)), ("none", 2, (9473, 1040, 1104)), ("none", 1, (20001, 272, 4176)),
          ("fc2", 18, (1, 16, 16), (2369, 528, 592)), ("fc2", 19, (20001, 16, 1616)), ("fc2", 3, (9473, 144, 80)), ("fc2", 17, (9473, 656, 80)),
          ("fc2", 1, (16001, 656, 1616)), ("pe", 18, (127, 144, 80)), ("pe", 17, (9473, 144, 80))]
 

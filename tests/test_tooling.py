@@ -78,14 +78,14 @@ def test_the_committed_table_is_what_its_sweep_produces():
 def test_the_committed_cost_model_is_what_its_sweep_produces(tmp_path):
     """csrc/sl8_cost_model.h is fitted: the fit leaves it as it is, and it picks as well as the comment beside it says."""
     points, constants, variants = sweep.read_csv(sweep.MODEL_CSV), sweep.cost_constants(), sweep.variant_tiles()
-    assert len({(r["cls"], r["N"], r["K"]) for r in points}) == sum(map(len, sweep.MODEL_SHAPES.values())) == 18
+    assert len({(r["cls"], r["N"], r["K"]) for r in points}) == sum(map(len, sweep.MODEL_SHAPES.values())) == 24
     rows = sweep.asked_rows(points)
     assert 300 < len(rows) < len(points)
     assert sweep.fit_model(rows, constants, variants) == constants
     sweep.emit_model(constants, "siglip_b200/sweeps/b200_model.csv", tmp_path / "m.h")
     assert (tmp_path / "m.h").read_text() == sweep.MODEL_HEADER.read_text()
     lost = {cls: [x for x, _ in points] for cls, points in sweep.model_regret(rows, constants, variants).items()}
-    assert max(map(max, lost.values())) < 0.0935 and all(0.0005 < sum(x) / len(x) < 0.0115 for x in lost.values())
+    assert max(map(max, lost.values())) < 0.1495 and all(0.0005 < sum(x) / len(x) < 0.0225 for x in lost.values())
 
 
 def test_the_cost_formula_is_the_one_the_library_uses(tmp_path):
