@@ -241,7 +241,8 @@ def test_layernorm_quantize_feeds_fc1(engine, oracle):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,cols", [(40, 8), (3, 768), (7200, 768), (7200, 776), (3, 1280), (50, 1288), (1300, 1792), (50, 1800),
-                                       (1300, 2048), (50, 2056)])     # edges of the widths kept in registers; more rows than warps x ring
+                                       (1300, 2048), (50, 2056),
+                                       (10923, 1152), (16300, 776)])     # edges of the widths kept in registers; more rows than warps x ring
 def test_layernorm_widths_on_gpu(engine, oracle, dtype, rows, cols):
     rng = np.random.default_rng(rows + cols)
     x = torch.from_numpy((rng.standard_normal((rows, cols + 8)) * 2 + 0.5).astype(np.float32)).to(dtype).to(DEV)[:, :cols]     # pitch != width
