@@ -708,7 +708,8 @@ __global__ void __launch_bounds__(kLnThreads) layernorm_quantize_plain_kernel(co
     }
 }
 
-// Wider rows: a warp per row, three passes over it (the second and third hit L1 / L2).
+// Wider rows: a warp per row, three passes over it (the second and third hit L1 / L2).  Twice the blocks that are resident: their
+// rows end at different times (20 000 bf16 rows of 2 304 / 4 304 / 8 192: 45.4 / 89.8 / 169.6 -> 41.9 / 85.4 / 158.2 us).
 template <typename T>
 __global__ void __launch_bounds__(kLnThreads) layernorm_quantize_wide_kernel(const T* x, long long rows, int cols, long long ld, const float* gamma,
                                                                              const float* beta, float eps, const float* scale, uint8_t* out, long long ld_out) {
@@ -761,7 +762,7 @@ cudaError_t launch_layernorm(int sm_count, cudaStream_t s, const T* x, long long
     if (cols <= 1280) return launch(layernorm_quantize_kernel<T, 5>, LnShape<T, 5>::PER_SM);
     if (cols <= 1792) return launch(layernorm_quantize_kernel<T, 7>, LnShape<T, 7>::PER_SM);
     if (cols <= 2048) return launch(layernorm_quantize_kernel<T, 8>, LnShape<T, 8>::PER_SM);
-    return launch(layernorm_quantize_wide_kernel<T>, 16);
+    return launch(layernorm_quantize_wide_kernel<T>, 32);
 }
 
 }  // namespace
