@@ -223,6 +223,8 @@ class Engine:
         period, N = pos.shape
         self._on_device("pos", pos)
         self._readable("bias", bias)
+        if bias is not None and bias.numel() < N:
+            raise ValueError(f"bias must have {N} elements")
         # (converted on the stream that reads them)
         with contextlib.nullcontext() if stream is None else torch.cuda.stream(torch.cuda.ExternalStream(self._stream(stream), device=self.device)):
             pos = pos.contiguous().float()

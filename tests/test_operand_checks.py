@@ -141,6 +141,7 @@ BIAS_REFUSED = {f"{f}_{what}": (lambda e, f=f, b=b, kw=kw: gemm(e, f, bias=b(), 
     "mlp_bias1_fp16": lambda e: gemm(e, "mlp", bias1=cuda(64, dtype=F16)),
     "mlp_types_differ": lambda e: gemm(e, "mlp", bias1=cuda(64, dtype=F32), bias2=cuda(32, dtype=BF16)),
     "mlp_types_differ_too": lambda e: gemm(e, "mlp", bias1=cuda(64, dtype=BF16), bias2=cuda(32, dtype=F32)),
+    "table_short": lambda e: e.make_table(cuda(31, dtype=F32), cuda(100, 32, dtype=F32), **S),
     "mlp_bias1_short": lambda e: gemm(e, "mlp", bias1=cuda(32, dtype=BF16)),
     "mlp_bias2_short": lambda e: gemm(e, "mlp", bias2=cuda(31, dtype=BF16)),
 }
