@@ -5,6 +5,8 @@
 // counterpart of the reference's persistent_gemm<EpilogueOp> (kernel_body.cuh:448-815) and
 // epilogue_store (kernel_body.cuh:47-442), rebuilt around run-time M/N/K:
 //
+//   Every role walks its loop as a whole warp and issues through an elected lane (see the MMA role).
+//
 //   warp 0        TMA producer of A: streams A[128 x 128B] k-blocks into a ring of STAGES
 //                 shared-memory stages (SWIZZLE_128B), one mbarrier pair (full / empty) per stage,
 //                 and announces the stage's bytes.
@@ -181,12 +183,22 @@ struct WaitCtx {
 
 // Polls `bar` until the phase with parity `parity` has completed.  Returns false if the CTA
 // is aborting or the budget ran out (in which case it records `code` and raises the flag).
-// SPIN: poll without parking the thread (the two single-thread roles on the critical path, whose wake-up
-// latency is paid by the whole CTA pair); otherwise each poll may park the thread until the phase completes.
+// All lanes of a warp call it together: a branch for one lane, its reconvergence and a second poll by the others cost 700 -
+// 1 000 cycles where the barrier had long completed (embed of one image, from the last MMA to the first tcgen05.ld 2 000
+// cycles, 400 as it stands; a block of 729 rows 46.9 -> 45.7 us).
+// SPIN: poll without parking the warp (the roles on the critical path, whose wake-up latency is paid by the whole CTA
+// pair); otherwise kPolls polls, and from then on each may park the warp until the phase completes (a parking poll costs
+// several hundred cycles even on a barrier that is complete).
+constexpr uint32_t kPolls = 64;
 template <bool SPIN = false>
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, const WaitCtx& w, uint32_t code,
                                          uint32_t which) {
-    if (SPIN ? (mbar_test_wait(bar, parity) != 0u) : mbar_try_wait(bar, parity)) return true;
+    if (mbar_test_wait(bar, parity) != 0u) return true;
+    if constexpr (!SPIN) {
+#pragma unroll 1
+        for (uint32_t i = 0; i < kPolls; ++i)
+            if (mbar_test_wait(bar, parity) != 0u) return true;
+    }
     unsigned long long t0 = 0;
     for (uint32_t spins = 1;; ++spins) {
         if (SPIN ? (mbar_test_wait(bar, parity) != 0u) : mbar_try_wait(bar, parity)) return true;
@@ -508,53 +520,60 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
-    // Everything above (barriers, tensor memory, descriptors) runs beside the tail of the kernel ahead on the stream.  No
+    // Everything above (barriers, tensor memory, descriptors) runs beside the tail of the kernel ahead on the stream, and so
+    // does what each role can do without global memory: it calls pdl_wait() directly in front of its first access.  No
     // two GEMM CTAs share an SM (each takes more than half its shared memory), so the next GEMM's CTAs move in as these leave.
-    pdl_wait();
-    pdl_release();
 
     // ---------------------------------------------------------------- roles
     if (warp == 0 || warp == 3 + EPI_WARPS) {
         // ===== TMA producers: warp 0 brings A, the last warp brings B =====
+        // Whole warps with an elected lane, like the MMA role: from a branch that only lane 0 takes, a k-block took 450 - 500
+        // cycles to issue, more than the MMAs of a 128-column tile need (FC2 1152 x 4304 at 729 rows: 437 -> 373 cycles per k-block).
         // Both wait for the stage to be free and then issue their own copies.  Only the A producer arrives on
         // the stage's full barrier (in a CTA pair: only the leader's), announcing the bytes of everything that
         // will land on it; the other copies just count down.  The transaction count may run negative until
         // that arrive lands, and the phase cannot complete before it.  A B copy can never be a whole phase
         // ahead of the arrive it belongs to: the stage is only handed back (empty barrier) after the MMAs have
         // read it, i.e. after the previous phase of the full barrier completed, arrive included.
-        if (lane == 0) {
-            const bool is_a = (warp == 0);
-            int stage = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            const bool prof_total = p.prof != nullptr && is_a;
-            const bool prof = prof_total && !(p.flags & (FLAG_COARSE_TRACE | DBG_COARSE_TRACE));
-            const uint32_t full_bar_leader = (CG == 2) ? map_to_cta(full_bar0, 0) : full_bar0;
-            long long t_wait = 0;
-            const long long t_begin = clock64();
-            for (int tile = cluster_id; ok && tile < p.num_tiles; tile += num_clusters) {
-                wc.tile = tile;
-                const int tm = tile / p.tiles_n;
-                const int tn = tile - tm * p.tiles_n;
-                const int m0 = tm * (T::TILE_M_CTA * CG) + static_cast<int>(cta_rank) * T::TILE_M_CTA;
-                // The last N tile may be narrower: each CTA of a pair then holds tail_cols / CG rows of B,
-                // brought by a tensor map whose box is that tall (map_bt), and the MMAs are issued with N = tail_cols.
-                const bool tail = (tn == p.tiles_n - 1) && (p.tail_cols != TN);
-                const int b_rows = tail ? p.tail_cols / CG : T::B_ROWS;
-                const int nb = tn * TN + static_cast<int>(cta_rank) * b_rows;
-                // (measurement builds: DBG_SKIP_A / DBG_SKIP_B leave one operand's copies out; the MMAs then read stale shared memory)
-                const uint32_t stage_tx = static_cast<uint32_t>((SL8_DBG(p.flags, DBG_SKIP_A) ? 0 : T::A_BYTES) +
-                                                                (SL8_DBG(p.flags, DBG_SKIP_B) ? 0 : T::KATOMS * b_rows * 128));
-                const bool skip_mine = is_a ? SL8_DBG(p.flags, DBG_SKIP_A) : SL8_DBG(p.flags, DBG_SKIP_B);
-                const CUtensorMap* const bmap = tail ? &map_bt : &map_b;
-                const int drop_kb = (!is_a && (p.flags & FLAG_TEST_DROP_B) && tile == cluster_id) ? 1 : -1;   // evaluated once per tile
-                for (int kb = 0; kb < p.k_blocks; kb++) {
-                    const long long t0 = prof ? clock64() : 0;
-                    ok = wait_bar<SL8_SPIN_CRITICAL>(empty_bar0 + 8 * stage, phase ^ 1u, wc, ST_PRODUCER_EMPTY_WAIT, stage);
-                    if (prof) t_wait += clock64() - t0;
-                    if (!ok) break;
-                    const uint32_t a_dst = base + stage * T::STAGE_BYTES;
-                    const uint32_t b_dst = a_dst + T::A_BYTES;
+        const bool is_a = (warp == 0);
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        const bool prof_total = p.prof != nullptr && is_a;
+        const bool prof = prof_total && !(p.flags & (FLAG_COARSE_TRACE | DBG_COARSE_TRACE));
+        const uint32_t full_bar_leader = (CG == 2) ? map_to_cta(full_bar0, 0) : full_bar0;
+        long long t_wait = 0, t_begin = 0;
+        bool waited = false;
+        for (int tile = cluster_id; ok && tile < p.num_tiles; tile += num_clusters) {
+            wc.tile = tile;
+            const int tm = tile / p.tiles_n;
+            const int tn = tile - tm * p.tiles_n;
+            const int m0 = tm * (T::TILE_M_CTA * CG) + static_cast<int>(cta_rank) * T::TILE_M_CTA;
+            // The last N tile may be narrower: each CTA of a pair then holds tail_cols / CG rows of B,
+            // brought by a tensor map whose box is that tall (map_bt), and the MMAs are issued with N = tail_cols.
+            const bool tail = (tn == p.tiles_n - 1) && (p.tail_cols != TN);
+            const int b_rows = tail ? p.tail_cols / CG : T::B_ROWS;
+            const int nb = tn * TN + static_cast<int>(cta_rank) * b_rows;
+            // (measurement builds: DBG_SKIP_A / DBG_SKIP_B leave one operand's copies out; the MMAs then read stale shared memory)
+            const uint32_t stage_tx = static_cast<uint32_t>((SL8_DBG(p.flags, DBG_SKIP_A) ? 0 : T::A_BYTES) +
+                                                            (SL8_DBG(p.flags, DBG_SKIP_B) ? 0 : T::KATOMS * b_rows * 128));
+            const bool skip_mine = is_a ? SL8_DBG(p.flags, DBG_SKIP_A) : SL8_DBG(p.flags, DBG_SKIP_B);
+            const CUtensorMap* const bmap = tail ? &map_bt : &map_b;
+            const int drop_kb = (!is_a && (p.flags & FLAG_TEST_DROP_B) && tile == cluster_id) ? 1 : -1;   // evaluated once per tile
+            for (int kb = 0; kb < p.k_blocks; kb++) {
+                const long long t0 = prof ? clock64() : 0;
+                ok = __all_sync(0xffffffffu, wait_bar<SL8_SPIN_CRITICAL>(empty_bar0 + 8 * stage, phase ^ 1u, wc, ST_PRODUCER_EMPTY_WAIT, stage)) != 0;
+                if (prof) t_wait += clock64() - t0;
+                if (!ok) break;
+                const uint32_t a_dst = base + stage * T::STAGE_BYTES;
+                const uint32_t b_dst = a_dst + T::A_BYTES;
+                if (!waited) {
+                    pdl_wait();
+                    pdl_release();
+                    waited = true;
+                    t_begin = clock64();
+                }
+                if (elect_one()) {
                     if (SL8_DBG(p.flags, DBG_SKIP_LOAD)) {   // measurement aid: MMAs run on whatever shared memory holds
                         if (cta_rank == 0 && is_a) mbar_arrive(full_bar0 + 8 * stage);
                     } else if constexpr (CG == 2) {
@@ -584,14 +603,15 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                                 tma_load_2d(b_dst + a * T::B_ATOM_BYTES, bmap, kb * T::TILE_K + 128 * a, nb, bar);
                         }
                     }
-                    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                 }
+                __syncwarp();
+                if (++stage == STAGES) { stage = 0; phase ^= 1u; }
             }
-            if (prof_total) {
-                long long* slot = p.prof + static_cast<size_t>(blockIdx.x) * PROF_SLOTS;
-                slot[PROF_PRODUCER_WAIT] = t_wait;
-                slot[PROF_PRODUCER_TOTAL] = clock64() - t_begin;
-            }
+        }
+        if (prof_total && lane == 0) {
+            long long* slot = p.prof + static_cast<size_t>(blockIdx.x) * PROF_SLOTS;
+            slot[PROF_PRODUCER_WAIT] = t_wait;
+            slot[PROF_PRODUCER_TOTAL] = clock64() - t_begin;
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -621,6 +641,8 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const bool prof_any = p.prof != nullptr;
             const bool prof = prof_any && !(p.flags & (FLAG_COARSE_TRACE | DBG_COARSE_TRACE));
             long long t_full = 0, t_tmem = 0, n_tiles = 0, t_mma = 0, t_commit = 0;
+            pdl_wait();              // nothing to wait for before that: the bounded waits start with the kernel's own work
+            pdl_release();
             const long long t_begin = clock64();
             uint32_t ready = 0;      // look-ahead: the barrier of `stage` was already seen complete
 
@@ -765,8 +787,6 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         static_assert(!HAS_SIDE || NBUF >= 2, "side data needs a buffer to land in while another is stored");
 
         EpiCtx e;
-        e.scale = (p.scale_a ? ld_f32(p.scale_a) : 1.0f) * (p.scale_b ? ld_f32(p.scale_b) : 1.0f);
-        e.inv_out = __frcp_rn(p.out_scale ? ld_f32(p.out_scale) : 1.0f);   // IEEE 1/x, as the CPU oracle computes it
         e.flags = p.flags;
         e.swz = (T::REGION_ROW_BYTES == 128) ? (lane & 7) : ((lane >> 1) & 3);
         e.row_off = lane * T::REGION_ROW_BYTES;
@@ -784,6 +804,18 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         float bnext[NB], bcur[NB];
 #pragma unroll
         for (int i = 0; i < NB; i++) bcur[i] = bnext[i] = 0.0f;
+        bool ok = true;
+        uint32_t seq = 0;                          // regions processed so far by this warp
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        const bool prof_total = p.prof != nullptr && ew == 0;
+        const bool prof = prof_total && !(p.flags & (FLAG_COARSE_TRACE | DBG_COARSE_TRACE));   // inner timers cost ~35 cycles each
+        long long t_acc = 0, t_store = 0, t_ld = 0, t_math = 0, t_issue = 0, t_refill = 0;
+        pdl_wait();
+        pdl_release();
+        const long long t_begin = clock64();
+        e.scale = (p.scale_a ? ld_f32(p.scale_a) : 1.0f) * (p.scale_b ? ld_f32(p.scale_b) : 1.0f);
+        e.inv_out = __frcp_rn(p.out_scale ? ld_f32(p.out_scale) : 1.0f);   // IEEE 1/x, as the CPU oracle computes it
         if constexpr (HAS_BIAS) {
             if (cluster_id < p.num_tiles) {
                 const int tn0 = cluster_id % p.tiles_n;
@@ -796,14 +828,6 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 __syncwarp();
             }
         }
-        bool ok = true;
-        uint32_t seq = 0;                          // regions processed so far by this warp
-        int acc = 0;
-        uint32_t acc_phase = 0;
-        const bool prof_total = p.prof != nullptr && ew == 0;
-        const bool prof = prof_total && !(p.flags & (FLAG_COARSE_TRACE | DBG_COARSE_TRACE));   // inner timers cost ~35 cycles each
-        long long t_acc = 0, t_store = 0, t_ld = 0, t_math = 0, t_issue = 0, t_refill = 0;
-        const long long t_begin = clock64();
         for (int tile = cluster_id; ok && tile < p.num_tiles; tile += num_clusters) {
             wc.tile = tile;
             const int tm = tile / p.tiles_n;
@@ -818,11 +842,8 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 if (has_next) load_bias<NB>(bnext, p.bias, p.flags, (next_tile % p.tiles_n) * TN + col_begin, lane, p.N);
             }
 
-            // One lane polls; the others then confirm with a single try_wait of their own.
             long long t0 = prof_total ? clock64() : 0;       // once per tile: timed in the coarse mode too
-            if (lane == 0) ok = wait_bar(tfull_bar0 + 8 * acc, acc_phase, wc, ST_EPI_TMEM_FULL_WAIT, acc);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (ok && lane != 0) ok = wait_bar(tfull_bar0 + 8 * acc, acc_phase, wc, ST_EPI_TMEM_FULL_WAIT, acc);
+            ok = wait_bar(tfull_bar0 + 8 * acc, acc_phase, wc, ST_EPI_TMEM_FULL_WAIT, acc);
             ok = __all_sync(0xffffffffu, ok);
             if (prof_total) t_acc += clock64() - t0;
             if (!ok) break;
@@ -842,13 +863,11 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     // this region's side values have landed: one lane polls, the others confirm
                     const uint32_t sbar = my_side_bar + 8 * (seq % NBUF);
                     const uint32_t spar = (seq / NBUF) & 1u;
-                    if (lane == 0) ok = wait_bar(sbar, spar, wc, ST_EPI_SIDE_WAIT, seq % NBUF);
-                    ok = __shfl_sync(0xffffffffu, ok, 0);
-                    if (ok && lane != 0) ok = wait_bar(sbar, spar, wc, ST_EPI_SIDE_WAIT, seq % NBUF);
+                    ok = wait_bar(sbar, spar, wc, ST_EPI_SIDE_WAIT, seq % NBUF);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                 } else {
-                    if (lane == 0) tma_store_wait_read<NBUF - 1>();   // the buffer is no longer read by an older store
+                    if (elect_one()) tma_store_wait_read<NBUF - 1>();   // the buffer is no longer read by an older store
                     __syncwarp();
                 }
                 if (prof) t_store += clock64() - t0;
@@ -873,7 +892,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                                 // Last read of this accumulator: hand the TMEM buffer back before the math.
                                 tc_fence_before();
                                 __syncwarp();
-                                if (lane == 0) {
+                                if (elect_one()) {
                                     if constexpr (CG == 2) mbar_arrive_cluster(map_to_cta(tempty_bar0 + 8 * acc, 0));
                                     else mbar_arrive(tempty_bar0 + 8 * acc);
                                 }
@@ -904,16 +923,16 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     if (!SL8_DBG(p.flags, DBG_SKIP_STORE)) {
                         fence_proxy_async_smem();
                         __syncwarp();
-                        if (lane == 0 && warp_rows_ok) tma_store_2d(&map_d, region, col0, static_cast<int>(m_warp));
+                        if (warp_rows_ok && elect_one()) tma_store_2d(&map_d, region, col0, static_cast<int>(m_warp));
                     }
                     if (prof) t_issue += clock64() - t0;
                 }
-                if (lane == 0) tma_store_commit();       // one bulk group per region, possibly empty
+                if (elect_one()) tma_store_commit();       // one bulk group per region, possibly empty
                 if constexpr (HAS_SIDE) {
                     // Once the PREVIOUS region's store has read its buffer, hand that buffer back to the
                     // side-data loader (this region's store may still be reading its own).
                     if (prof) t0 = clock64();
-                    if (lane == 0) {
+                    if (elect_one()) {
                         tma_store_wait_read<1>();
                         if (seq > 0) mbar_arrive(my_side_free + 8 * ((seq - 1) % NBUF));
                     }
@@ -925,7 +944,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             if (!released) {                             // tile whose last region lies past N
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) {
+                if (elect_one()) {
                     if constexpr (CG == 2) mbar_arrive_cluster(map_to_cta(tempty_bar0 + 8 * acc, 0));
                     else mbar_arrive(tempty_bar0 + 8 * acc);
                 }
@@ -947,7 +966,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         }
         // The staging buffers must have been read before this CTA's shared memory is given back; the writes themselves
         // are complete for whoever is ordered after the kernel, as every write of a kernel is.
-        if (lane == 0) tma_store_wait_read<0>();
+        if (elect_one()) tma_store_wait_read<0>();
         __syncwarp();
         if (prof_total && lane == 0) {
             long long* slot = p.prof + static_cast<size_t>(blockIdx.x) * PROF_SLOTS;
@@ -975,7 +994,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             int my_tiles = 0;
             if (cluster_id < p.num_tiles) my_tiles = (p.num_tiles - cluster_id + num_clusters - 1) / num_clusters;
             const uint32_t total = static_cast<uint32_t>(my_tiles) * RPT;
-            bool ok = true;
+            bool ok = true, waited = false;
             for (uint32_t s = 0; ok && s < total; s++) {
                 const int tile = cluster_id + static_cast<int>(s / RPT) * num_clusters;
                 const int tm = tile / p.tiles_n;
@@ -989,12 +1008,12 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     const uint32_t freed = side_free0 + 8 * (g * NBUF + bsel);
                     const uint32_t buf = staging_base + (g * NBUF + bsel) * BOX_BYTES;
                     // the box's previous occupant (region s - NBUF) has been stored by all four warps
-                    if (lane == 0) ok = wait_bar(freed, ((s / NBUF) & 1u) ^ 1u, wc, ST_SIDE_LOADER_WAIT, g);
-                    ok = __shfl_sync(0xffffffffu, ok, 0);
+                    ok = __all_sync(0xffffffffu, wait_bar(freed, ((s / NBUF) & 1u) ^ 1u, wc, ST_SIDE_LOADER_WAIT, g)) != 0;
                     if (!ok) break;
                     const int col0 = tn * TN + g * T::COLS_PER_WARP + static_cast<int>(s % RPT) * T::REGION_COLS;
                     if (col0 >= p.N || skip_side) {
-                        if (lane == 0) mbar_arrive(landed);
+                        if (elect_one()) mbar_arrive(landed);
+                        __syncwarp();
                         continue;
                     }
                     int y = static_cast<int>(m_cta);
@@ -1003,11 +1022,17 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                         y = static_cast<int>((static_cast<uint32_t>(m_cta) + static_cast<uint32_t>(p.row_phase)) % static_cast<uint32_t>(p.period));
                         wraps = y + T::TILE_M_CTA > p.table_rows;   // only a table without periodic padding wraps
                     }
+                    if (!waited) {
+                        pdl_wait();
+                        pdl_release();
+                        waited = true;
+                    }
                     if (!wraps) {
-                        if (lane == 0) {
+                        if (elect_one()) {
                             mbar_arrive_expect_tx(landed, BOX_BYTES);
                             tma_load_2d(buf, &map_s, col0, y, landed);
                         }
+                        __syncwarp();
                     } else {
                         const int piece = lane & 7;                 // 16-byte piece (8 bf16 columns) of the 128-byte row
                         const int col = col0 + piece * 8;
@@ -1033,7 +1058,8 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                             }
                         }
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(landed);
+                        if (elect_one()) mbar_arrive(landed);
+                        __syncwarp();
                     }
                 }
             }
