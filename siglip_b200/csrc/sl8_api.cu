@@ -335,6 +335,7 @@ int run(sl8_handle_t h, const Problem& q, cudaStream_t stream) {
 
     const int grid = grid_for(h, v, slot, p.num_tiles);
     h->last_grid = grid;
+    sl8::set_tile_walk(p, grid / v->cg);
     if (h->d_prof && grid > h->prof_blocks) return fail(h, SL8_ERR_INVALID_VALUE, "tracing buffer smaller than the grid");
     cudaError_t e = v->launch[slot](&map_a, &map_b, &map_bt, &map_d, &map_s, &p, grid, stream);
     if (e != cudaSuccess) return fail_cuda(h, e, "kernel launch");

@@ -15,8 +15,7 @@
 //                 TMA unit has generated the requests of its previous one (2 cycles per 128-byte row:
 //                 64 bytes per clock per issuing thread, measured), while the unit itself serves two
 //                 threads at once at 128 bytes per clock: one thread cannot feed a 256 x 256 tile.
-//   warp 1        allocates tensor memory; one elected thread of the leader CTA's issues
-//                 tcgen05.mma kind::f8f6f4 (E4M3 x E4M3 -> FP32 in TMEM), four K=32 steps per
+//   warp 1        one elected thread of the leader CTA's issues tcgen05.mma kind::f8f6f4 (E4M3 x E4M3 -> FP32 in TMEM), four K=32 steps per
 //                 k-block (fewer in the K tail), and commits to the stage's empty barrier and,
 //                 after the last k-block, to the accumulator's full barrier.
 //   warps 2..     epilogue: tcgen05.ld of the finished accumulator (two accumulators in TMEM,
@@ -110,6 +109,8 @@ struct KernelParams {
     int K;
     int tiles_n;
     int num_tiles;
+    unsigned tiles_n_magic;          // ceil(2^32 / tiles_n), 0 for tiles_n == 1 (see TileWalk)
+    int step_m, step_n;              // what one round adds to a cluster's tile: clusters / tiles_n row-blocks, clusters % tiles_n columns
     int k_blocks;          // ceil(K / TILE_K)
     int last_kblock_mmas;  // K = 32 steps needed in the last k-block (1 .. TILE_K / 32)
     int tail_cols;         // columns of the last N tile: N - (tiles_n - 1) * TN, a multiple of 16 (== TN when N % TN == 0)
@@ -172,6 +173,29 @@ struct KernelTraits {
     // A launch that waits for the one ahead of it (pdl_wait) already holds tensor memory: it must not sit on that one's SMs.
     static_assert(2 * SMEM_BYTES > 228 * 1024, "two CTAs must not fit one SM");
 };
+
+// The tiles of one cluster: cluster, cluster + clusters, ... in N-fastest order.  No division: the first tile's number is
+// small enough for a multiplication (exact while cluster * tiles_n < 2^32; N is below 2^31 / 128 tiles), later ones are steps.
+struct TileWalk {
+    int tile, tm, tn;
+    __device__ __forceinline__ TileWalk(const KernelParams& p, int cluster)
+        : tile(cluster), tm(p.tiles_n_magic ? static_cast<int>(static_cast<uint64_t>(cluster) * p.tiles_n_magic >> 32) : cluster) {
+        tn = cluster - tm * p.tiles_n;
+    }
+    __device__ __forceinline__ void next(const KernelParams& p, int clusters) {
+        tile += clusters;
+        tm += p.step_m;
+        tn += p.step_n;
+        if (tn >= p.tiles_n) { tn -= p.tiles_n; tm++; }
+    }
+};
+
+// Host side of TileWalk: the launch's clusters are known.
+inline void set_tile_walk(KernelParams& p, int clusters) {
+    p.tiles_n_magic = p.tiles_n > 1 ? static_cast<unsigned>((0x100000000ull + p.tiles_n - 1) / p.tiles_n) : 0u;
+    p.step_m = clusters / p.tiles_n;
+    p.step_n = clusters % p.tiles_n;
+}
 
 struct WaitCtx {
     volatile uint32_t* abort_flag;  // shared memory, one per CTA
@@ -483,46 +507,53 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     wc.tile = 0;
 
     // ---------------------------------------------------------------- set-up
-    if (threadIdx.x == 0) {
-        *abort_flag = 0u;
-        prefetch_tensormap(&map_a);
-        prefetch_tensormap(&map_b);
-        prefetch_tensormap(&map_bt);
-        prefetch_tensormap(&map_d);
-        if constexpr (OP != OP_FC1) prefetch_tensormap(&map_s);
-    }
+    // Each part by a warp of its own, and the roles begin before the parts are joined: what a role works out from the
+    // parameters runs (and its code and constants are brought in) while the tensor memory is allocated and the pair's other
+    // CTA arrives.  A CTA needs 0.8 (alone) to 1.2 us (pair) of set-up otherwise, all of it on the way where the kernel ahead
+    // leaves no room for it: behind another GEMM.
     if (warp == 1) {
-        if (lane == 0) {
-            for (int s = 0; s < STAGES; s++) {
-                mbar_init(full_bar0 + 8 * s, 1);    // one arrive.expect_tx (the leader's, for the whole pair)
-                mbar_init(empty_bar0 + 8 * s, 1);   // one tcgen05.commit
-            }
-            for (int b = 0; b < 2; b++) {
-                mbar_init(tfull_bar0 + 8 * b, 1);                  // one tcgen05.commit
-                mbar_init(tempty_bar0 + 8 * b, EPI_WARPS * CG);    // one arrival per epilogue warp of the pair
-            }
-            for (int b = 0; b < (EPI_WARPS / 4) * NBUF; b++) {
-                mbar_init(side_bar0 + 8 * b, 1);     // one arrive (+ bytes) per fill of a group's box
-                mbar_init(side_free0 + 8 * b, 4);    // released by the group's four warps
-            }
+        // lane by lane: full[STAGES] empty[STAGES] tmem_full[2] tmem_empty[2] | side data landed, box reusable [boxes]
+        constexpr int PIPE = 2 * STAGES + 4, BOXES = (EPI_WARPS / 4) * NBUF;
+        static_assert(PIPE + 2 * BOXES <= 32, "one barrier per lane");
+        if (lane < PIPE + 2 * BOXES) {
+            // stages: one arrive.expect_tx (the leader's, for the whole pair) / one tcgen05.commit; accumulators: one commit /
+            // one arrival per epilogue warp of the pair; boxes: one arrive (+ bytes) per fill / the group's four warps
+            const uint32_t count = (lane < PIPE - 2) ? 1u : (lane < PIPE) ? EPI_WARPS * CG : (lane < PIPE + BOXES) ? 1u : 4u;
+            mbar_init(bar_base + 8 * lane + (lane < PIPE ? 0 : 16), count);
             fence_mbar_init();
         }
-        __syncwarp();
+    } else if (warp == 2) {
         tmem_alloc<CG>(tmem_ptr_addr, T::TMEM_COLS);
         tmem_relinquish<CG>();
+    } else if (warp == 0) {
+        if (elect_one()) {
+            *abort_flag = 0u;
+            prefetch_tensormap(&map_a);
+        }
+    } else if (warp == 3 + EPI_WARPS) {
+        if (elect_one()) {
+            prefetch_tensormap(&map_b);
+            prefetch_tensormap(&map_bt);
+        }
+    } else if (warp == 2 + EPI_WARPS) {
+        if (elect_one()) {
+            prefetch_tensormap(&map_d);
+            if constexpr (OP != OP_FC1) prefetch_tensormap(&map_s);
+        }
     }
+    __syncwarp();
     tc_fence_before();
-    if constexpr (CG == 2) {
-        cluster_arrive();
-        cluster_wait();
-    } else {
-        __syncthreads();
-    }
-    tc_fence_after();
-    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
-    // Everything above (barriers, tensor memory, descriptors) runs beside the tail of the kernel ahead on the stream, and so
-    // does what each role can do without global memory: it calls pdl_wait() directly in front of its first access.  No
-    // two GEMM CTAs share an SM (each takes more than half its shared memory), so the next GEMM's CTAs move in as these leave.
+    if constexpr (CG == 2) cluster_arrive();
+    // Every warp calls this once, before it touches a barrier, shared memory or tensor memory.  Everything above it (and what a
+    // role does before it calls pdl_wait(), directly in front of its first access to global memory) may run beside the tail of
+    // the kernel ahead on the stream.  No two GEMM CTAs share an SM (each takes more than half its shared memory), so the next
+    // GEMM's CTAs move in as these leave.
+    const auto join_setup = [&]() {
+        if constexpr (CG == 2) cluster_wait();
+        else __syncthreads();
+        tc_fence_after();
+    };
+    const auto tmem_address = [&]() { return __shfl_sync(0xffffffffu, *tmem_ptr, 0); };
 
     // ---------------------------------------------------------------- roles
     if (warp == 0 || warp == 3 + EPI_WARPS) {
@@ -543,15 +574,16 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const bool prof = prof_total && !(p.flags & (FLAG_COARSE_TRACE | DBG_COARSE_TRACE));
         const uint32_t full_bar_leader = (CG == 2) ? map_to_cta(full_bar0, 0) : full_bar0;
         long long t_wait = 0, t_begin = 0;
-        bool waited = false;
+        bool waited = false, joined = false;
+        TileWalk walk(p, cluster_id);
         if (!is_a) {
             // The first tile's weights are asked into L2 before the kernel ahead has finished (a hint: were that kernel to write
             // them, L2 would hold what it wrote).  The row-blocks of the first round share the work: each asks for every
             // `sharing`-th k-block of its columns.  A model's weights come from HBM whenever a layer is reached, and a copy that
             // misses L2 takes 0.4 us longer, twice in a row where K is deep (block of 729 rows 45.1 -> 42.8 us, 1 568 rows
             // 42.5 -> 40.7; of 5 003 rows and more no difference).
-            const int tm = cluster_id / p.tiles_n, tn = cluster_id - tm * p.tiles_n;
-            const int sharing = (num_clusters + p.tiles_n - 1) / p.tiles_n;
+            const int tm = walk.tm, tn = walk.tn;
+            const int sharing = p.step_m + (p.step_n != 0 ? 1 : 0);
             const bool tail = (tn == p.tiles_n - 1) && (p.tail_cols != TN);
             const int nb = tn * TN + static_cast<int>(cta_rank) * (tail ? p.tail_cols / CG : T::B_ROWS);
             const CUtensorMap* const bmap = tail ? &map_bt : &map_b;
@@ -563,10 +595,9 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 __syncwarp();
             }
         }
-        for (int tile = cluster_id; ok && tile < p.num_tiles; tile += num_clusters) {
-            wc.tile = tile;
-            const int tm = tile / p.tiles_n;
-            const int tn = tile - tm * p.tiles_n;
+        for (; ok && walk.tile < p.num_tiles; walk.next(p, num_clusters)) {
+            wc.tile = walk.tile;
+            const int tm = walk.tm, tn = walk.tn;
             const int m0 = tm * (T::TILE_M_CTA * CG) + static_cast<int>(cta_rank) * T::TILE_M_CTA;
             // The last N tile may be narrower: each CTA of a pair then holds tail_cols / CG rows of B,
             // brought by a tensor map whose box is that tall (map_bt), and the MMAs are issued with N = tail_cols.
@@ -578,7 +609,8 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                                                             (SL8_DBG(p.flags, DBG_SKIP_B) ? 0 : T::KATOMS * b_rows * 128));
             const bool skip_mine = is_a ? SL8_DBG(p.flags, DBG_SKIP_A) : SL8_DBG(p.flags, DBG_SKIP_B);
             const CUtensorMap* const bmap = tail ? &map_bt : &map_b;
-            const int drop_kb = (!is_a && (p.flags & FLAG_TEST_DROP_B) && tile == cluster_id) ? 1 : -1;   // evaluated once per tile
+            const int drop_kb = (!is_a && (p.flags & FLAG_TEST_DROP_B) && walk.tile == cluster_id) ? 1 : -1;   // evaluated once per tile
+            if (!joined) { join_setup(); joined = true; }
             for (int kb = 0; kb < p.k_blocks; kb++) {
                 const long long t0 = prof ? clock64() : 0;
                 ok = __all_sync(0xffffffffu, wait_bar<SL8_SPIN_CRITICAL>(empty_bar0 + 8 * stage, phase ^ 1u, wc, ST_PRODUCER_EMPTY_WAIT, stage)) != 0;
@@ -660,6 +692,9 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const bool prof_any = p.prof != nullptr;
             const bool prof = prof_any && !(p.flags & (FLAG_COARSE_TRACE | DBG_COARSE_TRACE));
             long long t_full = 0, t_tmem = 0, n_tiles = 0, t_mma = 0, t_commit = 0;
+            TileWalk walk(p, cluster_id);
+            join_setup();
+            const uint32_t tmem_base = tmem_address();
             pdl_wait();              // nothing to wait for before that: the bounded waits start with the kernel's own work
             pdl_release();
             const long long t_begin = clock64();
@@ -682,8 +717,8 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 else mma_commit(empty_bar0 + 8 * st);
             };
 
-            for (int tile = cluster_id; ok && tile < p.num_tiles; tile += num_clusters) {
-                wc.tile = tile;
+            for (; ok && walk.tile < p.num_tiles; walk.next(p, num_clusters)) {
+                wc.tile = walk.tile;
                 long long t0 = prof_any ? clock64() : 0;     // once per tile: timed in the coarse mode too
                 ok = all_ok(wait_bar<SL8_SPIN_CRITICAL>(tempty_bar0 + 8 * acc, acc_phase ^ 1u, wc, ST_MMA_TMEM_EMPTY_WAIT, acc));
                 if (prof_any) t_tmem += clock64() - t0;
@@ -691,7 +726,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * T::ACC_STRIDE;
-                idesc = (tile % p.tiles_n == p.tiles_n - 1) ? idesc_tail : idesc_full;
+                idesc = (walk.tn == p.tiles_n - 1) ? idesc_tail : idesc_full;
                 int kb = 0;
                 const int k_full = p.k_blocks - 1;           // k-blocks that hold all their MMAs
                 if (!prof && !SL8_DBG(p.flags, DBG_SKIP_MMA)) {
@@ -792,6 +827,8 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 slot[PROF_MMA_ISSUE] = t_mma;
                 slot[PROF_MMA_COMMIT] = t_commit;
             }
+        } else {
+            join_setup();
         }
         __syncwarp();
     } else if (warp < 2 + EPI_WARPS) {
@@ -830,15 +867,17 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const bool prof_total = p.prof != nullptr && ew == 0;
         const bool prof = prof_total && !(p.flags & (FLAG_COARSE_TRACE | DBG_COARSE_TRACE));   // inner timers cost ~35 cycles each
         long long t_acc = 0, t_store = 0, t_ld = 0, t_math = 0, t_issue = 0, t_refill = 0;
+        TileWalk walk(p, cluster_id);
+        join_setup();
+        const uint32_t tmem_base = tmem_address();
         pdl_wait();
         pdl_release();
         const long long t_begin = clock64();
         e.scale = (p.scale_a ? ld_f32(p.scale_a) : 1.0f) * (p.scale_b ? ld_f32(p.scale_b) : 1.0f);
         e.inv_out = __frcp_rn(p.out_scale ? ld_f32(p.out_scale) : 1.0f);   // IEEE 1/x, as the CPU oracle computes it
         if constexpr (HAS_BIAS) {
-            if (cluster_id < p.num_tiles) {
-                const int tn0 = cluster_id % p.tiles_n;
-                load_bias<NB>(bnext, p.bias, p.flags, tn0 * TN + col_begin, lane, p.N);
+            if (walk.tile < p.num_tiles) {
+                load_bias<NB>(bnext, p.bias, p.flags, walk.tn * TN + col_begin, lane, p.N);
 #pragma unroll
                 for (int i = 0; i < NB; i++) {
                     if constexpr (BSM) bias_w[lane + 32 * i] = bnext[i];
@@ -847,18 +886,17 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 __syncwarp();
             }
         }
-        for (int tile = cluster_id; ok && tile < p.num_tiles; tile += num_clusters) {
-            wc.tile = tile;
-            const int tm = tile / p.tiles_n;
-            const int tn = tile - tm * p.tiles_n;
-            const long long m_warp = static_cast<long long>(tm) * (T::TILE_M_CTA * CG) + warp_row_in_tile;
+        while (ok && walk.tile < p.num_tiles) {
+            wc.tile = walk.tile;
+            const int tn = walk.tn;
+            const long long m_warp = static_cast<long long>(walk.tm) * (T::TILE_M_CTA * CG) + warp_row_in_tile;
             const int n0 = tn * TN;
 
             // The next tile's bias travels to registers while this tile is processed.
-            const int next_tile = tile + num_clusters;
-            const bool has_next = next_tile < p.num_tiles;
+            walk.next(p, num_clusters);
+            const bool has_next = walk.tile < p.num_tiles;
             if constexpr (HAS_BIAS) {
-                if (has_next) load_bias<NB>(bnext, p.bias, p.flags, (next_tile % p.tiles_n) * TN + col_begin, lane, p.N);
+                if (has_next) load_bias<NB>(bnext, p.bias, p.flags, walk.tn * TN + col_begin, lane, p.N);
             }
 
             long long t0 = prof_total ? clock64() : 0;       // once per tile: timed in the coarse mode too
@@ -1010,16 +1048,13 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             constexpr int GROUPS = EPI_WARPS / 4;
             constexpr uint32_t BOX_BYTES = 4 * T::REGION_BYTES;
             const bool skip_side = SL8_DBG(p.flags, DBG_SKIP_SIDE);
-            int my_tiles = 0;
-            if (cluster_id < p.num_tiles) my_tiles = (p.num_tiles - cluster_id + num_clusters - 1) / num_clusters;
-            const uint32_t total = static_cast<uint32_t>(my_tiles) * RPT;
             bool ok = true, waited = false;
-            for (uint32_t s = 0; ok && s < total; s++) {
-                const int tile = cluster_id + static_cast<int>(s / RPT) * num_clusters;
-                const int tm = tile / p.tiles_n;
-                const int tn = tile - tm * p.tiles_n;
-                const long long m_cta = static_cast<long long>(tm) * (T::TILE_M_CTA * CG) + cta_rank * T::TILE_M_CTA;
-                wc.tile = tile;
+            TileWalk walk(p, cluster_id);
+            join_setup();
+            for (uint32_t s = 0; ok && walk.tile < p.num_tiles; s++) {
+                const int tn = walk.tn;
+                const long long m_cta = static_cast<long long>(walk.tm) * (T::TILE_M_CTA * CG) + cta_rank * T::TILE_M_CTA;
+                wc.tile = walk.tile;
 #pragma unroll 1
                 for (int g = 0; g < GROUPS; g++) {
                     const uint32_t bsel = s % NBUF;
@@ -1081,7 +1116,10 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                         __syncwarp();
                     }
                 }
+                if (s % RPT == RPT - 1) walk.next(p, num_clusters);
             }
+        } else {
+            join_setup();
         }
         __syncwarp();
     }
@@ -1102,9 +1140,9 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         }
         __syncthreads();
     }
-    if (warp == 1) {
+    if (warp == 2) {      // the warp that allocated
         tc_fence_after();
-        tmem_dealloc<CG>(tmem_base, T::TMEM_COLS);
+        tmem_dealloc<CG>(tmem_address(), T::TMEM_COLS);
     }
 }
 

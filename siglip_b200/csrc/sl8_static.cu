@@ -183,6 +183,7 @@ SL8_API int sl8_fc1_gelu_fp8_static(const void* A, int64_t lda, const void* B, i
     p.K = K;
     p.tiles_n = tiles_n;
     p.num_tiles = static_cast<int>(nt);
+    sl8::set_tile_walk(p, clusters);
     p.k_blocks = (K + v->tk - 1) / v->tk;
     p.last_kblock_mmas = (K - (p.k_blocks - 1) * v->tk + 31) / 32;
     p.tail_cols = tail_cols;
