@@ -267,7 +267,7 @@ int run(sl8_handle_t h, const Problem& q, cudaStream_t stream) {
 
     CUtensorMap map_a, map_b, map_bt, map_d;
     rc = encode_2d(h, &map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.A, (unsigned long long)q.K, (unsigned long long)q.M,
-                   (unsigned long long)q.lda, 128, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+                   (unsigned long long)q.lda, 128, v->tn / v->cg == 64 ? 32 : 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);      // (SPLIT_A)
     if (rc != SL8_OK) return rc;
     rc = encode_2d(h, &map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.B, (unsigned long long)q.K, (unsigned long long)q.N,
                    (unsigned long long)q.ldb, 128, (unsigned)(v->tn / v->cg), CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
@@ -281,8 +281,8 @@ int run(sl8_handle_t h, const Problem& q, cudaStream_t stream) {
                        (unsigned long long)q.ldb, 128, (unsigned)(tail_cols / v->cg), CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
         if (rc != SL8_OK) return rc;
     }
-    // Staging rows (= store boxes) are 128 bytes wide, 64 where one epilogue warp's columns fill no more.
-    const int row_bytes = (v->tn / (v->epi_warps / 4)) * ob < 128 ? 64 : 128;
+    // Staging rows (= store boxes) are 128 bytes wide, 64 where one epilogue warp's columns are no multiple of that.
+    const int row_bytes = (v->tn / (v->epi_warps / 4)) * ob % 128 != 0 ? 64 : 128;
     rc = encode_2d(h, &map_d, ob == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, ob, q.D,
                    (unsigned long long)q.N, (unsigned long long)q.M, (unsigned long long)q.ldd * ob,
                    (unsigned)(row_bytes / ob), 32, CU_TENSOR_MAP_L2_PROMOTION_NONE,

@@ -134,7 +134,7 @@ struct KernelParams {
 template <int CG, int TN, int TK, int STAGES, int EPI_WARPS, int OUT, int NBUF>
 struct KernelTraits {
     static_assert(CG == 1 || CG == 2, "one CTA or a CTA pair per tile");
-    static_assert(TN == 128 || TN == 256, "tile N");
+    static_assert(TN == 64 || TN == 128 || TN == 192 || TN == 256, "tile N");
     static_assert(EPI_WARPS == 4 || EPI_WARPS == 8 || EPI_WARPS == 16, "one, two or four warps per TMEM lane quadrant");
     static_assert(NBUF >= 1 && NBUF <= 4, "staging buffers per epilogue warp");
     static constexpr int TILE_M_CTA = 128;                       // rows per CTA = TMEM lanes
@@ -142,18 +142,21 @@ struct KernelTraits {
     static constexpr int TILE_K = TK;                            // bytes of K per stage
     static constexpr int KATOMS = TK / 128;                      // 128-byte swizzle atoms per stage and operand
     static constexpr int B_ROWS = TN / CG;                       // B rows this CTA loads per stage
+    // Where a CTA's share of B has 64 rows, the B producer brings the last 32 of A's 128 as well (boxes of 32 rows): an issuing
+    // thread's copies take 2 cycles per row, so 96 + 96 rows take 192 cycles per k-block and 128 + 64 take 256.
+    static constexpr bool SPLIT_A = (B_ROWS == 64 && KATOMS == 1);
     static constexpr int A_ATOM_BYTES = TILE_M_CTA * 128;        // 16 KiB: 128 rows x 128 bytes
     static constexpr int B_ATOM_BYTES = B_ROWS * 128;
     static constexpr int A_BYTES = KATOMS * A_ATOM_BYTES;
     static constexpr int B_BYTES = KATOMS * B_ATOM_BYTES;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;        // also the bytes one CTA's TMA adds per stage
     static constexpr int ACC_STRIDE = TN;                        // TMEM columns between the two accumulators
-    static constexpr int TMEM_COLS = 2 * TN;                     // 256 or 512: a power of two >= 32
+    static constexpr int TMEM_COLS = (TN == 192) ? 512 : 2 * TN; // a power of two >= 32
     static constexpr int OUT_BYTES = (OUT == OUT_BF16) ? 2 : 1;
     static constexpr int COLS_PER_WARP = TN / (EPI_WARPS / 4);   // columns one epilogue warp covers
-    // A staging row is 128 bytes (SWIZZLE_128B), or 64 (SWIZZLE_64B) where a warp's columns fill no more: e4m3
-    // output from sixteen epilogue warps, 64 one-byte columns each.
-    static constexpr int REGION_ROW_BYTES = (COLS_PER_WARP * OUT_BYTES < 128) ? 64 : 128;
+    // A staging row is 128 bytes (SWIZZLE_128B), or 64 (SWIZZLE_64B) where a warp's columns are no multiple of that: e4m3
+    // output, 64 one-byte columns per warp (sixteen warps, 64-column tiles) or 192.
+    static constexpr int REGION_ROW_BYTES = (COLS_PER_WARP * OUT_BYTES % 128 != 0) ? 64 : 128;
     static constexpr int REGION_COLS = REGION_ROW_BYTES / OUT_BYTES;   // output columns in one staging row
     static constexpr int REGION_BYTES = 32 * REGION_ROW_BYTES;   // 32 rows of one warp
     static constexpr int STAGING_BYTES = EPI_WARPS * NBUF * REGION_BYTES;
@@ -559,7 +562,8 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     if (warp == 0 || warp == 3 + EPI_WARPS) {
         // ===== TMA producers: warp 0 brings A, the last warp brings B =====
         // Whole warps with an elected lane, like the MMA role: from a branch that only lane 0 takes, a k-block took 450 - 500
-        // cycles to issue, more than the MMAs of a 128-column tile need (FC2 1152 x 4304 at 729 rows: 437 -> 373 cycles per k-block).
+        // cycles to issue, more than the MMAs of a 128-column tile need (FC2 1152 x 4304 at 729 rows: 437 -> 373 cycles per k-block;
+        // the whole loop inside one elected branch: 12 % slower than this).
         // Both wait for the stage to be free and then issue their own copies.  Only the A producer arrives on
         // the stage's full barrier (in a CTA pair: only the leader's), announcing the bytes of everything that
         // will land on it; the other copies just count down.  The transaction count may run negative until
@@ -571,7 +575,6 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         uint32_t phase = 0;
         bool ok = true;
         const bool prof_total = p.prof != nullptr && is_a;
-        const bool prof = prof_total && !(p.flags & (FLAG_COARSE_TRACE | DBG_COARSE_TRACE));
         const uint32_t full_bar_leader = (CG == 2) ? map_to_cta(full_bar0, 0) : full_bar0;
         long long t_wait = 0, t_begin = 0;
         bool waited = false, joined = false;
@@ -595,10 +598,40 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 __syncwarp();
             }
         }
+        // The k-blocks kb .. end - 1 of a tile: wait for the stage, `issue` from one lane, go on.  What stands in this loop is what
+        // paces a small tile (its MMAs need 170 - 290 cycles per k-block), so each producer has an instance of its own,
+        // nothing in it is conditional on tracing or tests, and its clock is read only where it waits: 290 (A) and 340 cycles (B)
+        // per k-block before that (FC2 1152 x 4304 at 729 rows on 256 x 128 pairs 9.4 -> 9.1 us, on 128 x 64 tiles 9.05 -> 8.15;
+        // block of 729 rows 42.74 -> 42.33, 1 568 rows 40.6 -> 39.8).  One instance per producer, not one per tensor map:
+        // the larger code cost what the shorter loop saved.
+        const auto stream = [&](int kb, int end, auto&& issue) {
+#pragma unroll 1
+            for (; kb < end; kb++) {
+                if (!__all_sync(0xffffffffu, mbar_test_wait(empty_bar0 + 8 * stage, phase ^ 1u) != 0u)) {
+                    const long long t0 = clock64();
+                    ok = __all_sync(0xffffffffu, wait_bar<SL8_SPIN_CRITICAL>(empty_bar0 + 8 * stage, phase ^ 1u, wc, ST_PRODUCER_EMPTY_WAIT, stage)) != 0;
+                    t_wait += clock64() - t0;
+                    if (!ok) return;
+                }
+                if (!waited) {
+                    pdl_wait();
+                    pdl_release();
+                    waited = true;
+                    t_begin = clock64();
+                }
+                if (elect_one()) issue(kb, base + stage * T::STAGE_BYTES, (CG == 2 ? full_bar_leader : full_bar0) + 8 * stage);
+                __syncwarp();
+                if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+            }
+        };
+        const auto load = [](uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+            if constexpr (CG == 2) tma_load_2d_pair(dst, map, x, y, bar);
+            else tma_load_2d(dst, map, x, y, bar);
+        };
         for (; ok && walk.tile < p.num_tiles; walk.next(p, num_clusters)) {
             wc.tile = walk.tile;
-            const int tm = walk.tm, tn = walk.tn;
-            const int m0 = tm * (T::TILE_M_CTA * CG) + static_cast<int>(cta_rank) * T::TILE_M_CTA;
+            const int tn = walk.tn;
+            const int m0 = walk.tm * (T::TILE_M_CTA * CG) + static_cast<int>(cta_rank) * T::TILE_M_CTA;
             // The last N tile may be narrower: each CTA of a pair then holds tail_cols / CG rows of B,
             // brought by a tensor map whose box is that tall (map_bt), and the MMAs are issued with N = tail_cols.
             const bool tail = (tn == p.tiles_n - 1) && (p.tail_cols != TN);
@@ -607,56 +640,41 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             // (measurement builds: DBG_SKIP_A / DBG_SKIP_B leave one operand's copies out; the MMAs then read stale shared memory)
             const uint32_t stage_tx = static_cast<uint32_t>((SL8_DBG(p.flags, DBG_SKIP_A) ? 0 : T::A_BYTES) +
                                                             (SL8_DBG(p.flags, DBG_SKIP_B) ? 0 : T::KATOMS * b_rows * 128));
-            const bool skip_mine = is_a ? SL8_DBG(p.flags, DBG_SKIP_A) : SL8_DBG(p.flags, DBG_SKIP_B);
-            const CUtensorMap* const bmap = tail ? &map_bt : &map_b;
-            const int drop_kb = (!is_a && (p.flags & FLAG_TEST_DROP_B) && walk.tile == cluster_id) ? 1 : -1;   // evaluated once per tile
+            const bool skip_mine = SL8_DBG(p.flags, DBG_SKIP_LOAD) || (is_a ? SL8_DBG(p.flags, DBG_SKIP_A) : SL8_DBG(p.flags, DBG_SKIP_B));
             if (!joined) { join_setup(); joined = true; }
-            for (int kb = 0; kb < p.k_blocks; kb++) {
-                const long long t0 = prof ? clock64() : 0;
-                ok = __all_sync(0xffffffffu, wait_bar<SL8_SPIN_CRITICAL>(empty_bar0 + 8 * stage, phase ^ 1u, wc, ST_PRODUCER_EMPTY_WAIT, stage)) != 0;
-                if (prof) t_wait += clock64() - t0;
-                if (!ok) break;
-                const uint32_t a_dst = base + stage * T::STAGE_BYTES;
-                const uint32_t b_dst = a_dst + T::A_BYTES;
-                if (!waited) {
-                    pdl_wait();
-                    pdl_release();
-                    waited = true;
-                    t_begin = clock64();
-                }
-                if (elect_one()) {
-                    if (SL8_DBG(p.flags, DBG_SKIP_LOAD)) {   // measurement aid: MMAs run on whatever shared memory holds
-                        if (cta_rank == 0 && is_a) mbar_arrive(full_bar0 + 8 * stage);
-                    } else if constexpr (CG == 2) {
-                        const uint32_t bar = full_bar_leader + 8 * stage;
-                        if (is_a) {
-                            if (cta_rank == 0) mbar_arrive_expect_tx(full_bar0 + 8 * stage, 2 * stage_tx);
-                            if (!skip_mine) {
-#pragma unroll
-                                for (int a = 0; a < T::KATOMS; a++)
-                                    tma_load_2d_pair(a_dst + a * T::A_ATOM_BYTES, &map_a, kb * T::TILE_K + 128 * a, m0, bar);
-                            }
-                        } else if (!skip_mine && kb != drop_kb) {
-#pragma unroll
-                            for (int a = 0; a < T::KATOMS; a++)
-                                tma_load_2d_pair(b_dst + a * T::B_ATOM_BYTES, bmap, kb * T::TILE_K + 128 * a, nb, bar);
-                        }
-                    } else {
-                        const uint32_t bar = full_bar0 + 8 * stage;
-                        if (is_a) {
-                            mbar_arrive_expect_tx(bar, stage_tx);
-#pragma unroll
-                            for (int a = 0; a < T::KATOMS; a++)
-                                tma_load_2d(a_dst + a * T::A_ATOM_BYTES, &map_a, kb * T::TILE_K + 128 * a, m0, bar);
-                        } else if (kb != drop_kb) {
-#pragma unroll
-                            for (int a = 0; a < T::KATOMS; a++)
-                                tma_load_2d(b_dst + a * T::B_ATOM_BYTES, bmap, kb * T::TILE_K + 128 * a, nb, bar);
-                        }
+            if (is_a) {
+                stream(0, p.k_blocks, [&](int kb, uint32_t a_dst, uint32_t bar) {
+                    if (cta_rank == 0) {
+                        if (SL8_DBG(p.flags, DBG_SKIP_LOAD)) mbar_arrive(full_bar0 + 8 * stage);   // measurement aid: MMAs run on whatever shared memory holds
+                        else mbar_arrive_expect_tx(full_bar0 + 8 * stage, CG * stage_tx);
                     }
+                    if (skip_mine) return;
+                    if constexpr (T::SPLIT_A) {
+#pragma unroll
+                        for (int r = 0; r < 3; r++) load(a_dst + r * 32 * 128, &map_a, kb * T::TILE_K, m0 + 32 * r, bar);
+                    } else {
+#pragma unroll
+                        for (int a = 0; a < T::KATOMS; a++) load(a_dst + a * T::A_ATOM_BYTES, &map_a, kb * T::TILE_K + 128 * a, m0, bar);
+                    }
+                });
+            } else {
+                const auto b_loop = [&](int kb0, int end, const CUtensorMap* map) {
+                    stream(kb0, end, [&](int kb, uint32_t a_dst, uint32_t bar) {
+                        if (skip_mine) return;
+                        if constexpr (T::SPLIT_A) load(a_dst + 96 * 128, &map_a, kb * T::TILE_K, m0 + 96, bar);
+#pragma unroll
+                        for (int a = 0; a < T::KATOMS; a++) load(a_dst + T::A_BYTES + a * T::B_ATOM_BYTES, map, kb * T::TILE_K + 128 * a, nb, bar);
+                    });
+                };
+                // (test aid: with FLAG_TEST_DROP_B k-block 1 of the first tile is never brought)
+                int kb0 = 0, end = ((p.flags & FLAG_TEST_DROP_B) && walk.tile == cluster_id) ? 1 : p.k_blocks;
+                for (;;) {
+                    b_loop(kb0, end, tail ? &map_bt : &map_b);
+                    if (!ok || end == p.k_blocks) break;
+                    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+                    kb0 = 2;
+                    end = p.k_blocks;
                 }
-                __syncwarp();
-                if (++stage == STAGES) { stage = 0; phase ^= 1u; }
             }
         }
         if (prof_total && lane == 0) {
