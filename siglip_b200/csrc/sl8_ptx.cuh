@@ -77,6 +77,12 @@ __device__ __forceinline__ uint4 ld_16(const void* p) {
     return q;
 }
 
+// 32 bytes from a 32-byte boundary.
+__device__ __forceinline__ void ld_32(const void* p, uint32_t (&w)[8]) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p) : "memory");
+}
+
 // ---------------------------------------------------------------- mbarrier
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
