@@ -41,7 +41,6 @@ __device__ __forceinline__ uint4 ld_once_16(const void* p) {         // 16 bytes
 // pixels), in pairs (even patch: a pair never straddles two patches), or whole (a patch is a whole number of chunks).
 enum : int { UNFOLD_BYTES = 0, UNFOLD_PAIRS = 1, UNFOLD_CHUNKS = 2 };
 constexpr int kUnfoldThreads = 256;     // at most: a whole number of image rows, chunk by chunk
-constexpr int kUnfoldBatch = 4;         // chunks a thread has in flight
 
 __device__ __forceinline__ void sts_u8(uint32_t at, uint32_t v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(at), "r"(v) : "memory"); }
 __device__ __forceinline__ void sts_u16(uint32_t at, uint16_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(v) : "memory"); }
@@ -93,15 +92,15 @@ __device__ __forceinline__ void unfold_put(const uint4& q, uint64_t inv2, uint32
 // (aligned down from the first pixel; what lies outside the group is dropped), quantised, placed in shared memory at
 // the position they have in the group's rows of A (column c * P * P + py * P + px, the flattening order of a Conv2d
 // weight [N, C, P, P]) and those rows are then written whole, pad included.
-// Bound by HBM where three things are seen to.  Bytes in flight: four 16-byte loads per thread (it was one load of two
-// pixels).  Banks: rows of A are multiples of 128 bytes, so unpadded the same pixel of every patch falls into one bank; 16
+// Bound by HBM where three things are seen to.  Bytes in flight: three, four or six 16-byte loads per thread (it was one load of
+// two pixels), see unfold_batch.  Banks: rows of A are multiples of 128 bytes, so unpadded the same pixel of every patch falls into one bank; 16
 // bytes of pad per row spread eight patches over all of them.  Instructions: a thread keeps its chunk position and walks
 // down the image rows, so that where its codes go is worked out once (ALIGNED: every image row starts on a 16-byte
 // boundary, and an image is less than 4 GiB) and a chunk costs its load, conversion, stores and a few additions; dividing
 // for every pair of pixels took 24 instructions per pixel, and the kernel ran at a third of the bandwidth, issue-bound.
-// 256 images of 384 x 384, patch 14: bf16 130 -> 70 us (4.9 TB/s), fp32 123 -> 97 us (5.7 TB/s); 32 images of 224 x 224,
-// patch 16, fp32: 11.5 -> 5.0 us; one such image 7.1 -> 2.2 us.
-template <typename PT, int MODE, bool ALIGNED>
+// 256 images of 384 x 384, patch 14: bf16 130 -> 65.5 us (5.3 TB/s), fp32 123 -> 89.5 us (6.2 TB/s); 32 images of 224 x 224,
+// patch 16, fp32: 11.5 -> 4.3 us; one such image 7.1 -> 2.0 us.
+template <typename PT, int MODE, bool ALIGNED, int BATCH>
 __global__ void __launch_bounds__(kUnfoldThreads, 4)
 patchify_quantize_kernel(const PT* pixels, long long total, int H, int W, int P, int C, int gh, int gw, int G, int groups,
                          int rows_per_step, FastDiv by_chunks, FastDiv by_patch, FastDiv by_vecs, const float* scale,
@@ -138,28 +137,28 @@ patchify_quantize_kernel(const PT* pixels, long long total, int H, int W, int P,
             uint32_t src = static_cast<uint32_t>(row0) * W * sizeof(PT) + 16u * v, dst = tile + row0 * P;
             while (py >= P) { py -= P; src += plane_step; }
             while (left > 0) {
-                uint4 q[kUnfoldBatch];
+                uint4 q[BATCH];
 #pragma unroll
-                for (int b = 0; b < kUnfoldBatch; b++) {
+                for (int b = 0; b < BATCH; b++) {
                     if (left > b * rows_per_step) q[b] = ld_once_16(base + src);
                     src += row_step;
                     py += rows_per_step;
                     while (py >= P) { py -= P; src += plane_step; }
                 }
 #pragma unroll
-                for (int b = 0; b < kUnfoldBatch; b++) {
+                for (int b = 0; b < BATCH; b++) {
                     if (left > b * rows_per_step) unfold_put<PT, MODE, false, NO>(q[b], inv2, dst, to);
                     dst += dst_step;
                 }
-                left -= kUnfoldBatch * rows_per_step;
+                left -= BATCH * rows_per_step;
             }
         }
     } else if (row0 < rows_per_step) {
-        for (int cp0 = row0; cp0 < CP; cp0 += rows_per_step * kUnfoldBatch) {
-            uint4 q[kUnfoldBatch];
-            int x[kUnfoldBatch];                          // first pixel of the chunk relative to the group
+        for (int cp0 = row0; cp0 < CP; cp0 += rows_per_step * BATCH) {
+            uint4 q[BATCH];
+            int x[BATCH];                          // first pixel of the chunk relative to the group
 #pragma unroll
-            for (int b = 0; b < kUnfoldBatch; b++) {
+            for (int b = 0; b < BATCH; b++) {
                 const int cp = cp0 + b * rows_per_step;
                 x[b] = len;
                 if (cp >= CP) continue;
@@ -177,7 +176,7 @@ patchify_quantize_kernel(const PT* pixels, long long total, int H, int W, int P,
                 }
             }
 #pragma unroll
-            for (int b = 0; b < kUnfoldBatch; b++) {
+            for (int b = 0; b < BATCH; b++) {
                 if (x[b] >= len) continue;
                 unfold_offsets<VP, NO>(to, x[b], len, P, by_patch, pitch, -1);
                 unfold_put<PT, MODE, true, NO>(q[b], inv2, tile + (cp0 + b * rows_per_step) * P, to);
@@ -210,18 +209,39 @@ patchify_quantize_kernel(const PT* pixels, long long total, int H, int W, int P,
     }
 }
 
+// Chunks a thread has in flight, of the `steps` it takes in all: as many as leave the fewest places of the last round empty, and of
+// those the most; the fewest where patch rows are cut into groups, because there are hardly two blocks per SM.  A round that is not full is a trip to memory for less.  256 images of 384 x 384, patch 14 (9 steps bf16, 21 fp32):
+// 3 / 4 / 6 in flight 65.5 / 70.6 / 73.5 us, 89.5 / 94.5 / 95.6; 512 of 224 x 224, patch 16, bf16 (6): 47.7 / 51.0 / 44.9; 32 of them, fp32 (12):
+// 5.3 / 5.0 / 4.3; 976 of 128 x 160, patch 16 (4 and 8): 40.7 / 36.7 / 41.9, 50.5 / 48.2 / 58.1; cut into groups (6), 13 of 224 x 224, patch 16: 2.8 / 3.0 / 3.2.
+inline int unfold_batch(int steps, bool cut) {
+    int best = 3, idle = (3 - steps % 3) % 3;
+    for (int b : {4, 6}) {
+        const int i = (b - steps % b) % b;
+        if (i < idle || (i == idle && !cut)) best = b, idle = i;
+    }
+    return best;
+}
+
+template <typename PT, int MODE, bool ALIGNED, int BATCH>
+cudaError_t launch_unfold_batch(unsigned grid, unsigned threads, size_t smem, cudaStream_t s, const PT* pixels, long long total, int H, int W, int P, int C, int gh, int gw,
+                                int G, int groups, int rows_per_step, int chunks, const float* scale, uint8_t* A, long long lda, int row_bytes) {
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(patchify_quantize_kernel<PT, MODE, ALIGNED, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    return sl8_launch_chained(patchify_quantize_kernel<PT, MODE, ALIGNED, BATCH>, grid, threads, smem, s, pixels, total, H, W, P, C, gh, gw, G, groups, rows_per_step,
+                              fast_div(chunks), fast_div(P), fast_div(row_bytes / 16), scale, A, lda, row_bytes);
+}
+
 template <typename PT, int MODE, bool ALIGNED>
 cudaError_t launch_unfold(unsigned grid, size_t smem, cudaStream_t s, const PT* pixels, int images, int C, int H, int W, int P,
                           int gh, int gw, int G, int groups, int chunks, const float* scale, uint8_t* A, long long lda, int row_bytes) {
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(patchify_quantize_kernel<PT, MODE, ALIGNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
     const int rows_per_step = kUnfoldThreads / chunks;                       // image rows a step of the block covers
-    const int threads = (rows_per_step * chunks + 31) / 32 * 32;
+    const unsigned threads = static_cast<unsigned>((rows_per_step * chunks + 31) / 32 * 32);
     const long long total = static_cast<long long>(images) * C * H * W;
-    return sl8_launch_chained(patchify_quantize_kernel<PT, MODE, ALIGNED>, grid, threads, smem, s, pixels, total, H, W, P, C, gh, gw, G, groups, rows_per_step,
-                              fast_div(chunks), fast_div(P), fast_div(row_bytes / 16), scale, A, lda, row_bytes);
+    const int batch = unfold_batch((C * P + rows_per_step - 1) / rows_per_step, groups > 1);
+    auto go = [&](auto launch) { return launch(grid, threads, smem, s, pixels, total, H, W, P, C, gh, gw, G, groups, rows_per_step, chunks, scale, A, lda, row_bytes); };
+    return batch == 3 ? go(launch_unfold_batch<PT, MODE, ALIGNED, 3>) : batch == 4 ? go(launch_unfold_batch<PT, MODE, ALIGNED, 4>) : go(launch_unfold_batch<PT, MODE, ALIGNED, 6>);
 }
 
 template <typename PT>
