@@ -92,7 +92,7 @@ enum {
 typedef struct sl8_config {
     int cta_group;     /* 1 = one CTA per tile, 2 = CTA pair (tcgen05 cta_group::2)        */
     int tile_m;        /* rows per tile (128 * cta_group)                                    */
-    int tile_n;        /* columns per tile                                                   */
+    int tile_n;        /* columns per tile (128 too where two neighbouring CTAs halve such a tile: variant 20) */
     int tile_k;        /* K bytes per pipeline stage                                         */
     int stages;        /* depth of the TMA -> MMA shared-memory ring                          */
     int epi_warps;     /* epilogue warps per CTA                                              */
@@ -290,7 +290,8 @@ int sl8_mlp_chain_fp8_host(sl8_handle_t h,
 int sl8_query_config(sl8_handle_t h, int op, int out_dtype, int64_t M, int N, int K, sl8_config* out);
 int sl8_query_config_flags(sl8_handle_t h, int op, int out_dtype, unsigned flags, int64_t M, int N, int K, sl8_config* out);
 
-/* Number of compiled variants, and the description of variant `variant_id`. */
+/* Number of variants whose tiles have 128 or 256 columns, and the description of variant `variant_id` of them.  The dispatch has one
+ * more, with 192 columns: sl8_query_config names it, sl8_set_variant takes it. */
 int sl8_num_variants(void);
 int sl8_describe_variant(int variant_id, sl8_config* out);
 

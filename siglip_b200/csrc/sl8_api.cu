@@ -27,6 +27,7 @@ const VariantEntry* variant(int id) {
     case id_:                             \
         return sl8_variant_##id_();
         SL8_VARIANT_LIST(SL8_CASE)
+        SL8_192_LIST(SL8_CASE)
 #undef SL8_CASE
         default:
             return nullptr;
@@ -67,13 +68,14 @@ int kernel_slot(int op, int out_dtype) {
 // hides its mainloop (`next` per k-block, more than `first` when every SM asks L2) behind the epilogue ahead of it or the
 // other way round (`tile`: the epilogue's own pace).  The constants (sl8_cost_model.h) are fitted so that the cheapest variant by
 // the formula is the fastest one measured, from 512 to 4 800 wide and 50 to 186 624 rows: on that sweep (488 points that the table
-// leaves to it, sweeps/b200_model.csv) it is 0.1 - 2.2 % off the fastest on average, by class, and 15 % at worst (GELU, 32 000 x
-// 1 152 x 4 304).  What it decides: 128 x 128 tiles on single CTAs with
-// eight epilogue warps (18) while there are few tiles (an epilogue half as long at the end: FC1 4 304 x 1 152 at 512 rows
-// 9.9 us with v3, 7.3 with v18; FC2 1 152 x 1 152 at 2 048 rows 10.0 with v1, 7.3); 256 x 128 pairs (19) where
-// 256 x 256 tiles leave most of the last round empty (FC2 1 152 x 1 152 at 5 003 rows 14.8 with v1, 11.8); eight epilogue warps
-// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 52.0 with v1,
-// 38.6 with v17); a fifth stage (2) where K is deep behind a light epilogue (hardware tanh, 1 152 x 4 304 at 46 656 rows 197.7 with v3, 180.8).
+// leaves to it, sweeps/b200_model.csv) it is 0.1 - 0.9 % off the fastest on average, by class, and 14 % at worst (no activation);
+// at eighteen other widths with sixteen row counts each 0.5 - 1.0 % and 12 %.  What it decides: tiles of 128 x 64 on single CTAs (20)
+// while there are too few of 128 x 128 to fill the chip, or their ring of four stages would wait for L2 (FC2 1 152 x 1 152 at 729 rows
+// 5.2 us with 18, 4.6 with 20); then 128 x 128 with eight epilogue warps (18); pairs
+// with 256 x 128 (19) and 256 x 192 (21) where 256 x 256 tiles leave most of the last round empty (FC2 1 152 x 4 304 at 5 003 rows 27.0 with 1,
+// 23.7 with 21; 1 152 x 1 152 13.1 with 1, 11.8 with 19, 11.4 with 21); eight epilogue warps
+// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 52.0 with 1,
+// 38.6 with 17); a fifth stage (2) where K is deep behind a light epilogue (hardware tanh, 1 152 x 4 304 at 46 656 rows 197.7 with 3, 180.8 with 2).
 enum CostClass : int { COST_GELU, COST_TANH, COST_NONE, COST_FC2, COST_PE };
 struct VariantCost {
     CostClass cls;
@@ -90,12 +92,16 @@ long long clusters_of(sl8_handle_t h, const VariantEntry* v) {
     return h && h->max_clusters_override > 0 && clusters > h->max_clusters_override ? h->max_clusters_override : clusters;
 }
 
+// Tiles of 64 and 192 columns are candidates from this width on.  The sweep's narrowest layer has 512 columns, and 432 were tried
+// beside it; below, where a last column of tiles is most of a layer, the choice is left to the variants it was made for.
+constexpr int kNewTilesFrom = 416;
+
 int cheapest_variant(sl8_handle_t h, CostClass cls, int slot, long long M, int N, int K) {
     int best = 1;
     float best_us = 3.4e38f;
     for (const VariantCost& c : kVariantCost) {
         const VariantEntry* v = c.cls == cls ? variant(c.variant) : nullptr;
-        if (!v || !v->kernel[slot]) continue;
+        if (!v || !v->kernel[slot] || (N < kNewTilesFrom && (v->tn == 64 || v->tn == 192))) continue;
         const long long tiles = ((M + 128 * v->cg - 1) / (128 * v->cg)) * ((N + v->tn - 1) / v->tn), clusters = clusters_of(h, v);
         const float rounds = static_cast<float>((tiles + clusters - 1) / clusters), k_blocks = static_cast<float>((K + 127) / 128);
         const float later = k_blocks * c.next > c.tile ? k_blocks * c.next : c.tile;
@@ -345,7 +351,7 @@ int run(sl8_handle_t h, const Problem& q, cudaStream_t stream) {
 void fill_config(const VariantEntry* v, int slot, int grid, sl8_config* out) {
     out->cta_group = v->cg;
     out->tile_m = 128 * v->cg;
-    out->tile_n = v->tn;
+    out->tile_n = v->tn == 64 ? 128 : v->tn;      // (two neighbouring CTAs halve a tile of 128 columns)
     out->tile_k = v->tk;
     out->stages = v->stages;
     out->epi_warps = v->epi_warps;
@@ -790,10 +796,10 @@ SL8_API int sl8_mlp_chain_fp8_host(sl8_handle_t h, const void* A, int64_t lda, c
 
 // =========================================================================== dispatch
 
-SL8_API int sl8_num_variants(void) { return SL8_NUM_VARIANTS; }
+SL8_API int sl8_num_variants(void) { return SL8_LISTED_VARIANTS; }
 
 SL8_API int sl8_describe_variant(int variant_id, sl8_config* out) {
-    const VariantEntry* v = variant(variant_id);
+    const VariantEntry* v = variant_id < SL8_LISTED_VARIANTS ? variant(variant_id) : nullptr;
     if (!v || !out) return SL8_ERR_INVALID_VALUE;
     fill_config(v, sl8::K_FC1_BF16, 0, out);
     return SL8_OK;

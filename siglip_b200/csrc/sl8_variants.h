@@ -11,6 +11,7 @@
 
 // X(id, CG, TN, TK, STAGES, EPI_WARPS, NBUF)
 //   CG         1 = one CTA per 128 x TN tile, 2 = CTA pair per 256 x TN tile
+//   TN         columns of a CTA's (pair's) tile; with 64 two neighbouring CTAs halve a tile of 128 columns, which is what is reported
 //   TK         bytes of K per pipeline stage: 128 or 256 (one or two swizzle atoms; with 256 the
 //              MMA thread issues eight MMAs per barrier round trip instead of four)
 //   STAGES     depth of the operand ring (bounded by the 227 KiB of shared memory)
@@ -39,9 +40,14 @@
     X(16, 2, 256, 128, 6, 4, 2)  \
     X(17, 2, 256, 128, 4, 8, 3)  \
     X(18, 1, 128, 128, 4, 8, 2)  \
-    X(19, 2, 128, 128, 6, 8, 2)
+    X(19, 2, 128, 128, 6, 8, 2)  \
+    X(20, 1, 64, 128, 8, 4, 2)
 
-#define SL8_NUM_VARIANTS 20
+// A last one that the dispatch and sl8_set_variant reach, beside those that sl8_describe_variant lists (tiles of 128 and 256 columns).
+#define SL8_192_LIST(X) X(21, 2, 192, 128, 6, 4, 3)
+
+#define SL8_LISTED_VARIANTS 21
+#define SL8_NUM_VARIANTS 22
 
 namespace sl8 {
 
@@ -66,4 +72,5 @@ struct VariantEntry {
 
 #define SL8_DECLARE_VARIANT(id, CG, TN, TK, ST, EW, NB) extern "C" const sl8::VariantEntry* sl8_variant_##id();
 SL8_VARIANT_LIST(SL8_DECLARE_VARIANT)
+SL8_192_LIST(SL8_DECLARE_VARIANT)
 #undef SL8_DECLARE_VARIANT
