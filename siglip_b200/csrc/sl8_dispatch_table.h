@@ -17,7 +17,7 @@ static const Sl8DispatchRow kSl8DispatchTable[] = {
     {SL8_OP_PATCH_EMBED, 1152, 588, 4374LL, 19},
     {SL8_OP_PATCH_EMBED, 1152, 588, 7290LL, 17},
     {SL8_OP_PATCH_EMBED, 1152, 588, 8748LL, 19},
-    {SL8_OP_PATCH_EMBED, 1152, 588, 46656LL, 5},
+    {SL8_OP_PATCH_EMBED, 1152, 588, 46656LL, 17},
     {SL8_OP_FC1_GELU, 3072, 768, 0LL, 20},
     {SL8_OP_FC1_GELU, 3072, 768, 490LL, 18},
     {SL8_OP_FC1_GELU, 3072, 768, 6272LL, 14},

@@ -103,6 +103,11 @@ def best_rows(rows: list[dict], keep_margin: float = 0.02) -> list[dict]:
                 # limit sets the pace, and boxes differ by more than that
                 choice = next((int(r["variant"]) for r in cands if str(r["tile_n"]) != "192"
                                and float(r["ms_median"]) <= float(best["ms_median"]) * 1.03), choice)
+            if op == OPS["pe"] and str(best.get("tile_n")) == "256" and str(best.get("epi_warps")) == "4":
+                # a burst ranks four epilogue warps up to 2 % ahead of eight, sustained they are 1.4 % behind (186 624 x 1 152 x 588 with
+                # the unfold ahead of it 261.1 against 257.6 us)
+                choice = next((int(r["variant"]) for r in cands if str(r.get("epi_warps")) == "8" and str(r.get("tile_n")) == "256"
+                               and float(r["ms_median"]) <= float(best["ms_median"]) * 1.02), choice)
             if prev is not None and prev != choice and not (str(best.get("tile_n")) == "192" and prev == int(best["variant"])):
                 mine = [r for r in cands if int(r["variant"]) == prev]
                 if mine and float(mine[0]["ms_median"]) <= float(best["ms_median"]) * (1.0 + keep_margin):
