@@ -92,7 +92,7 @@ enum {
 typedef struct sl8_config {
     int cta_group;     /* 1 = one CTA per tile, 2 = CTA pair (tcgen05 cta_group::2)        */
     int tile_m;        /* rows per tile (128 * cta_group)                                    */
-    int tile_n;        /* columns per tile (128 too where two neighbouring CTAs halve such a tile: variant 20) */
+    int tile_n;        /* columns per tile                                                   */
     int tile_k;        /* K bytes per pipeline stage                                         */
     int stages;        /* depth of the TMA -> MMA shared-memory ring                          */
     int epi_warps;     /* epilogue warps per CTA                                              */

@@ -351,7 +351,7 @@ int run(sl8_handle_t h, const Problem& q, cudaStream_t stream) {
 void fill_config(const VariantEntry* v, int slot, int grid, sl8_config* out) {
     out->cta_group = v->cg;
     out->tile_m = 128 * v->cg;
-    out->tile_n = v->tn == 64 ? 128 : v->tn;      // (two neighbouring CTAs halve a tile of 128 columns)
+    out->tile_n = v->tn;
     out->tile_k = v->tk;
     out->stages = v->stages;
     out->epi_warps = v->epi_warps;

@@ -11,7 +11,6 @@
 
 // X(id, CG, TN, TK, STAGES, EPI_WARPS, NBUF)
 //   CG         1 = one CTA per 128 x TN tile, 2 = CTA pair per 256 x TN tile
-//   TN         columns of a CTA's (pair's) tile; with 64 two neighbouring CTAs halve a tile of 128 columns, which is what is reported
 //   TK         bytes of K per pipeline stage: 128 or 256 (one or two swizzle atoms; with 256 the
 //              MMA thread issues eight MMAs per barrier round trip instead of four)
 //   STAGES     depth of the operand ring (bounded by the 227 KiB of shared memory)

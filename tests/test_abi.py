@@ -41,7 +41,7 @@ def test_version_and_variants(lib):
     for v in range(n):
         c = describe_variant(v)
         assert c["variant_id"] == v and c["cta_group"] in (1, 2) and c["tile_m"] == 128 * c["cta_group"]
-        assert c["tile_n"] in (128, 256) and c["tile_k"] in (128, 256) and c["smem_bytes"] <= 232448
+        assert c["tile_n"] in (64, 128, 256) and c["tile_k"] in (128, 256) and c["smem_bytes"] <= 232448
         seen.add((c["cta_group"], c["tile_n"], c["stages"], c["epi_warps"], c["staging_buffers"]))
     assert len(seen) == n
     with pytest.raises(Exception):
@@ -56,8 +56,25 @@ def test_query_config_without_handle(lib):
     assert lib.sl8_query_config(None, L.SL8_OP_FC2_RESIDUAL, L.SL8_OUT_BF16, 46656, 1152, 4304, C.byref(cfg)) == 0
     assert cfg.tile_n == 256
     assert lib.sl8_query_config(None, L.SL8_OP_FC2_RESIDUAL, L.SL8_OUT_BF16, 729, 1152, 4304, C.byref(cfg)) == 0
-    assert cfg.tile_n == 128 and cfg.cta_group == 1       # too few 256-wide tiles for 148 SMs
+    assert cfg.tile_n == 64 and cfg.cta_group == 1        # too few 256-wide tiles for 148 SMs
     assert lib.sl8_query_config(None, 7, 0, 10, 16, 16, C.byref(cfg)) == L.SL8_ERR_INVALID_VALUE
+
+
+def test_the_reported_tile_is_the_one_the_grid_walks(lib):
+    """Rows and columns of a tile, as reported, give the tiles of a call: one CTA (pair) each until the GPU is full."""
+    import siglip_b200.lib as L
+    from siglip_b200.layers import describe_variant
+    from siglip_b200.sweep import variant_tiles
+    tiles = variant_tiles()
+    cfg = L.Config()
+    for v in range(lib.sl8_num_variants()):
+        c = describe_variant(v)
+        assert (c["cta_group"], c["tile_n"]) == tiles[v]
+    for op, n, k in ((L.SL8_OP_PATCH_EMBED, 768, 768), (L.SL8_OP_FC1_GELU, 3072, 768), (L.SL8_OP_FC2_RESIDUAL, 1152, 4304), (L.SL8_OP_FC2_RESIDUAL, 1600, 4800)):
+        for m in (1, 196, 729, 1568, 5003, 46656):
+            assert lib.sl8_query_config(None, op, L.SL8_OUT_BF16, m, n, k, C.byref(cfg)) == 0
+            count = -(-m // cfg.tile_m) * -(-n // cfg.tile_n)
+            assert cfg.grid == min(count, 148 // cfg.cta_group) * cfg.cta_group, (op, m, n, k)
 
 
 def test_null_handle_is_rejected(lib):

@@ -1,4 +1,4 @@
-"""Tiles of 64 columns (variant 20, halves of a 128-column tile) and of 192 (variant 21), and what else the cost model picks beside the
+"""Tiles of 64 columns (variant 20) and of 192 (variant 21), and what else the cost model picks beside the
 rows of tests/test_gpu_dispatch.py: bit for bit what the general variant gives."""
 import pytest
 import torch
