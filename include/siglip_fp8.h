@@ -290,8 +290,7 @@ int sl8_mlp_chain_fp8_host(sl8_handle_t h,
 int sl8_query_config(sl8_handle_t h, int op, int out_dtype, int64_t M, int N, int K, sl8_config* out);
 int sl8_query_config_flags(sl8_handle_t h, int op, int out_dtype, unsigned flags, int64_t M, int N, int K, sl8_config* out);
 
-/* Number of variants whose tiles have 128 or 256 columns, and the description of variant `variant_id` of them.  The dispatch has one
- * more, with 192 columns: sl8_query_config names it, sl8_set_variant takes it. */
+/* Number of compiled variants, and the description of variant `variant_id`. */
 int sl8_num_variants(void);
 int sl8_describe_variant(int variant_id, sl8_config* out);
 

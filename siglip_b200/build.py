@@ -42,15 +42,14 @@ def nvcc() -> str:
     return exe
 
 
-def variant_ids(compiled: bool = False) -> list[int]:
-    """The ids that ``sl8_describe_variant`` lists; ``compiled``: and the one beside them."""
+def variant_ids() -> list[int]:
     text = (CSRC / "sl8_variants.h").read_text()
-    body = text.split("#define SL8_VARIANT_LIST(X)")[1].split("#define SL8_LISTED_VARIANTS")[0]
+    body = text.split("#define SL8_VARIANT_LIST(X)")[1].split("#define SL8_NUM_VARIANTS")[0]
     ids = [int(m) for m in re.findall(r"X\((\d+),", body)]
-    listed, declared = (int(re.search(rf"#define {name} (\d+)", text).group(1)) for name in ("SL8_LISTED_VARIANTS", "SL8_NUM_VARIANTS"))
+    declared = int(re.search(r"#define SL8_NUM_VARIANTS (\d+)", text).group(1))
     if ids != list(range(declared)):
-        raise RuntimeError(f"variant ids {ids} do not match SL8_NUM_VARIANTS {declared}")
-    return ids if compiled else ids[:listed]
+        raise RuntimeError(f"SL8_VARIANT_LIST ids {ids} do not match SL8_NUM_VARIANTS {declared}")
+    return ids
 
 
 def sources_mtime() -> float:
@@ -125,7 +124,7 @@ def build_library(verbose: bool) -> None:
     exe = nvcc()
     jobs = []
     objs = []
-    for vid in variant_ids(compiled=True):
+    for vid in variant_ids():
         o = OBJ / f"variant_{vid}.o"
         objs.append(o)
         jobs.append(([exe, *NVCC_FLAGS, f"-DSL8_VARIANT_ID={vid}", "-c", str(CSRC / "sl8_variant.cu"), "-o", str(o)],

@@ -27,7 +27,6 @@ const VariantEntry* variant(int id) {
     case id_:                             \
         return sl8_variant_##id_();
         SL8_VARIANT_LIST(SL8_CASE)
-        SL8_192_LIST(SL8_CASE)
 #undef SL8_CASE
         default:
             return nullptr;
@@ -796,10 +795,10 @@ SL8_API int sl8_mlp_chain_fp8_host(sl8_handle_t h, const void* A, int64_t lda, c
 
 // =========================================================================== dispatch
 
-SL8_API int sl8_num_variants(void) { return SL8_LISTED_VARIANTS; }
+SL8_API int sl8_num_variants(void) { return SL8_NUM_VARIANTS; }
 
 SL8_API int sl8_describe_variant(int variant_id, sl8_config* out) {
-    const VariantEntry* v = variant_id < SL8_LISTED_VARIANTS ? variant(variant_id) : nullptr;
+    const VariantEntry* v = variant(variant_id);
     if (!v || !out) return SL8_ERR_INVALID_VALUE;
     fill_config(v, sl8::K_FC1_BF16, 0, out);
     return SL8_OK;

@@ -77,7 +77,6 @@ const VariantEntry* make_entry() {
         static const sl8::VariantEntry* get() { return sl8::make_entry<id, CG, TN, TK, ST, EW, NB>(); } \
     };
 SL8_VARIANT_LIST(SL8_DEFINE_IF_SELECTED)
-SL8_192_LIST(SL8_DEFINE_IF_SELECTED)
 #undef SL8_DEFINE_IF_SELECTED
 
 // Only the Pick<id> specialisation matching SL8_VARIANT_ID is ever instantiated, so only its

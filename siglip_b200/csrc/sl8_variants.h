@@ -40,12 +40,9 @@
     X(17, 2, 256, 128, 4, 8, 3)  \
     X(18, 1, 128, 128, 4, 8, 2)  \
     X(19, 2, 128, 128, 6, 8, 2)  \
-    X(20, 1, 64, 128, 8, 4, 2)
+    X(20, 1, 64, 128, 8, 4, 2)   \
+    X(21, 2, 192, 128, 6, 4, 3)
 
-// A last one that the dispatch and sl8_set_variant reach, beside those that sl8_describe_variant lists (tiles of 128 and 256 columns).
-#define SL8_192_LIST(X) X(21, 2, 192, 128, 6, 4, 3)
-
-#define SL8_LISTED_VARIANTS 21
 #define SL8_NUM_VARIANTS 22
 
 namespace sl8 {
@@ -71,5 +68,4 @@ struct VariantEntry {
 
 #define SL8_DECLARE_VARIANT(id, CG, TN, TK, ST, EW, NB) extern "C" const sl8::VariantEntry* sl8_variant_##id();
 SL8_VARIANT_LIST(SL8_DECLARE_VARIANT)
-SL8_192_LIST(SL8_DECLARE_VARIANT)
 #undef SL8_DECLARE_VARIANT

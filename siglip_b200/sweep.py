@@ -141,17 +141,6 @@ def read_csv(path: Path) -> list[dict]:
 
 
 # ----------------------------------------------------------------------------- timing (GPU)
-def every_variant(eng) -> list[dict]:
-    """The configuration of every compiled variant, as a handle that is forced to it answers."""
-    from siglip_b200 import build
-    out = []
-    for v in build.variant_ids(compiled=True):
-        eng.set_variant(v)
-        out.append(dict(eng.query_config(OPS["fc1"], 1 << 20, 4096, 1024), variant_id=v))
-    eng.set_variant(-1)
-    return out
-
-
 def ladder(per_image: int, octaves: int, per_octave: int) -> list[int]:
     """per_image * 2^j; below 16 images, where the last round of tiles weighs, also the points that divide an octave into per_octave."""
     return [(per_image << j) + (per_image << j) * q // per_octave for j in range(octaves) for q in range(per_octave if j < min(4, octaves - 1) else 1)]
@@ -185,14 +174,14 @@ def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out
     """Times every admissible variant on every (layer, N, K) of the named shape sets over the M ladder."""
     import torch
     import siglip_b200
-    from siglip_b200 import build, synth
+    from siglip_b200 import build, layers, synth
     from siglip_b200.lib import SL8Error
 
     dev = "cuda"
     eng = siglip_b200.Engine(0)
     stream = torch.cuda.Stream()
     resources = parse_resources(build.resource_report())
-    all_variants = every_variant(eng)
+    all_variants = [layers.describe_variant(v) for v in range(layers.num_variants())]
     rows = []
     out_path.parent.mkdir(parents=True, exist_ok=True)
     with open(out_path, "w", newline="") as f:
@@ -421,11 +410,11 @@ def run_model_sweep(out_path: Path, repeats: int = 3, log=print) -> None:
     """Graph-replay microseconds of every admissible variant over MODEL_SHAPES x MODEL_ROWS, two operand sets in turn."""
     import torch
     import siglip_b200
-    from siglip_b200 import build, lib, synth
+    from siglip_b200 import build, layers, lib, synth
 
     eng, stream = siglip_b200.Engine(0), torch.cuda.Stream()
     resources = parse_resources(build.resource_report())
-    every = every_variant(eng)
+    every = [layers.describe_variant(v) for v in range(layers.num_variants())]
     gen = torch.Generator(device="cuda").manual_seed(0)
     normal = lambda *s: torch.randn(s, generator=gen, device="cuda").to(torch.bfloat16)
     codes = lambda r, c: (torch.randint(0, 256, (r, synth.pitch128(c)), generator=gen, device="cuda", dtype=torch.uint8) & 0xBF)[:, :c]

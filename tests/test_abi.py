@@ -41,7 +41,7 @@ def test_version_and_variants(lib):
     for v in range(n):
         c = describe_variant(v)
         assert c["variant_id"] == v and c["cta_group"] in (1, 2) and c["tile_m"] == 128 * c["cta_group"]
-        assert c["tile_n"] in (64, 128, 256) and c["tile_k"] in (128, 256) and c["smem_bytes"] <= 232448
+        assert c["tile_n"] in (64, 128, 192, 256) and c["tile_k"] in (128, 256) and c["smem_bytes"] <= 232448
         seen.add((c["cta_group"], c["tile_n"], c["stages"], c["epi_warps"], c["staging_buffers"]))
     assert len(seen) == n
     with pytest.raises(Exception):
@@ -75,6 +75,25 @@ def test_the_reported_tile_is_the_one_the_grid_walks(lib):
             assert lib.sl8_query_config(None, op, L.SL8_OUT_BF16, m, n, k, C.byref(cfg)) == 0
             count = -(-m // cfg.tile_m) * -(-n // cfg.tile_n)
             assert cfg.grid == min(count, 148 // cfg.cta_group) * cfg.cta_group, (op, m, n, k)
+
+
+def test_what_the_query_names_can_be_described(lib):
+    """The variant of a call, by its id, is among those that are listed, and described as the query does (shared memory and grid
+    are the call's own)."""
+    import siglip_b200.lib as L
+    from siglip_b200.build import variant_ids
+    from siglip_b200.layers import describe_variant, num_variants
+    assert variant_ids() == list(range(num_variants()))
+    cfg = L.Config()
+    named = set()
+    for op, n, k in ((L.SL8_OP_PATCH_EMBED, 1152, 588), (L.SL8_OP_FC1_GELU, 1600, 512), (L.SL8_OP_FC2_RESIDUAL, 1152, 4304), (L.SL8_OP_FC2_RESIDUAL, 768, 3072)):
+        for m in (1, 300, 729, 1568, 2187, 3136, 5003, 11664, 46656):
+            assert lib.sl8_query_config(None, op, L.SL8_OUT_BF16, m, n, k, C.byref(cfg)) == 0
+            listed = describe_variant(cfg.variant_id)
+            for field in ("cta_group", "tile_m", "tile_n", "tile_k", "stages", "epi_warps", "staging_buffers"):
+                assert listed[field] == getattr(cfg, field), (op, m, field)
+            named.add(cfg.tile_n)
+    assert 192 in named          # (FC2 1152 x 4304 at 5 003 rows)
 
 
 def test_null_handle_is_rejected(lib):
