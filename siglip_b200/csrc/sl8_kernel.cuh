@@ -577,7 +577,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const bool prof_total = p.prof != nullptr && is_a;
         const uint32_t full_bar_leader = (CG == 2) ? map_to_cta(full_bar0, 0) : full_bar0;
         long long t_wait = 0, t_begin = 0;
-        bool waited = false, joined = false;
+        bool waited = false;
         TileWalk walk(p, cluster_id);
         if (!is_a) {
             // The first tile's weights are asked into L2 before the kernel ahead has finished (a hint: were that kernel to write
@@ -628,6 +628,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             if constexpr (CG == 2) tma_load_2d_pair(dst, map, x, y, bar);
             else tma_load_2d(dst, map, x, y, bar);
         };
+        join_setup();            // ahead of the loop, like every role: a CTA without a tile joins too
         for (; ok && walk.tile < p.num_tiles; walk.next(p, num_clusters)) {
             wc.tile = walk.tile;
             const int tn = walk.tn;
@@ -641,7 +642,6 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const uint32_t stage_tx = static_cast<uint32_t>((SL8_DBG(p.flags, DBG_SKIP_A) ? 0 : T::A_BYTES) +
                                                             (SL8_DBG(p.flags, DBG_SKIP_B) ? 0 : T::KATOMS * b_rows * 128));
             const bool skip_mine = SL8_DBG(p.flags, DBG_SKIP_LOAD) || (is_a ? SL8_DBG(p.flags, DBG_SKIP_A) : SL8_DBG(p.flags, DBG_SKIP_B));
-            if (!joined) { join_setup(); joined = true; }
             if (is_a) {
                 stream(0, p.k_blocks, [&](int kb, uint32_t a_dst, uint32_t bar) {
                     if (cta_rank == 0) {
