@@ -19,6 +19,8 @@ from __future__ import annotations
 
 import argparse
 import csv
+import math
+import random
 import re
 import statistics
 import sys
@@ -76,12 +78,18 @@ def prune(variants: list[dict], op: int, resources: dict | None = None, out_dtyp
 
 
 # ----------------------------------------------------------------------------- table (CPU)
+def beats(a: dict, b: dict, margin: float) -> bool:
+    """Whether `a` is faster than `b` by more than `margin` and by more than the two deviations that the sweep recorded."""
+    spread = sum(float(r.get("ms_stdev") or 0.0) for r in (a, b))
+    return float(b["ms_median"]) - float(a["ms_median"]) > max(margin * float(a["ms_median"]), spread)
+
+
 def best_rows(rows: list[dict], keep_margin: float = 0.02) -> list[dict]:
     """CSV rows -> dispatch rows {op, N, K, m_min, variant}.
 
     Per (op, N, K) the M ladder is walked upwards; the winner of the previous (smaller) M is kept unless
-    another variant beats it by more than ``keep_margin`` (noise must not flip the table), and neighbouring
-    M with the same winner collapse into one row whose ``m_min`` is the smallest of them (0 for the first).  At the
+    another variant beats it by more than ``keep_margin`` and by more than the two deviations recorded (noise must not flip the
+    table), and neighbouring M with the same winner collapse into one row whose ``m_min`` is the smallest of them (0 for the first).  At the
     smallest M a single-CTA variant within 3 % of the best is taken: a CTA pair waits for two free SMs side by side."""
     groups: dict[tuple, dict[int, list[dict]]] = {}
     for r in rows:
@@ -98,19 +106,9 @@ def best_rows(rows: list[dict], keep_margin: float = 0.02) -> list[dict]:
             if prev is None:
                 choice = next((int(r["variant"]) for r in cands if str(r.get("cta_group")) == "1"
                                and float(r["ms_median"]) <= float(best["ms_median"]) * 1.03), choice)
-            if str(best.get("tile_n")) == "192":
-                # within 3 % of the best a tile of 128 or 256 columns is taken: from tens of thousands of rows on the board's power
-                # limit sets the pace, and boxes differ by more than that
-                choice = next((int(r["variant"]) for r in cands if str(r["tile_n"]) != "192"
-                               and float(r["ms_median"]) <= float(best["ms_median"]) * 1.03), choice)
-            if op == OPS["pe"] and str(best.get("tile_n")) == "256" and str(best.get("epi_warps")) == "4":
-                # a burst ranks four epilogue warps up to 2 % ahead of eight, sustained they are 1.4 % behind (186 624 x 1 152 x 588 with
-                # the unfold ahead of it 261.1 against 257.6 us)
-                choice = next((int(r["variant"]) for r in cands if str(r.get("epi_warps")) == "8" and str(r.get("tile_n")) == "256"
-                               and float(r["ms_median"]) <= float(best["ms_median"]) * 1.02), choice)
-            if prev is not None and prev != choice and not (str(best.get("tile_n")) == "192" and prev == int(best["variant"])):
-                mine = [r for r in cands if int(r["variant"]) == prev]
-                if mine and float(mine[0]["ms_median"]) <= float(best["ms_median"]) * (1.0 + keep_margin):
+            if prev is not None and prev != choice:
+                mine = next((r for r in cands if int(r["variant"]) == prev), None)
+                if mine is not None and not beats(best, mine, keep_margin):
                     choice = prev
             if choice != prev:
                 table.append({"op": op, "N": n, "K": k, "m_min": 0 if i == 0 else m, "variant": choice})
@@ -159,14 +157,25 @@ def capture(go, iters: int, stream):
     return graph
 
 
-def replay_ms(graph, iters: int) -> float:
+def replay_ms(graph, iters: int, lead: int = 0, count: int = 1) -> float:
+    """Milliseconds per launch over `count` replays of a graph of `iters` launches, `lead` untimed ones directly ahead of them."""
     import torch
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    for _ in range(lead):
+        graph.replay()
     e0.record()
-    graph.replay()
+    for _ in range(count):
+        graph.replay()
     e1.record()
     torch.cuda.synchronize()
-    return e0.elapsed_time(e1) / iters
+    return e0.elapsed_time(e1) / (iters * count)
+
+
+# From this many rows on the board's power limit sets the pace, and a sample is 100 ms of a variant's own launches behind 100 ms of the
+# same: bursts of ten launches, paced by what ran ahead of them, differ by 1 - 9 % from one another and 25 ms by 1 - 6 %, 100 ms by 0.2 -
+# 0.7 % (FC2 1 152 x 4 304 at 46 656 and 373 248 rows, patch embedding 1 152 x 588 at 186 624, FC1 4 304 x 1 152 at 46 656, twenty samples each).
+SUSTAINED_FROM = 10_000
+SUSTAINED_MS = 100.0
 
 
 def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out_path: Path, variants_only=None,
@@ -228,11 +237,13 @@ def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out
                     # power-bound under these kernels and whoever runs last on a warm GPU would look slower.
                     cands = [v for v in prune(all_variants, op, resources)
                              if variants_only is None or v["variant_id"] in variants_only]
+                    sustained = m >= SUSTAINED_FROM
+                    order = random.Random(m)
                     samples = {v["variant_id"]: [] for v in cands}
                     status = {v["variant_id"]: "ok" for v in cands}
-                    graphs = {}
-                    for rnd in range(repeats + 1):               # round 0 captures and warms up and is not recorded
-                        for v in cands:
+                    graphs, count = {}, {}
+                    for rnd in range(repeats + 1):                 # round 0 captures and warms up and is not recorded
+                        for v in order.sample(cands, len(cands)):
                             vid = v["variant_id"]
                             if status[vid] != "ok":
                                 continue
@@ -240,10 +251,12 @@ def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out
                                 if rnd == 0:
                                     eng.set_variant(vid)
                                     graphs[vid] = capture(go, iters, stream)
-                                ms = replay_ms(graphs[vid], iters)
+                                ms = replay_ms(graphs[vid], iters, *((count[vid], count[vid]) if rnd and sustained else ()))
                                 eng.device_status()
                                 if rnd:
                                     samples[vid].append(ms)
+                                else:
+                                    count[vid] = math.ceil(SUSTAINED_MS / (ms * iters))
                             except SL8Error as e:        # a bounded device wait ran out, or the variant refused the shape
                                 status[vid] = "timeout" if "TIMEOUT" in str(e).upper() else "error"
                     del graphs

@@ -53,6 +53,20 @@ def test_best_rows_keeps_the_previous_winner_inside_the_margin_and_merges_neighb
                      {"op": 2, "N": 1152, "K": 4304, "m_min": 0, "variant": 1}]
 
 
+def test_a_row_that_changes_the_variant_has_a_margin_above_the_spread():
+    """In the committed sweep, where one row of the table follows another: the variant it brings is faster than the one before it by
+    more than the two deviations that were recorded there."""
+    times = {(int(r["op"]), int(r["N"]), int(r["K"]), int(r["M"]), int(r["variant"])): (float(r["ms_median"]), float(r["ms_stdev"]))
+             for r in sweep.read_csv(sweep.PKG / "sweeps" / "b200.csv") if r["status"] == "ok"}
+    table = sweep.best_rows(sweep.read_csv(sweep.PKG / "sweeps" / "b200.csv"))
+    changes = [(a, b) for a, b in zip(table, table[1:]) if (a["op"], a["N"], a["K"]) == (b["op"], b["N"], b["K"])]
+    assert len(changes) > 10
+    for a, b in changes:
+        at = (b["op"], b["N"], b["K"], b["m_min"])
+        (before, s0), (after, s1) = times[(*at, a["variant"])], times[(*at, b["variant"])]
+        assert before - after > s0 + s1 and before > 1.02 * after, (a, b)
+
+
 def test_emit_header_writes_one_initialiser_per_row(tmp_path):
     table = [{"op": 1, "N": 4304, "K": 1152, "m_min": 0, "variant": 6}, {"op": 0, "N": 1152, "K": 588, "m_min": 2916, "variant": 5}]
     text = sweep.emit_header(table, "x.csv", tmp_path / "t.h")
