@@ -61,20 +61,21 @@ int kernel_slot(int op, int out_dtype) {
     return out_dtype == SL8_OUT_E4M3 ? sl8::K_FC1_E4M3 : sl8::K_FC1_BF16;
 }
 
-// What a launch takes with a variant, in microseconds: its CTAs (or pairs) go through ceil(tiles / CTAs) rounds of tiles;
+// What ranks the variants of a launch: its CTAs (or pairs) go through ceil(tiles / CTAs) rounds of tiles;
 //     start + k_blocks * first + (rounds - 1) * max(k_blocks * next, tile)
-// `start` is set-up, the first operands' way in and the last tile's epilogue; `first` a k-block of the first tile; a later tile
+// `start` stands for set-up, the first operands' way in and the last tile's epilogue; `first` for a k-block of the first tile; a later tile
 // hides its mainloop (`next` per k-block, more than `first` when every SM asks L2) behind the epilogue ahead of it or the
 // other way round (`tile`: the epilogue's own pace).  The constants (sl8_cost_model.h) are fitted so that the cheapest variant by
-// the formula is the fastest one measured, from 512 to 4 800 wide and 50 to 186 624 rows: on that sweep (488 points that the table
-// leaves to it, sweeps/b200_model.csv) it is 0.1 - 0.9 % off the fastest on average, by class, and 14 % at worst (no activation);
-// at eighteen other widths with sixteen row counts each 0.5 - 1.0 % and 12 %.  What it decides: tiles of 128 x 64 on single CTAs (20)
+// the formula is the fastest one measured, and to nothing else: a cost is 0.4 - 3 times the microseconds of the launch.  From 16 to
+// 4 800 wide and 50 to 186 624 rows (sweeps/b200_model.csv, 1 276 points that the table leaves to it) the pick is 0.4 - 1.0 % off the
+// fastest on average, by class; at worst 12 % from 512 columns on (no activation) and 32 % below (patch embedding 144 wide, where a last,
+// narrower tile costs less than the formula says).  What it decides, measured there: tiles of 128 x 64 on single CTAs (20)
 // while there are too few of 128 x 128 to fill the chip, or their ring of four stages would wait for L2 (FC2 1 152 x 1 152 at 729 rows
-// 5.2 us with 18, 4.6 with 20); then 128 x 128 with eight epilogue warps (18); pairs
-// with 256 x 128 (19) and 256 x 192 (21) where 256 x 256 tiles leave most of the last round empty (FC2 1 152 x 4 304 at 5 003 rows 27.0 with 1,
-// 23.7 with 21; 1 152 x 1 152 13.1 with 1, 11.8 with 19, 11.4 with 21); eight epilogue warps
-// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 52.0 with 1,
-// 38.6 with 17); a fifth stage (2) where K is deep behind a light epilogue (hardware tanh, 1 152 x 4 304 at 46 656 rows 197.7 with 3, 180.8 with 2).
+// 5.1 us with 18, 4.5 with 20; 384 x 1 536 5.6, 4.9; GELU 144 x 1 616 at 5 003 rows 7.0, 5.7); then 128 x 128 with eight epilogue warps (18); pairs
+// with 256 x 128 (19) and 256 x 192 (21) where 256 x 256 tiles leave most of the last round empty (FC2 1 152 x 1 152 at 5 003 rows 12.1 with 1,
+// 10.4 with 19, 10.8 with 21; 1 600 x 4 800 at 5 832 rows 45.1 with 1, 44.4 with 19, 36.9 with 21); eight epilogue warps
+// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 43.7 with 1,
+// 35.4 with 17); a fifth stage (2) where K is deep behind a light epilogue (no activation, 3 456 x 1 152 at 46 656 rows 155 with 3, 141 with 2).
 enum CostClass : int { COST_GELU, COST_TANH, COST_NONE, COST_FC2, COST_PE };
 struct VariantCost {
     CostClass cls;
@@ -91,21 +92,17 @@ long long clusters_of(sl8_handle_t h, const VariantEntry* v) {
     return h && h->max_clusters_override > 0 && clusters > h->max_clusters_override ? h->max_clusters_override : clusters;
 }
 
-// Tiles of 64 and 192 columns are candidates from this width on.  The sweep's narrowest layer has 512 columns, and 432 were tried
-// beside it; below, where a last column of tiles is most of a layer, the choice is left to the variants it was made for.
-constexpr int kNewTilesFrom = 416;
-
 int cheapest_variant(sl8_handle_t h, CostClass cls, int slot, long long M, int N, int K) {
     int best = 1;
-    float best_us = 3.4e38f;
+    float best_cost = 3.4e38f;
     for (const VariantCost& c : kVariantCost) {
         const VariantEntry* v = c.cls == cls ? variant(c.variant) : nullptr;
-        if (!v || !v->kernel[slot] || (N < kNewTilesFrom && (v->tn == 64 || v->tn == 192))) continue;
+        if (!v || !v->kernel[slot]) continue;
         const long long tiles = ((M + 128 * v->cg - 1) / (128 * v->cg)) * ((N + v->tn - 1) / v->tn), clusters = clusters_of(h, v);
         const float rounds = static_cast<float>((tiles + clusters - 1) / clusters), k_blocks = static_cast<float>((K + 127) / 128);
         const float later = k_blocks * c.next > c.tile ? k_blocks * c.next : c.tile;
-        const float us = c.start + k_blocks * c.first + (rounds - 1.0f) * later;
-        if (us < best_us) best_us = us, best = c.variant;
+        const float cost = c.start + k_blocks * c.first + (rounds - 1.0f) * later;
+        if (cost < best_cost) best_cost = cost, best = c.variant;
     }
     return best;
 }

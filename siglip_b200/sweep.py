@@ -291,13 +291,14 @@ def run_sweep(shape_sets: list[str], m_steps: int, repeats: int, iters: int, out
 
 
 # ----------------------------------------------------------------------------- the cost model of pick_variant
-# (class, N, K): the widths of the two encoders and two of no model's, per kind of epilogue the model knows.
+# (class, N, K): the widths of the two encoders and of no model's, down to a single narrow tile, per kind of epilogue the model knows.
+NARROW = [(400, 592), (320, 1280), (256, 4176), (144, 1616), (64, 592), (16, 80)]
 MODEL_SHAPES = {
-    "GELU": [(4304, 1152), (3072, 768), (1600, 512), (4800, 1600), (1152, 4304), (1600, 4800)],
-    "TANH": [(4304, 1152), (3072, 768), (1152, 4304), (1600, 4800)],
-    "NONE": [(3456, 1152), (2304, 768), (4800, 1600), (1536, 512), (1152, 4304), (1600, 4800)],
-    "FC2": [(1152, 4304), (768, 3072), (1152, 1152), (768, 768), (1600, 4800), (512, 1600)],
-    "PE": [(1152, 588), (768, 768)],
+    "GELU": [(4304, 1152), (3072, 768), (1600, 512), (4800, 1600), (1152, 4304), (1600, 4800)] + NARROW,
+    "TANH": [(4304, 1152), (3072, 768), (1152, 4304), (1600, 4800)] + NARROW,
+    "NONE": [(3456, 1152), (2304, 768), (4800, 1600), (1536, 512), (1152, 4304), (1600, 4800)] + NARROW,
+    "FC2": [(1152, 4304), (768, 3072), (1152, 1152), (768, 768), (1600, 4800), (512, 1600), (384, 1536), (272, 2128)] + NARROW,
+    "PE": [(1152, 588), (768, 768), (1600, 768), (640, 588), (384, 768), (272, 588)] + [(n, k) for n, k in NARROW if k < 2048],
 }
 MODEL_ROWS = [50, 128, 196, 256, 392, 512, 729, 1000, 1458, 1568, 2048, 2916, 3700, 4374, 5003, 5832, 7000, 8748, 11664, 14580, 17496,
               23328, 32000, 46656, 93312, 186624]
@@ -330,9 +331,6 @@ def emit_model(constants: dict, source: str, path: Path = MODEL_HEADER) -> None:
     path.write_text("\n".join(lines) + "\n")
 
 
-NEW_TILES_FROM = 416          # columns from which tiles of 64 and 192 columns are candidates (cheapest_variant)
-
-
 def model_us(k: tuple, cg: int, tn: int, M: int, N: int, K: int, sms: int = 148) -> float:
     """The formula beside kVariantCost."""
     tiles, k_blocks = -(-M // (128 * cg)) * -(-N // tn), -(-K // 128)
@@ -340,29 +338,11 @@ def model_us(k: tuple, cg: int, tn: int, M: int, N: int, K: int, sms: int = 148)
     return k[0] + k_blocks * k[1] + (rounds - 1) * max(k_blocks * k[2], k[3])
 
 
-# Picks that a fit leaves as they are, {class: [((M, N, K), CTAs or pairs a launch may use, variant)]}: tests/test_gpu_dispatch.py and
-# tests/test_gpu_tooling.py state them, most of them at sizes that the sweep does not reach (a few columns, a k-block or two).
-KEPT = {
-    "GELU": [((1, 16, 16), 0, 18), ((769, 400, 592), 0, 18), ((9473, 144, 80), 0, 14), ((5121, 1296, 592), 0, 14), ((9473, 144, 2128), 0, 15),
-             ((50000, 2048, 1024), 0, 15), ((4096, 512, 1600), 0, 18), ((4096, 512, 1600), 8, 15)],
-    "TANH": [((127, 144, 80), 0, 18), ((9473, 144, 1616), 0, 3), ((9473, 144, 80), 0, 15), ((20001, 528, 2128), 0, 2)],
-    "NONE": [((129, 400, 592), 0, 18), ((9473, 144, 592), 0, 3), ((9473, 1040, 1104), 0, 2), ((20001, 272, 4176), 0, 1)],
-    "FC2": [((1, 16, 16), 0, 18), ((2369, 528, 592), 0, 18), ((20001, 16, 1616), 0, 19), ((9473, 144, 80), 0, 3), ((9473, 656, 80), 0, 17),
-            ((16001, 656, 1616), 0, 1), ((2048, 768, 768), 0, 18), ((2048, 768, 768), 8, 17)],
-    "PE": [((127, 144, 80), 0, 18), ((9473, 144, 80), 0, 17)],
-}
-
-
-def kept_picks_hold(cls: str, constants: dict, variants: dict) -> bool:
-    for (m, n, k), clusters, variant in KEPT.get(cls, ()):
-        cost = {}
-        for (c, v), x in constants.items():
-            cg, tn = variants[v]
-            if c == cls and (tn in (128, 256) or n >= NEW_TILES_FROM):
-                cost[v] = model_us(x, cg, tn, m, n, k, sms=min(148 // cg, clusters or 148) * cg)
-        if min(cost, key=cost.get) != variant or sorted(cost.values())[1] - cost[variant] < 1e-4:
-            return False
-    return True
+def cheapest(cls: str, M: int, N: int, K: int, clusters: int | None = None) -> int:
+    """The variant that the committed constants pick, on a handle held to `clusters` CTAs or pairs or on the whole chip."""
+    tiles = variant_tiles()
+    us = lambda v, k: model_us(k, *tiles[v], M, N, K, sms=min(148 // tiles[v][0], clusters or 148) * tiles[v][0])
+    return min((us(v, k), v) for (c, v), k in cost_constants().items() if c == cls)[1]
 
 
 def asked_rows(rows: list[dict]) -> list[dict]:
@@ -384,12 +364,12 @@ def model_regret(rows: list[dict], constants: dict, variants: dict) -> dict:
     return out
 
 
-def fit_model(rows: list[dict], constants: dict, variants: dict, steps=(0.98, 1.02, 0.95, 1.05, 0.9, 1.1)) -> dict:
+def fit_model(rows: list[dict], constants: dict, variants: dict, steps=(0.98, 1.02, 0.95, 1.05, 0.9, 1.1), least: float = 5e-4) -> dict:
     """`constants` with every number moved in small steps, one after the other and as long as it helps, to where the variant
-    picked is slower than the fastest by less: on average, plus a tenth of the worst case.  Its own result it leaves as it is,
-    and no step goes where a pick of KEPT would change."""
+    picked is slower than the fastest by less: on average, plus a tenth of the worst case.  A step has to gain `least` of that
+    (smaller ones follow the noise of one sweep: picks that they change are 3 % slower as often as faster).  Its own result it leaves
+    as it is."""
     out = dict(constants)
-    holds = {c for c in KEPT if {v for _, _, v in KEPT[c]} <= {v for x, v in constants if x == c} and kept_picks_hold(c, constants, variants)}
     for cls in sorted({c for c, _ in constants}):
         mine = [v for c, v in constants if c == cls]
         points = [(int(r["M"]), int(r["N"]), int(r["K"]), {int(f[1:]): float(t) for f, t in r.items() if f[0] == "v" and t}) for r in rows if r["cls"] == cls]
@@ -412,7 +392,7 @@ def fit_model(rows: list[dict], constants: dict, variants: dict, steps=(0.98, 1.
                         out[cls, v] = old[:j] + (float(f"{old[j] * f:.3g}"),) + old[j + 1:]
                         cost[v] = [model_us(out[cls, v], *variants[v], m, n, k) for m, n, k, _ in points]
                         now = score(lost())
-                        if now < best - 1e-5 and (cls not in holds or kept_picks_hold(cls, out, variants)):
+                        if now < best - least:
                             best, moved = now, True
                         else:
                             out[cls, v], cost[v] = old, kept
@@ -487,7 +467,7 @@ def main(argv=None) -> int:
     ap.add_argument("--variants", default="", help="restrict to these variant ids")
     ap.add_argument("--emit-table", type=Path, default=None, metavar="CSV",
                     help="no GPU work: turn this CSV into csrc/sl8_dispatch_table.h")
-    ap.add_argument("--model-sweep", action="store_true", help="time the points of the cost model (25 s of B200 time) into " + MODEL_CSV.name)
+    ap.add_argument("--model-sweep", action="store_true", help="time the points of the cost model into " + MODEL_CSV.name)
     ap.add_argument("--fit-model", type=Path, default=None, metavar="CSV",
                     help="no GPU work: move the constants of csrc/sl8_cost_model.h to where they pick best on this CSV")
     a = ap.parse_args(argv)

@@ -4,19 +4,25 @@ import pytest
 import torch
 
 import siglip_b200
-from siglip_b200 import lib as L, synth
+from siglip_b200 import lib as L, sweep, synth
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 GENERAL = 6       # 128 x 128 tiles on single CTAs: serves every layer and output type
 
-# (kind of call, the variant its cost picks, shapes): every row of the cost model, at row counts and widths that end in the
-# middle of a tile and K that ends in the middle of a block.
-CASES = [("gelu", 18, (1, 16, 16), (769, 400, 592)), ("gelu", 14, (9473, 144, 80), (5121, 1296, 592)), ("gelu", 15, (9473, 144, 2128)),
-         ("tanh", 18, (127, 144, 80)), ("tanh", 3, (9473, 144, 1616)), ("tanh", 15, (9473, 144, 80)), ("tanh", 2, (20001, 528, 2128)),
-         ("none", 18, (129, 400, 592)), ("none", 3, (9473, 144, 592)), ("none", 2, (9473, 1040, 1104)), ("none", 1, (20001, 272, 4176)),
-         ("fc2", 18, (1, 16, 16), (2369, 528, 592)), ("fc2", 19, (20001, 16, 1616)), ("fc2", 3, (9473, 144, 80)), ("fc2", 17, (9473, 656, 80)),
-         ("fc2", 1, (16001, 656, 1616)), ("pe", 18, (127, 144, 80)), ("pe", 17, (9473, 144, 80))]
+# Row counts and widths that end in the middle of a tile and K that ends in the middle of a block, from one row of one narrow tile up:
+# between them they reach every row of the cost model (tests/test_tooling.py).
+SHAPES = {
+    "gelu": [(1, 16, 16), (769, 400, 592), (9473, 144, 80), (5121, 1296, 592), (9473, 144, 2128), (769, 2320, 592), (300, 2064, 1616), (129, 416, 16),
+             (5003, 528, 1104), (5003, 528, 4176), (9001, 784, 4176)],
+    "tanh": [(127, 144, 80), (9473, 144, 1616), (9473, 144, 80), (20001, 528, 2128), (1300, 2320, 4176), (700, 656, 592), (129, 416, 272),
+             (5003, 784, 4176), (4000, 1600, 4176)],
+    "none": [(129, 400, 592), (9473, 144, 592), (9473, 1040, 1104), (20001, 272, 4176), (769, 2320, 3072), (3001, 2320, 16), (16001, 2320, 1616),
+             (700, 528, 1104), (129, 416, 16), (4000, 784, 1104), (5003, 1296, 4176)],
+    "fc2": [(1, 16, 16), (2369, 528, 592), (20001, 16, 1616), (9473, 144, 80), (9473, 656, 80), (16001, 656, 1616), (5121, 784, 3072), (1300, 2064, 16),
+            (700, 528, 16), (129, 416, 16), (5003, 1296, 4176)],
+    "pe": [(127, 144, 80), (9473, 144, 80), (769, 1552, 4176), (3001, 2320, 16), (700, 784, 2128), (129, 416, 16), (7001, 1040, 2128)],
+}
 
 
 def _codes(g, rows, cols):
@@ -24,9 +30,10 @@ def _codes(g, rows, cols):
     return full[:, :cols]
 
 
-@pytest.mark.parametrize("kind,variant,shape", [(kind, v, s) for kind, v, *shapes in CASES for s in shapes])
-def test_the_picked_variant_agrees_with_the_general_one(engine, kind, variant, shape):
+@pytest.mark.parametrize("kind,shape", [(kind, s) for kind, shapes in SHAPES.items() for s in shapes])
+def test_the_picked_variant_agrees_with_the_general_one(engine, kind, shape):
     M, N, K = shape
+    variant = sweep.cheapest(kind.upper(), M, N, K)
     g = torch.Generator(device=DEV).manual_seed(M + N + K)
     A, B = _codes(g, M, K), _codes(g, N, K)
     bias = torch.randn(N, generator=g, device=DEV).to(torch.bfloat16)
@@ -56,7 +63,9 @@ def test_the_picked_variant_agrees_with_the_general_one(engine, kind, variant, s
 
 def test_the_pick_follows_the_ctas_a_launch_may_use(engine, monkeypatch):
     """A handle held to eight CTAs (or pairs) has many rounds of tiles where the whole chip has less than one."""
-    for op, M, N, K, whole, held in ((2, 2048, 768, 768, 18, 17), (1, 4096, 512, 1600, 18, 15)):
+    for cls, op, M, N, K in (("FC2", 2, 2048, 768, 768), ("GELU", 1, 4096, 512, 1600)):
+        whole, held = sweep.cheapest(cls, M, N, K), sweep.cheapest(cls, M, N, K, clusters=8)
+        assert whole != held
         assert engine.query_config(op, M, N, K)["variant_id"] == whole
         monkeypatch.setenv("SL8_MAX_CLUSTERS", "8")
         with siglip_b200.Engine(0) as few:

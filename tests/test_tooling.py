@@ -92,14 +92,21 @@ def test_the_committed_table_is_what_its_sweep_produces():
 def test_the_committed_cost_model_is_what_its_sweep_produces(tmp_path):
     """csrc/sl8_cost_model.h is fitted: the fit leaves it as it is, and it picks as well as the comment beside it says."""
     points, constants, variants = sweep.read_csv(sweep.MODEL_CSV), sweep.cost_constants(), sweep.variant_tiles()
-    assert len({(r["cls"], r["N"], r["K"]) for r in points}) == sum(map(len, sweep.MODEL_SHAPES.values())) == 24
+    assert len({(r["cls"], r["N"], r["K"]) for r in points}) == sum(map(len, sweep.MODEL_SHAPES.values())) == 59
     rows = sweep.asked_rows(points)
     assert 300 < len(rows) < len(points)
     assert sweep.fit_model(rows, constants, variants) == constants
     sweep.emit_model(constants, "siglip_b200/sweeps/b200_model.csv", tmp_path / "m.h")
     assert (tmp_path / "m.h").read_text() == sweep.MODEL_HEADER.read_text()
-    lost = {cls: [x for x, _ in points] for cls, points in sweep.model_regret(rows, constants, variants).items()}
-    assert max(map(max, lost.values())) < 0.1495 and all(0.0005 < sum(x) / len(x) < 0.0225 for x in lost.values())
+    # (the layers of a few hundred columns that are all epilogue are where it is worst: patch embedding 144 wide, 17 496 rows)
+    for some, worst in (([r for r in rows if int(r["N"]) >= 512], 0.1495), (rows, 0.325)):
+        lost = {cls: [x for x, _ in points] for cls, points in sweep.model_regret(some, constants, variants).items()}
+        assert max(map(max, lost.values())) < worst and all(0.0005 < sum(x) / len(x) < 0.0225 for x in lost.values())
+
+
+def test_every_row_of_the_cost_model_is_picked_somewhere():
+    from tests.test_gpu_dispatch import SHAPES
+    assert {(kind.upper(), sweep.cheapest(kind.upper(), *s)) for kind, shapes in SHAPES.items() for s in shapes} == set(sweep.cost_constants())
 
 
 def test_the_cost_formula_is_the_one_the_library_uses(tmp_path):
@@ -112,8 +119,6 @@ def test_the_cost_formula_is_the_one_the_library_uses(tmp_path):
     constants, variants = sweep.cost_constants(), sweep.variant_tiles()
     kinds = {"GELU": (1, 0), "TANH": (1, L.SL8_FLAG_GELU_HW_TANH), "NONE": (1, L.SL8_FLAG_NO_ACTIVATION), "FC2": (2, 0), "PE": (0, 0)}
     for r in sweep.asked_rows(sweep.read_csv(sweep.MODEL_CSV)):
-        if r["cls"] == "PE":              # (both widths are the table's)
-            continue
         m, n, k = int(r["M"]), int(r["N"]), int(r["K"])
         op, flags = kinds[r["cls"]]
         cost = {v: sweep.model_us(c, *variants[v], m, n, k) for (cls, v), c in constants.items() if cls == r["cls"]}
