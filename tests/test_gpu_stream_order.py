@@ -86,6 +86,40 @@ def test_calls_behind_a_fork_and_a_fill_are_captured_in_order(engine):
         assert torch.equal(out, want)
 
 
+@pytest.mark.parametrize("rows,n,k", [(100, 512, 256), (729, 1152, 4304), (3000, 4304, 1152)])
+def test_weights_written_by_the_kernel_ahead(engine, rows, n, k):
+    """A GEMM asks its first tile's weights into L2 before the kernel ahead has finished.  Where that kernel writes them, the GEMM
+    still reads what it wrote: two weights in turn through one operand buffer, back to back and captured."""
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    a = synth.quantize_e4m3(torch.randn((rows, k), generator=g, device=DEV))[0]
+    weights = [torch.randn((n, k), generator=g, device=DEV).to(torch.bfloat16) for _ in range(2)]
+    scale, res = torch.full((1,), 0.02, device=DEV), torch.randn((rows, n), generator=g, device=DEV).to(torch.bfloat16)
+    b = torch.zeros((n, synth.pitch128(k)), dtype=torch.uint8, device=DEV)[:, :k]
+    outs = [torch.empty((rows, n), dtype=torch.bfloat16, device=DEV) for _ in range(8)]
+
+    def run(step):
+        for i, out in enumerate(outs):
+            engine.quantize_e4m3(weights[i % 2], scale, out=b); step()
+            if i % 4 < 2:
+                engine.fc2_residual(a, b, None, res, scale_b=scale, out=out); step()
+            else:
+                engine.fc1_gelu(a, b, None, scale_b=scale, out=out); step()
+
+    run(torch.cuda.synchronize)
+    want = [out.clone() for out in outs]
+    assert not torch.equal(want[0], want[1]) and not torch.equal(want[2], want[3])
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        run(lambda: None)
+    for go in [lambda: run(lambda: None)] * 5 + [graph.replay] * 5:
+        for out in outs:
+            out.zero_()
+        go()
+        torch.cuda.synchronize()
+        assert all(torch.equal(out, w) for out, w in zip(outs, want))
+    engine.device_status()
+
+
 def test_two_threads_on_their_own_streams(engine):
     """Chains of overlapped launches from two threads at once, through one handle: each stream keeps its own order."""
     chains = [_chain(engine, rows, d, ff, seed=rows) for rows, d, ff in ((729, 1152, 4304), (1300, 768, 3072))]
