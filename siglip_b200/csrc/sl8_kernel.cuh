@@ -639,16 +639,15 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const int b_rows = tail ? p.tail_cols / CG : T::B_ROWS;
             const int nb = tn * TN + static_cast<int>(cta_rank) * b_rows;
             // (measurement builds: DBG_SKIP_A / DBG_SKIP_B leave one operand's copies out; the MMAs then read stale shared memory)
-            const uint32_t stage_tx = static_cast<uint32_t>((SL8_DBG(p.flags, DBG_SKIP_A) ? 0 : T::A_BYTES) +
-                                                            (SL8_DBG(p.flags, DBG_SKIP_B) ? 0 : T::KATOMS * b_rows * 128));
-            const bool skip_mine = SL8_DBG(p.flags, DBG_SKIP_LOAD) || (is_a ? SL8_DBG(p.flags, DBG_SKIP_A) : SL8_DBG(p.flags, DBG_SKIP_B));
+            const bool skip_a = SL8_DBG(p.flags, DBG_SKIP_LOAD | DBG_SKIP_A), skip_b = SL8_DBG(p.flags, DBG_SKIP_LOAD | DBG_SKIP_B);
+            const uint32_t stage_tx = static_cast<uint32_t>((skip_a ? 0 : T::A_BYTES) + (skip_b ? 0 : T::KATOMS * b_rows * 128));
             if (is_a) {
                 stream(0, p.k_blocks, [&](int kb, uint32_t a_dst, uint32_t bar) {
                     if (cta_rank == 0) {
-                        if (SL8_DBG(p.flags, DBG_SKIP_LOAD)) mbar_arrive(full_bar0 + 8 * stage);   // measurement aid: MMAs run on whatever shared memory holds
+                        if (skip_a && skip_b) mbar_arrive(full_bar0 + 8 * stage);   // measurement aid: MMAs run on whatever shared memory holds
                         else mbar_arrive_expect_tx(full_bar0 + 8 * stage, CG * stage_tx);
                     }
-                    if (skip_mine) return;
+                    if (skip_a) return;
                     if constexpr (T::SPLIT_A) {
 #pragma unroll
                         for (int r = 0; r < 3; r++) load(a_dst + r * 32 * 128, &map_a, kb * T::TILE_K, m0 + 32 * r, bar);
@@ -660,8 +659,10 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             } else {
                 const auto b_loop = [&](int kb0, int end, const CUtensorMap* map) {
                     stream(kb0, end, [&](int kb, uint32_t a_dst, uint32_t bar) {
-                        if (skip_mine) return;
-                        if constexpr (T::SPLIT_A) load(a_dst + 96 * 128, &map_a, kb * T::TILE_K, m0 + 96, bar);
+                        if constexpr (T::SPLIT_A) {
+                            if (!skip_a) load(a_dst + 96 * 128, &map_a, kb * T::TILE_K, m0 + 96, bar);
+                        }
+                        if (skip_b) return;
 #pragma unroll
                         for (int a = 0; a < T::KATOMS; a++) load(a_dst + T::A_BYTES + a * T::B_ATOM_BYTES, map, kb * T::TILE_K + 128 * a, nb, bar);
                     });
