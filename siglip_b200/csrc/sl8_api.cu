@@ -269,7 +269,7 @@ int run(sl8_handle_t h, const Problem& q, cudaStream_t stream) {
 
     CUtensorMap map_a, map_b, map_bt, map_d;
     rc = encode_2d(h, &map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.A, (unsigned long long)q.K, (unsigned long long)q.M,
-                   (unsigned long long)q.lda, 128, v->tn / v->cg == 64 ? 32 : 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);      // (SPLIT_A)
+                   (unsigned long long)q.lda, 128, (unsigned)v->a_box_rows, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     if (rc != SL8_OK) return rc;
     rc = encode_2d(h, &map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q.B, (unsigned long long)q.K, (unsigned long long)q.N,
                    (unsigned long long)q.ldb, 128, (unsigned)(v->tn / v->cg), CU_TENSOR_MAP_L2_PROMOTION_L2_256B);

@@ -145,6 +145,7 @@ struct KernelTraits {
     // Where a CTA's share of B has 64 rows, the B producer brings the last 32 of A's 128 as well (boxes of 32 rows): an issuing
     // thread's copies take 2 cycles per row, so 96 + 96 rows take 192 cycles per k-block and 128 + 64 take 256.
     static constexpr bool SPLIT_A = (B_ROWS == 64 && KATOMS == 1);
+    static constexpr int A_BOX_ROWS = SPLIT_A ? 32 : TILE_M_CTA; // rows of one copy of A: the box of map_a (VariantEntry::a_box_rows)
     static constexpr int A_ATOM_BYTES = TILE_M_CTA * 128;        // 16 KiB: 128 rows x 128 bytes
     static constexpr int B_ATOM_BYTES = B_ROWS * 128;
     static constexpr int A_BYTES = KATOMS * A_ATOM_BYTES;
@@ -174,6 +175,7 @@ struct KernelTraits {
     static_assert(COLS_PER_WARP % REGION_COLS == 0, "a warp stores whole staging regions");
     static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KiB a CTA may use");
     // A launch that waits for the one ahead of it (pdl_wait) already holds tensor memory: it must not sit on that one's SMs.
+    static_assert(!SPLIT_A || 96 + A_BOX_ROWS == TILE_M_CTA, "three boxes from one producer, the last one from the other");
     static_assert(2 * SMEM_BYTES > 228 * 1024, "two CTAs must not fit one SM");
 };
 
@@ -650,7 +652,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     if (skip_a) return;
                     if constexpr (T::SPLIT_A) {
 #pragma unroll
-                        for (int r = 0; r < 3; r++) load(a_dst + r * 32 * 128, &map_a, kb * T::TILE_K, m0 + 32 * r, bar);
+                        for (int r = 0; r < 96; r += T::A_BOX_ROWS) load(a_dst + r * 128, &map_a, kb * T::TILE_K, m0 + r, bar);
                     } else {
 #pragma unroll
                         for (int a = 0; a < T::KATOMS; a++) load(a_dst + a * T::A_ATOM_BYTES, &map_a, kb * T::TILE_K + 128 * a, m0, bar);

@@ -164,7 +164,7 @@ SL8_API int sl8_fc1_gelu_fp8_static(const void* A, int64_t lda, const void* B, i
 
     CUtensorMap map_a, map_b, map_bt, map_d;
     if ((rc = encode_2d(s->encode, &map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, A, (unsigned long long)K, (unsigned long long)M,
-                        (unsigned long long)lda, 128, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)) != SL8_OK) return rc;
+                        (unsigned long long)lda, 128, (unsigned)v->a_box_rows, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)) != SL8_OK) return rc;
     if ((rc = encode_2d(s->encode, &map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, B, (unsigned long long)K, (unsigned long long)N,
                         (unsigned long long)ldb, 128, (unsigned)(v->tn / v->cg), CU_TENSOR_MAP_L2_PROMOTION_L2_256B)) != SL8_OK) return rc;
     const int tail_cols = N % v->tn == 0 ? v->tn : N % v->tn;    // the last N tile is as wide as what is left of N

@@ -52,7 +52,7 @@ const VariantEntry* make_entry() {
     constexpr bool E4 = (TN / (EW / 4)) % 64 == 0;   // an e4m3 staging region is 128 or 64 columns wide
     using T8 = std::conditional_t<E4, KernelTraits<CG, TN, TK, STAGES, EW, E4 ? OUT_E4M3 : OUT_BF16, NBUF>, T16>;
     static const VariantEntry e = {
-        ID, CG, TN, TK, STAGES, EW, NBUF, T16::THREADS,
+        ID, CG, TN, TK, STAGES, EW, NBUF, T16::A_BOX_ROWS, T16::THREADS,
         {T16::SMEM_BYTES, T16::SMEM_BYTES, T8::SMEM_BYTES, T16::SMEM_BYTES},
         {Slot<CG, TN, TK, STAGES, EW, OP_PE, OUT_BF16, NBUF, SIDE>::kernel(), Slot<CG, TN, TK, STAGES, EW, OP_FC1, OUT_BF16, NBUF, true>::kernel(),
          Slot<CG, TN, TK, STAGES, EW, OP_FC1, OUT_E4M3, NBUF, E4>::kernel(), Slot<CG, TN, TK, STAGES, EW, OP_FC2, OUT_BF16, NBUF, SIDE>::kernel()},

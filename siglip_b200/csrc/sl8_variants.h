@@ -58,6 +58,7 @@ typedef cudaError_t (*launch_fn)(const CUtensorMap* map_a, const CUtensorMap* ma
 struct VariantEntry {
     int id;
     int cg, tn, tk, stages, epi_warps, nbuf;
+    int a_box_rows;                  // rows of A that one copy brings: the box of map_a
     int threads;
     int smem_bytes[K_COUNT];
     const void* kernel[K_COUNT];     // for cudaFuncSetAttribute / occupancy queries; null = layer not served
