@@ -47,7 +47,7 @@ UNIT = "TFLOP/s"
 
 # DRAM bytes per launch of each layer's kernel at the FULL size of its configuration (dram__bytes_read.sum +
 # dram__bytes_write.sum, one-pass ncu capture of launches 11 - 19 of this bench with the caches left as the previous
-# launch left them: profiles/dram_traffic_full_size.md), per GEMM row so that a changed batch scales it.
+# launch left them: summarised under profiles/), per GEMM row so that a changed batch scales it.
 NCU_DRAM_BYTES_PER_ROW = {"C2": (53.9e6 + 401.2e6) / 46656, "C3": (310.7e6 + 108.0e6) / 46656, "C4": (119.6e6 + 428.5e6) / 186624}
 
 
@@ -831,7 +831,7 @@ def main() -> None:
         per_row = NCU_DRAM_BYTES_PER_ROW.get(args.config)
         line["roofline"] = roofline_of(p, ms, peaks, traffic=None if per_row is None else per_row * p.M)
         line["roofline"]["traffic_note"] = ("DRAM bytes per launch from a one-pass ncu capture of this bench at full size, caches left as the "
-                                            "previous launch left them (profiles/dram_traffic_full_size.md); algorithmic bytes: "
+                                            "previous launch left them; algorithmic bytes: "
                                             f"{p.min_bytes():.0f}")
         line["roofline"]["power_note"] = ("the board sits at its 1 kW power cap under these kernels (sw_power_cap): the SM clock, not "
                                           "the tensor pipe or HBM, sets the rate; see `sustained`")

@@ -25,7 +25,7 @@
 //                 values of a 32-row x 128-byte region are brought into that same staging buffer
 //                 by a TMA load a few regions ahead, added in place and stored from there.
 //
-//   last warp     side-data loader (patch-embed, FC2): one lane issues the TMA loads that bring the table /
+//   warp 2 + EPI  side-data loader (patch-embed, FC2): one lane issues the TMA loads that bring the table /
 //                 residual regions into the epilogue warps' staging buffers as those become free, so
 //                 the epilogue warps never wait for a TMA instruction to be accepted.
 //
@@ -180,7 +180,7 @@ struct KernelTraits {
 };
 
 // The tiles of one cluster: cluster, cluster + clusters, ... in N-fastest order.  No division: the first tile's number is
-// small enough for a multiplication (exact while cluster * tiles_n < 2^32; N is below 2^31 / 128 tiles), later ones are steps.
+// small enough for a multiplication (exact for any tiles_n while there are no more than 2^16 clusters), later ones are steps.
 struct TileWalk {
     int tile, tm, tn;
     __device__ __forceinline__ TileWalk(const KernelParams& p, int cluster)
@@ -938,7 +938,7 @@ sl8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 const uint32_t region = my_staging + (seq % NBUF) * 4 * T::REGION_BYTES;
                 if (prof) t0 = clock64();
                 if constexpr (HAS_SIDE) {
-                    // this region's side values have landed: one lane polls, the others confirm
+                    // this region's side values have landed
                     const uint32_t sbar = my_side_bar + 8 * (seq % NBUF);
                     const uint32_t spar = (seq / NBUF) & 1u;
                     ok = wait_bar(sbar, spar, wc, ST_EPI_SIDE_WAIT, seq % NBUF);
