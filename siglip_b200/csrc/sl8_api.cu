@@ -67,15 +67,15 @@ int kernel_slot(int op, int out_dtype) {
 // hides its mainloop (`next` per k-block, more than `first` when every SM asks L2) behind the epilogue ahead of it or the
 // other way round (`tile`: the epilogue's own pace).  The constants (sl8_cost_model.h) are fitted so that the cheapest variant by
 // the formula is the fastest one measured, and to nothing else: a cost is 0.4 - 3 times the microseconds of the launch.  From 16 to
-// 4 800 wide and 50 to 186 624 rows (sweeps/b200_model.csv, 1 276 points that the table leaves to it) the pick is 0.4 - 1.0 % off the
-// fastest on average, by class; at worst 12 % from 512 columns on (no activation) and 32 % below (patch embedding 144 wide, where a last,
+// 4 800 wide and 50 to 186 624 rows (sweeps/b200_model.csv, 2 018 points that the table leaves to it) the pick is 0.4 - 1.1 % off the
+// fastest on average, by class; at worst 11 % from 512 columns on (no activation) and 30 % below (patch embedding 144 wide, where a last,
 // narrower tile costs less than the formula says).  What it decides, measured there: tiles of 128 x 64 on single CTAs (20)
 // while there are too few of 128 x 128 to fill the chip, or their ring of four stages would wait for L2 (FC2 1 152 x 1 152 at 729 rows
-// 5.1 us with 18, 4.5 with 20; 384 x 1 536 5.6, 4.9; GELU 144 x 1 616 at 5 003 rows 7.0, 5.7); then 128 x 128 with eight epilogue warps (18); pairs
-// with 256 x 128 (19) and 256 x 192 (21) where 256 x 256 tiles leave most of the last round empty (FC2 1 152 x 1 152 at 5 003 rows 12.1 with 1,
-// 10.4 with 19, 10.8 with 21; 1 600 x 4 800 at 5 832 rows 45.1 with 1, 44.4 with 19, 36.9 with 21); eight epilogue warps
-// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 43.7 with 1,
-// 35.4 with 17); a fifth stage (2) where K is deep behind a light epilogue (no activation, 3 456 x 1 152 at 46 656 rows 155 with 3, 141 with 2).
+// 5.3 us with 18, 4.7 with 20; 384 x 1 536 5.8, 4.9; GELU 144 x 1 616 at 5 003 rows 7.0, 5.6); then 128 x 128 with eight epilogue warps (18); pairs
+// with 256 x 128 (19) and 256 x 192 (21) where 256 x 256 tiles leave most of the last round empty (FC2 1 152 x 1 152 at 5 003 rows 12.2 with 1,
+// 10.4 with 19, 10.7 with 21; 1 600 x 4 800 at 5 832 rows 42.4 with 1, 42.7 with 19, 36.8 with 21); eight epilogue warps
+// with two or three staging boxes (3, 17) where K is short and the epilogue sets the pace (FC2 768 x 768 at 46 656 rows 43.4 with 1,
+// 35.9 with 17); a fifth stage (2) where K is deep behind a light epilogue (no activation, 3 456 x 1 152 at 46 656 rows 165 with 3, 144 with 2).
 enum CostClass : int { COST_GELU, COST_TANH, COST_NONE, COST_FC2, COST_PE };
 struct VariantCost {
     CostClass cls;

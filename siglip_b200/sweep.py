@@ -4,7 +4,7 @@ Counterpart of the reference's ``tools/grid_search.py`` (constraint pruning ``:8
 parsing ``:124-151``, per-configuration timeout, CSV ``:170-251``) for the run-time variants of this library:
 instead of recompiling one binary per macro combination it walks the compiled variant list
 (``siglip_b200/csrc/sl8_variants.h``) through ``sl8_set_variant``, times every admissible variant on the
-seeded synthetic operands of ``siglip_b200/synth.py`` over an M ladder (four points per octave up to 16 images: a few
+seeded synthetic operands of ``siglip_b200/synth.py`` over an M ladder (eight points per octave up to 16 images: a few
 rows more can cost a whole round of tiles) from captured graphs (a Python loop takes longer than a small layer), writes one CSV row per
 (layer, shape, variant) and turns the CSV into the table ``pick_variant`` (``sl8_api.cu``) consults:
 ``siglip_b200/csrc/sl8_dispatch_table.h``.
@@ -140,8 +140,14 @@ def read_csv(path: Path) -> list[dict]:
 
 # ----------------------------------------------------------------------------- timing (GPU)
 def ladder(per_image: int, octaves: int, per_octave: int) -> list[int]:
-    """per_image * 2^j; below 16 images, where the last round of tiles weighs, also the points that divide an octave into per_octave."""
-    return [(per_image << j) + (per_image << j) * q // per_octave for j in range(octaves) for q in range(per_octave if j < min(4, octaves - 1) else 1)]
+    """per_image * 2^j; where the last round of tiles weighs, also the points that divide an octave: into per_octave below 16 images,
+    into half as many up to 46 656 rows."""
+    points = []
+    for j in range(octaves):
+        m = per_image << j
+        parts = 1 if j == octaves - 1 else per_octave if j < 4 else max(1, per_octave // 2) if m < 46656 else 1
+        points += [m + m * q // parts for q in range(parts)]
+    return points
 
 
 def capture(go, iters: int, stream):
@@ -300,8 +306,8 @@ MODEL_SHAPES = {
     "FC2": [(1152, 4304), (768, 3072), (1152, 1152), (768, 768), (1600, 4800), (512, 1600), (384, 1536), (272, 2128)] + NARROW,
     "PE": [(1152, 588), (768, 768), (1600, 768), (640, 588), (384, 768), (272, 588)] + [(n, k) for n, k in NARROW if k < 2048],
 }
-MODEL_ROWS = [50, 128, 196, 256, 392, 512, 729, 1000, 1458, 1568, 2048, 2916, 3700, 4374, 5003, 5832, 7000, 8748, 11664, 14580, 17496,
-              23328, 32000, 46656, 93312, 186624]
+MODEL_ROWS = [50, 128, 196, 256, 392, 512, 729, 1000, 1200, 1458, 1568, 1800, 2048, 2400, 2916, 3300, 3700, 4374, 5003, 5400, 5832, 6400, 7000,
+              7800, 8748, 9500, 10300, 11664, 13000, 14580, 16000, 17496, 20000, 23328, 27000, 32000, 39000, 46656, 93312, 186624]
 MODEL_CSV = PKG / "sweeps" / "b200_model.csv"
 MODEL_HEADER = PKG / "csrc" / "sl8_cost_model.h"
 
@@ -364,11 +370,11 @@ def model_regret(rows: list[dict], constants: dict, variants: dict) -> dict:
     return out
 
 
-def fit_model(rows: list[dict], constants: dict, variants: dict, steps=(0.98, 1.02, 0.95, 1.05, 0.9, 1.1), least: float = 5e-4) -> dict:
+def fit_model(rows: list[dict], constants: dict, variants: dict, steps=(0.98, 1.02, 0.95, 1.05, 0.9, 1.1), least: float = 2e-4) -> dict:
     """`constants` with every number moved in small steps, one after the other and as long as it helps, to where the variant
-    picked is slower than the fastest by less: on average, plus a tenth of the worst case.  A step has to gain `least` of that
-    (smaller ones follow the noise of one sweep: picks that they change are 3 % slower as often as faster).  Its own result it leaves
-    as it is."""
+    picked is slower than the fastest by less: on average plus a tenth of the worst case, from 512 columns on and below added up (the
+    worst cases are narrow, and would hide the others').  A step has to gain `least`: smaller ones follow the noise of one sweep.  Its own
+    result it leaves as it is."""
     out = dict(constants)
     for cls in sorted({c for c, _ in constants}):
         mine = [v for c, v in constants if c == cls]
@@ -379,8 +385,10 @@ def fit_model(rows: list[dict], constants: dict, variants: dict, steps=(0.98, 1.
         def lost():
             return [t[min((cost[v][i], v) for v in t)[1]] for i, (_, _, _, t) in enumerate(points)]
 
+        halves = [h for h in ([i for i, p in enumerate(points) if p[1] >= 512], [i for i, p in enumerate(points) if p[1] < 512]) if h]
+
         def score(now):
-            return statistics.fmean(now) + 0.1 * max(now)
+            return sum(statistics.fmean(now[i] for i in h) + 0.1 * max(now[i] for i in h) for h in halves)
 
         best, moved = score(lost()), True
         while moved:
@@ -459,7 +467,7 @@ def main(argv=None) -> int:
     ap = argparse.ArgumentParser(description=__doc__, formatter_class=argparse.RawDescriptionHelpFormatter)
     ap.add_argument("--shapes", default="so400m,b16", help="comma-separated shape sets: " + ", ".join(SHAPE_SETS))
     ap.add_argument("--m-steps", type=int, default=11, help="M from rows_per_image to rows_per_image * 2^(m-steps - 1)")
-    ap.add_argument("--per-octave", type=int, default=4, help="points of the M ladder per doubling, up to 16 images")
+    ap.add_argument("--per-octave", type=int, default=8, help="points of the M ladder per doubling, up to 16 images; half as many up to 46 656 rows")
     ap.add_argument("--max-rows", type=int, default=None)
     ap.add_argument("--repeats", type=int, default=5)
     ap.add_argument("--iters", type=int, default=10)

@@ -14,13 +14,13 @@ GENERAL = 6       # 128 x 128 tiles on single CTAs: serves every layer and outpu
 # between them they reach every row of the cost model (tests/test_tooling.py).
 SHAPES = {
     "gelu": [(1, 16, 16), (769, 400, 592), (9473, 144, 80), (5121, 1296, 592), (9473, 144, 2128), (769, 2320, 592), (300, 2064, 1616), (129, 416, 16),
-             (5003, 528, 1104), (5003, 528, 4176), (9001, 784, 4176)],
-    "tanh": [(127, 144, 80), (9473, 144, 1616), (9473, 144, 80), (20001, 528, 2128), (1300, 2320, 4176), (700, 656, 592), (129, 416, 272),
+             (5003, 528, 1104), (5003, 528, 4176), (9001, 784, 4176), (5003, 3088, 80)],
+    "tanh": [(1300, 3088, 592), (127, 144, 80), (9473, 144, 1616), (9473, 144, 80), (20001, 528, 2128), (1300, 2320, 4176), (700, 656, 592), (129, 416, 272),
              (5003, 784, 4176), (4000, 1600, 4176)],
     "none": [(129, 400, 592), (9473, 144, 592), (9473, 1040, 1104), (20001, 272, 4176), (769, 2320, 3072), (3001, 2320, 16), (16001, 2320, 1616),
              (700, 528, 1104), (129, 416, 16), (4000, 784, 1104), (5003, 1296, 4176)],
     "fc2": [(1, 16, 16), (2369, 528, 592), (20001, 16, 1616), (9473, 144, 80), (9473, 656, 80), (16001, 656, 1616), (5121, 784, 3072), (1300, 2064, 16),
-            (700, 528, 16), (129, 416, 16), (5003, 1296, 4176)],
+            (700, 528, 16), (129, 416, 16), (5003, 1296, 4176), (7001, 1040, 4176)],
     "pe": [(127, 144, 80), (9473, 144, 80), (769, 1552, 4176), (3001, 2320, 16), (700, 784, 2128), (129, 416, 16), (7001, 1040, 2128)],
 }
 
